@@ -150,6 +150,7 @@ void release(aed_handle* h) {
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
                   (void*)h->d_slol})
     mem_dev_free(p, h->stream);
+  mom_rows_free(h->mrows, h->stream);
   delete h->mp;
   delete h->sp;
   mem_host_free(h->h_scal);
@@ -357,7 +358,19 @@ int handle_tune(aed_handle* h, bool f32, const void* x, void* y) {
   return v < 0 ? pick_variant(h, f32, x, y, &v) : AED_OK;
 }
 
+int handle_mom_rows(aed_handle* h) {
+  // AED_MOM_WALK=1 keeps the walking apply (a test compares the two bit for bit)
+  if (const char* e = std::getenv("AED_MOM_WALK"); e && e[0] == '1') {
+    h->mrows.rows = MomRows();
+    return AED_OK;
+  }
+  if (h->gen) return spin_mom_rows_build(*h->sp, *h->mp, h->sdev, h->spin_mom_tables(), h->mrows, h->stream);
+  return mom_rows_build(*h->mp, h->dt, h->mom_tables(), h->mrows, h->stream);
+}
+
 int handle_hv(aed_handle* h, bool f32, const void* x, void* y, double* alpha_part) {
+  if (h->mom && h->mrows.rows.ent)
+    return launch_mom_rows(h->mrows.rows, !h->gen, (const double*)x, (double*)y, alpha_part, h->stream);
   if (h->gen && h->mom)
     return launch_spin_mom_hv(*h->sp, *h->mp, h->sdev, h->spin_mom_tables(), (const double*)x, (double*)y,
                               alpha_part, h->stream);
@@ -703,7 +716,7 @@ int aed_create_momentum(const aed_model_desc* model, const aed_translations* tr,
   h->dim = dim;
   h->vlen = 2 * dim;
   if ((rc = mem_dev_alloc_n(&h->d_partA, (size_t)mom_tiles(dim) + 1)) ||
-      (rc = mem_dev_alloc_n(&h->d_partB, (size_t)red_chunks(h->vlen) + 1))) {
+      (rc = mem_dev_alloc_n(&h->d_partB, (size_t)red_chunks(h->vlen) + 1)) || (rc = handle_mom_rows(h))) {
     release(h);
     return rc;
   }
@@ -898,7 +911,7 @@ int aed_create_spin_momentum(const aed_model_desc* model, int32_t two_s, const a
   h->dim = dim;
   h->vlen = 2 * dim;
   if ((rc = mem_dev_alloc_n(&h->d_partA, (size_t)mom_tiles(dim) + 1)) ||
-      (rc = mem_dev_alloc_n(&h->d_partB, (size_t)red_chunks(h->vlen) + 1))) {
+      (rc = mem_dev_alloc_n(&h->d_partB, (size_t)red_chunks(h->vlen) + 1)) || (rc = handle_mom_rows(h))) {
     release(h);
     return rc;
   }
@@ -1082,11 +1095,12 @@ int aed_set_couplings(aed_handle* h, const aed_model_desc* model) {
   h->rec_live = false;
   if (h->gen) {  // same sector: new site terms and bonds
     spin_couplings(h->model, *h->sp);
+    if (h->mom && (rc = handle_mom_rows(h))) return rc;
     return spin_lo_table(h);
   }
   if (h->mom) {  // same basis and translations: new flip list and diagonal
     mom_flips(h->model, *h->mp);
-    if ((rc = launch_mom_diag(h->P, h->d_reps, h->dim, h->d_mdiag, h->stream))) return rc;
+    if ((rc = launch_mom_diag(h->P, h->d_reps, h->dim, h->d_mdiag, h->stream)) || (rc = handle_mom_rows(h))) return rc;
     AED_CUDA_TRY(cudaStreamSynchronize(h->stream));
     return AED_OK;
   }

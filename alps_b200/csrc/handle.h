@@ -51,6 +51,7 @@ struct aed_handle {
   double* d_mdiag = nullptr;
   uint32_t* d_map = nullptr;
   aed::MomTables mom_tables() const { return {d_reps, d_norm, d_mdiag, d_map, dim}; }
+  aed::MomRowStore mrows;  // the apply's stored rows
   uint64_t* d_sreps = nullptr;  // representatives of a spin-S momentum sector (mom && gen)
   aed::SpinMomTables spin_mom_tables() const { return {d_sreps, d_norm, d_map, dim}; }
   // spin-S sector (aed_create_spin): tables of spin.cuh
@@ -145,6 +146,9 @@ int spin_measure_pairs(aed_handle* h, const double* psi, int kind, int n, const 
 int spin_mom_expectation(aed_handle* h, const double* psi, int kind, int n, const int32_t* si, const int32_t* sj,
                          double* out);
 
+// Form the stored rows of a momentum handle for its couplings (none where
+// they do not fit: the apply then walks the representatives).
+int handle_mom_rows(aed_handle* h);
 int handle_hv(aed_handle* h, bool f32, const void* x, void* y, double* alpha_part);
 // AED_ERR_TIMEOUT (and the flag cleared) when a kernel of the handle gave up a
 // bounded wait since the last check; waits for the handle's stream.

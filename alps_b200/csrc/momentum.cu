@@ -5,10 +5,12 @@
 // Reference paths are relative to the ALPS source tree.
 
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
 #include "handle.h"
+#include "mom_rows.cuh"
 #include "momentum.cuh"
 #include "reduce.cuh"
 
@@ -269,6 +271,172 @@ __global__ void __launch_bounds__(kMomThreads) mom_hv_kernel(const __grid_consta
   }
 }
 
+// Stored rows (mom_rows.cuh).  The distinct normalisations of the sector into
+// slots[0 .. kMomRowNorms): whichever thread meets a new one claims a slot.
+__global__ void __launch_bounds__(kMomThreads) mom_row_norms_kernel(const double* __restrict__ norm, int64_t dim,
+                                                                    MomRowMarks* __restrict__ marks) {
+  for (int64_t i = blockIdx.x * (int64_t)kMomThreads + threadIdx.x; i < dim; i += (int64_t)gridDim.x * kMomThreads) {
+    const unsigned long long w = __double_as_longlong(norm[i]);  // not 0: every normalisation is positive
+    int s = 0;
+    for (; s < kMomRowNorms; ++s) {
+      unsigned long long was = *(volatile unsigned long long*)(marks->norm + s);
+      if (was == 0ull) was = atomicCAS(marks->norm + s, 0ull, w);
+      if (was == 0ull || was == w) break;
+    }
+    if (s == kMomRowNorms) marks->many = 1u;
+  }
+}
+
+// One warp per slice of 32 representatives.  kFill false: the width of every
+// slice (its longest row) and the pairs of normalisations that differ within
+// a term; true: the entries.
+template <bool kFill>
+__global__ void __launch_bounds__(kMomThreads) mom_row_kernel(const __grid_constant__ MomParams mp,
+                                                              const __grid_constant__ MomRowSpec spec,
+                                                              const DevTables t, const MomTables m,
+                                                              MomRowMarks* __restrict__ marks,
+                                                              uint32_t* __restrict__ width,
+                                                              const uint32_t* __restrict__ off,
+                                                              uint32_t* __restrict__ ent) {
+  const int64_t slices = (m.dim + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  const uint32_t lm = (1u << t.Nlo) - 1u;
+  for (int64_t s = (blockIdx.x * (int64_t)kMomThreads + threadIdx.x) / 32; s < slices;
+       s += (int64_t)gridDim.x * kMomThreads / 32) {
+    const int64_t i = s * 32 + lane;
+    uint64_t o = kFill ? off[s] : 0u;
+    if (i < m.dim) {
+      const uint32_t r = m.reps[i];
+      const double ni = m.norm[i];
+      for (int q = 0; q < mp.n_flip; ++q) {
+        const uint32_t f = mp.flip_mask[q], b = r & f;
+        if (b == 0u || b == f) continue;  // parallel spins: no flip
+        const uint32_t s2 = r ^ f;
+        const uint32_t e = __ldg(m.map + __ldg(t.thi + (s2 >> t.Nlo)) + __ldg(t.tlo + (s2 & lm)));
+        if (e == kMomNone) continue;
+        if (kFill)
+          ent[o * 32 + lane] = mom_row_entry(spec, m.norm, ni, spec.vid[q], e);
+        else
+          mom_row_mark(marks, m.norm, ni, e);
+        ++o;
+      }
+    }
+    if (kFill) {
+      for (const uint64_t o1 = off[s + 1]; o < o1; ++o) ent[o * 32 + lane] = kMomRowPad;
+    } else {
+      const uint32_t n = __reduce_max_sync(0xffffffffu, (uint32_t)o);
+      if (lane == 0) width[s] = n;
+    }
+  }
+}
+
+// U terms of a row: the x_j of all of them asked for, then added in order.  A
+// padding entry adds 0 * 0; a term whose n_j differs from n_i has its
+// coefficient beyond the n_base staged ones, in global memory.
+template <int U>
+__device__ __forceinline__ void mom_row_terms(const uint32_t (&e)[U], int jbits, uint32_t jmask, uint32_t n_base,
+                                              const double2* cf, const double2* __restrict__ cfg,
+                                              const double2* __restrict__ x, double& are, double& aim) {
+  double2 xj[U];
+#pragma unroll
+  for (int v = 0; v < U; ++v)
+    xj[v] = e[v] != kMomRowPad ? __ldg(x + (e[v] & jmask)) : make_double2(0.0, 0.0);
+#pragma unroll
+  for (int v = 0; v < U; ++v) {
+    const uint32_t k = e[v] >> jbits;
+    double2 c = make_double2(0.0, 0.0);
+    if (k < n_base)
+      c = cf[k];
+    else if (e[v] != kMomRowPad)
+      c = __ldg(cfg + k);
+    are = fma(c.x, xj[v].x, fma(-c.y, xj[v].y, are));
+    aim = fma(c.x, xj[v].y, fma(c.y, xj[v].x, aim));
+  }
+}
+
+// y = H x from the stored rows, one row per thread.  A row's terms are a
+// coalesced stream of entries and, U at a time, the x_j they name, so the
+// only dependent load left is x_j itself; the entries are read once and are
+// kept out of the way of x in L2.  The coefficients phase_t * element are
+// staged in shared memory, those of terms with n_j != n_i (an orbit that a
+// translation fixes: few) read from the handle's table.  alpha_part: one partial of
+// Re<x, y> per kMomTileRows rows, formed after the tile's rows in the thread
+// order and tree of the walking kernel (256 threads, four rows each).
+// Bound by the x_j gathers (one 32-byte sector each from L2): the walking
+// kernel, bound by the latency of four dependent loads a term, took 225.5 us
+// a product on the J1-J2 chain L=28 and 287 on the spin-1 chain L=18; this one
+// 84.5 and 100.
+template <bool kDiagFirst, int NT, int U, int MINB>
+__global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, const double2* __restrict__ x, double2* y,
+                                                            double* __restrict__ alpha_part) {
+  extern __shared__ __align__(16) unsigned char mom_rows_dyn[];
+  double2* cf = reinterpret_cast<double2*>(mom_rows_dyn);
+  __shared__ double red[kMomThreads / 32];
+  const uint32_t n_base = (uint32_t)rw.n_base;
+  for (uint32_t k = threadIdx.x; k < n_base; k += NT) cf[k] = __ldg(rw.cf + k);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const uint32_t jmask = (1u << rw.jbits) - 1u;
+  const int64_t ntile = mom_tiles(rw.dim);
+  for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+#pragma unroll 1
+    for (int u = 0; u < kMomTileRows / NT; ++u) {
+      const int64_t i = tile * kMomTileRows + u * NT + threadIdx.x;
+      if (i - lane >= rw.dim) break;  // the whole slice is past the end
+      const uint32_t o0 = __ldg(rw.off + i / 32), o1 = __ldg(rw.off + i / 32 + 1);
+      const uint32_t* ep = rw.ent + (size_t)o0 * 32 + lane;
+      const bool row = i < rw.dim;
+      double are = 0.0, aim = 0.0;
+      if (kDiagFirst && row) {
+        const double2 xi = __ldg(x + i);
+        const double d = __ldg(rw.diag + i);
+        are = d * xi.x;
+        aim = d * xi.y;
+      }
+      uint32_t o = o0;
+      for (; o + U <= o1; o += U, ep += U * 32) {
+        uint32_t e[U];
+#pragma unroll
+        for (int v = 0; v < U; ++v) e[v] = __ldcs(ep + v * 32);
+        mom_row_terms<U>(e, rw.jbits, jmask, n_base, cf, rw.cf, x, are, aim);
+      }
+      for (; o < o1; ++o, ep += 32) {
+        uint32_t e[1] = {__ldcs(ep)};
+        mom_row_terms<1>(e, rw.jbits, jmask, n_base, cf, rw.cf, x, are, aim);
+      }
+      if (!kDiagFirst && row) {
+        const double2 xi = __ldg(x + i);
+        const double d = __ldg(rw.diag + i);
+        are = fma(d, xi.x, are);
+        aim = fma(d, xi.y, aim);
+      }
+      if (row) y[i] = make_double2(are, aim);
+    }
+    if (alpha_part) {
+      __syncthreads();  // the tile's rows of y are written
+      double dot = 0.0;
+      if (threadIdx.x < kMomThreads) {
+#pragma unroll
+        for (int u = 0; u < kMomTileRows / kMomThreads; ++u) {
+          const int64_t i = tile * kMomTileRows + u * kMomThreads + threadIdx.x;
+          if (i < rw.dim) {
+            const double2 xi = __ldg(x + i), yi = y[i];
+            dot = fma(xi.x, yi.x, fma(xi.y, yi.y, dot));
+          }
+        }
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, o);
+        if (lane == 0) red[threadIdx.x >> 5] = dot;
+      }
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        double r = lane < kMomThreads / 32 ? red[lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+        if (lane == 0) alpha_part[tile] = r;
+      }
+    }
+  }
+}
+
 // One pass per call: each CTA sums its rows' terms into part[blockIdx.x].
 template <int KIND>
 __global__ void __launch_bounds__(kMomThreads) mom_expect_kernel(const __grid_constant__ MomParams mp,
@@ -319,11 +487,15 @@ __global__ void __launch_bounds__(kMomThreads) mom_expect_kernel(const __grid_co
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-int grid_for(int64_t units) {
+int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t cap = (int64_t)sms * 8;
+  return sms;
+}
+
+int grid_for(int64_t units) {
+  const int64_t cap = (int64_t)sm_count() * 8;
   return (int)(units < 1 ? 1 : (units < cap ? units : cap));
 }
 
@@ -439,6 +611,155 @@ int mom_expectation(const MomParams& mp, const DevTables& t, const MomTables& m,
   else
     mom_expect_kernel<AED_OBS_SPSM><<<grid, kMomThreads, 0, st>>>(mp, t, m, p2, pairs, part);
   return check_launch_counted("mom_expect_kernel");
+}
+
+void mom_rows_free(MomRowStore& rs, cudaStream_t st) {
+  for (void* p : {(void*)rs.ent, (void*)rs.off, (void*)rs.width, (void*)rs.diag, (void*)rs.cf, (void*)rs.marks})
+    mem_dev_free(p, st);
+  rs = MomRowStore();
+}
+
+int mom_rows_begin(const double* norm, int64_t dim, MomRowStore& rs, cudaStream_t st) {
+  const int64_t slices = (dim + 31) / 32;
+  if ((!rs.off && mem_dev_alloc_n(&rs.off, (size_t)slices + 1)) ||
+      (!rs.width && mem_dev_alloc_n(&rs.width, (size_t)slices)) ||
+      (!rs.cf && mem_dev_alloc_n(&rs.cf, (size_t)kMomRowIdx)) || (!rs.marks && mem_dev_alloc_n(&rs.marks, 1)))
+    return kMomRowsNone;
+  AED_CUDA_TRY(cudaMemsetAsync(rs.marks, 0, sizeof(MomRowMarks), st));
+  mom_row_norms_kernel<<<grid_for((dim + kMomThreads - 1) / kMomThreads), kMomThreads, 0, st>>>(norm, dim, rs.marks);
+  return check_launch_counted("mom_row_norms_kernel");
+}
+
+int mom_rows_plan(const MomParams& mp, int64_t dim, MomRowSpec& spec, MomRowStore& rs, cudaStream_t st) {
+  const int64_t slices = (dim + 31) / 32;
+  MomRowMarks mk;
+  std::vector<uint32_t> w((size_t)slices), o((size_t)slices + 1);
+  AED_CUDA_TRY(cudaMemcpyAsync(&mk, rs.marks, sizeof mk, cudaMemcpyDeviceToHost, st));
+  AED_CUDA_TRY(cudaMemcpyAsync(w.data(), rs.width, (size_t)slices * 4, cudaMemcpyDeviceToHost, st));
+  AED_CUDA_TRY(cudaStreamSynchronize(st));
+  if (mk.many) return kMomRowsNone;
+  // the ratios n_j / n_i that occur, 1 first
+  std::vector<double> ratio{1.0};
+  for (int a = 0; a < kMomRowNorms; ++a)
+    for (int b = 0; b < kMomRowNorms; ++b) {
+      spec.ridx[a][b] = 0;
+      if (a == b || !(mk.used[a] >> b & 1u)) continue;
+      double na, nb;
+      std::memcpy(&na, &mk.norm[a], 8);
+      std::memcpy(&nb, &mk.norm[b], 8);
+      const double v = nb / na;
+      size_t k = 0;
+      while (k < ratio.size() && ratio[k] != v) ++k;
+      if (k == ratio.size()) ratio.push_back(v);
+      spec.ridx[a][b] = (uint8_t)k;
+    }
+  for (int a = 0; a < kMomRowNorms; ++a) std::memcpy(&spec.norm[a], &mk.norm[a], 8);
+  spec.n_trans = mp.n_trans;
+  const size_t n_idx = ratio.size() * (size_t)spec.n_val * (size_t)mp.n_trans;
+  int jb = 1;
+  while (((int64_t)1 << jb) <= dim) ++jb;  // dim < 2^jb
+  if (n_idx > (size_t)kMomRowIdx || n_idx >= ((uint64_t)1 << (32 - jb))) return kMomRowsNone;  // no entry is all ones
+  spec.jbits = jb;
+  uint64_t run = 0;
+  for (int64_t s = 0; s < slices; ++s) {
+    o[(size_t)s] = (uint32_t)run;
+    run += w[(size_t)s];
+  }
+  o[(size_t)slices] = (uint32_t)run;
+  if (run >= 0xffffffffull) return kMomRowsNone;
+  const size_t need = (size_t)run * 32;
+  if (need > rs.ent_cap) {
+    mem_dev_free(rs.ent, st);
+    rs.ent = nullptr;
+    rs.ent_cap = 0;
+    if (mem_dev_alloc_n(&rs.ent, need)) return kMomRowsNone;
+    rs.ent_cap = need;
+  }
+  // phase_t * (element * ratio), multiplied in the order of the walk
+  std::vector<double> cf(2 * n_idx);
+  size_t k = 0;
+  for (double rt : ratio)
+    for (int v = 0; v < spec.n_val; ++v)
+      for (int t = 0; t < mp.n_trans; ++t) {
+        const double f = spec.val[v] * rt;
+        cf[k++] = f * mp.phase_re[t];
+        cf[k++] = f * mp.phase_im[t];
+      }
+  AED_CUDA_TRY(cudaMemcpyAsync(rs.off, o.data(), o.size() * 4, cudaMemcpyHostToDevice, st));
+  AED_CUDA_TRY(cudaMemcpyAsync(rs.cf, cf.data(), cf.size() * 8, cudaMemcpyHostToDevice, st));
+  AED_CUDA_TRY(cudaStreamSynchronize(st));  // o and cf go out of scope
+  return AED_OK;
+}
+
+void mom_rows_done(const MomRowSpec& spec, int64_t dim, const double* diag, MomRowStore& rs) {
+  MomRows& r = rs.rows;
+  r.ent = rs.ent;
+  r.off = rs.off;
+  r.cf = rs.cf;
+  r.diag = diag;
+  r.dim = dim;
+  r.jbits = spec.jbits;
+  r.n_base = spec.n_val * spec.n_trans;
+}
+
+int mom_rows_build(const MomParams& mp, const DevTables& t, const MomTables& m, MomRowStore& rs, cudaStream_t st) {
+  rs.rows = MomRows();
+  if (m.dim == 0 || mp.n_flip == 0) return AED_OK;
+  MomRowSpec spec;
+  for (int q = 0; q < mp.n_flip; ++q) {
+    int v = 0;
+    while (v < spec.n_val && spec.val[v] != mp.flip_c[q]) ++v;
+    if (v == spec.n_val) {
+      if (v == kMomRowVals) return AED_OK;
+      spec.val[spec.n_val++] = mp.flip_c[q];
+    }
+    spec.vid[q] = (uint8_t)v;
+  }
+  const int grid = grid_for((m.dim + kMomThreads - 1) / kMomThreads);
+  int rc = mom_rows_begin(m.norm, m.dim, rs, st);
+  if (!rc) {
+    mom_row_kernel<false><<<grid, kMomThreads, 0, st>>>(mp, spec, t, m, rs.marks, rs.width, nullptr, nullptr);
+    rc = check_launch_counted("mom_row_kernel");
+  }
+  if (!rc) rc = mom_rows_plan(mp, m.dim, spec, rs, st);
+  if (!rc) {
+    mom_row_kernel<true><<<grid, kMomThreads, 0, st>>>(mp, spec, t, m, rs.marks, nullptr, rs.off, rs.ent);
+    rc = check_launch_counted("mom_row_kernel");
+  }
+  if (rc == kMomRowsNone) return AED_OK;  // the apply walks the representatives
+  if (!rc) mom_rows_done(spec, m.dim, m.diag, rs);
+  return rc;
+}
+
+template <int NT, int U, int MINB>
+void mom_rows_go(const MomRows& r, bool diag_first, unsigned grid, size_t dyn, const double2* x, double2* y,
+                 double* alpha_part, cudaStream_t st) {
+  if (diag_first)
+    mom_rows_kernel<true, NT, U, MINB><<<grid, NT, dyn, st>>>(r, x, y, alpha_part);
+  else
+    mom_rows_kernel<false, NT, U, MINB><<<grid, NT, dyn, st>>>(r, x, y, alpha_part);
+}
+
+// A tile per CTA.  Many tiles: 256 threads, five CTAs per SM (48 registers,
+// no spill), four x_j in flight per thread: 84.5 us a product on the J1-J2
+// chain L=28 (1.43M rows), against 87.6 with six in flight at four CTAs, 86.0
+// with 512 threads and 92.8-107 with fewer, larger CTAs.  Up to four tiles
+// per SM the 1024 rows of a tile run side by side instead of four deep, so
+// that a small sector still fills the SMs: a solve of the chain L=22, k = pi
+// (32 tiles) takes 5.0 ms against 6.1 with 256 threads.
+int launch_mom_rows(const MomRows& r, bool diag_first, const double* x, double* y,
+                    double* alpha_part, cudaStream_t st) {
+  if (r.dim == 0) return AED_OK;
+  const int64_t tiles = mom_tiles(r.dim);
+  const unsigned grid = (unsigned)(tiles < (int64_t)1 << 20 ? tiles : (int64_t)1 << 20);
+  const size_t dyn = (size_t)r.n_base * sizeof(double2);
+  const double2* xc = reinterpret_cast<const double2*>(x);
+  double2* yc = reinterpret_cast<double2*>(y);
+  if (tiles > (int64_t)sm_count() * 4)
+    mom_rows_go<256, 4, 5>(r, diag_first, grid, dyn, xc, yc, alpha_part, st);
+  else
+    mom_rows_go<1024, 6, 1>(r, diag_first, grid, dyn, xc, yc, alpha_part, st);
+  return check_launch_counted("mom_rows_kernel");
 }
 
 int launch_mom_hv(const MomParams& mp, const DevTables& t, const MomTables& m, const double* x, double* y,

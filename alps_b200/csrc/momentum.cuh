@@ -47,6 +47,32 @@ struct MomTables {
   int64_t dim;
 };
 
+// The stored rows of the apply (mom_rows.cuh); ent == nullptr: none, the apply
+// walks the representatives.
+constexpr int kMomRowVals = 64;    // distinct elements
+constexpr int kMomRowNorms = 16;   // distinct normalisations
+constexpr int kMomRowIdx = 2048;   // coefficients (ratios x elements x translations)
+struct MomRowMarks;
+struct MomRows {
+  const uint32_t* ent = nullptr;
+  const uint32_t* off = nullptr;  // per slice of 32 rows, in units of 32 entries
+  const double2* cf = nullptr;    // coefficients; the first n_base have n_j = n_i
+  const double* diag = nullptr;
+  int64_t dim = 0;
+  int jbits = 0, n_base = 0;
+};
+// Device memory of the stored rows, kept by the handle.
+struct MomRowStore {
+  uint32_t* ent = nullptr;
+  uint32_t* off = nullptr;
+  uint32_t* width = nullptr;
+  double2* cf = nullptr;
+  MomRowMarks* marks = nullptr;
+  double* diag = nullptr;  // spin S: the representatives' diagonal elements
+  size_t ent_cap = 0;      // entries allocated
+  MomRows rows;
+};
+
 // Build the sector's tables on the device: reps / norm / diag (dim entries)
 // and map (D entries) are allocated with mem_dev_alloc and owned by the
 // caller.  HvParams supplies the diagonal terms (site terms, then bonds).
@@ -58,6 +84,14 @@ int launch_mom_diag(const HvParams& P, const uint32_t* reps, int64_t dim, double
 // of Re<x, y> per kMomTileRows rows.
 int launch_mom_hv(const MomParams& mp, const DevTables& t, const MomTables& m, const double* x, double* y,
                   double* alpha_part, cudaStream_t st);
+// Form the stored rows for the couplings in mp; leaves st.rows.ent null when
+// an entry cannot hold the sector's indices or there is no memory for them.
+int mom_rows_build(const MomParams& mp, const DevTables& t, const MomTables& m, MomRowStore& rs, cudaStream_t st);
+void mom_rows_free(MomRowStore& rs, cudaStream_t st);
+// y = H x from the stored rows, alpha_part as launch_mom_hv; diag_first: the
+// diagonal term starts the row's sum (spin 1/2), else it ends it (spin S).
+int launch_mom_rows(const MomRows& r, bool diag_first, const double* x, double* y, double* alpha_part,
+                    cudaStream_t st);
 __host__ __device__ inline int64_t mom_tiles(int64_t dim) { return (dim + kMomTileRows - 1) / kMomTileRows; }
 
 // <psi| sum_p O(i_p, j_p) |psi> in a momentum sector for a list of site pairs
@@ -87,6 +121,8 @@ struct SpinMomTables {
 };
 int spin_mom_build(const MomParams& mp, const SpinDev& t, cudaStream_t st, uint64_t** reps, double** norm,
                    uint32_t** map, int64_t* dim);
+int spin_mom_rows_build(const SpinParams& p, const MomParams& mp, const SpinDev& t, const SpinMomTables& m,
+                        MomRowStore& rs, cudaStream_t st);
 // y = H x on interleaved complex vectors (spin.cu); alpha_part as launch_mom_hv.
 int launch_spin_mom_hv(const SpinParams& p, const MomParams& mp, const SpinDev& t, const SpinMomTables& m,
                        const double* x, double* y, double* alpha_part, cudaStream_t st);

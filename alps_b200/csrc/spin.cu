@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "handle.h"
+#include "mom_rows.cuh"
 #include "reduce.cuh"
 #include "spin.cuh"
 
@@ -665,6 +666,57 @@ __global__ void __launch_bounds__(kSpinThreads, 5) spin_mom_hv_kernel(const __gr
   }
 }
 
+// Stored rows of a spin-S momentum sector (mom_rows.cuh), tabulated forms
+// only: one warp per slice of 32 representatives.  kFill false: the width of
+// every slice (its longest row) and the normalisations that differ within a
+// term; true: the entries in walk order and the rows' diagonal elements.
+template <class Sh, bool kFill>
+__global__ void __launch_bounds__(kSpinThreads) spin_mom_row_kernel(const __grid_constant__ SpinParams p,
+                                                                    const __grid_constant__ MomRowSpec spec,
+                                                                    const SpinDev t, const SpinMomTables m,
+                                                                    MomRowMarks* __restrict__ marks,
+                                                                    uint32_t* __restrict__ width,
+                                                                    const uint32_t* __restrict__ off,
+                                                                    uint32_t* __restrict__ ent,
+                                                                    double* __restrict__ diag) {
+  __shared__ Sh sh;
+  const bool has_site = __syncthreads_or(stage_spin(p, t, sh)) != 0;
+  const int shift = t.bits * t.Nl;
+  const uint64_t lm = (1ull << shift) - 1ull;
+  const int64_t slices = (m.dim + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  for (int64_t s = (blockIdx.x * (int64_t)kSpinThreads + threadIdx.x) / 32; s < slices;
+       s += (int64_t)gridDim.x * kSpinThreads / 32) {
+    const int64_t i = s * 32 + lane;
+    uint64_t o = kFill ? off[s] : 0u;
+    if (i < m.dim) {
+      const uint64_t r = m.reps[i];
+      const uint32_t rh = (uint32_t)(r >> shift), rl = (uint32_t)(r & lm);
+      const double ni = m.norm[i];
+      const double dg = spin_row(sh, p.n_bonds, has_site, t, rh, rl, __ldg(t.thi + rh), __ldg(t.tlo + rl),
+                                 [&](double v, uint32_t rk) {
+        const uint32_t e = __ldg(m.map + rk);
+        if (e == kMomNone) return;
+        if (kFill) {
+          int q = 0;
+          while (spec.val[q] != v) ++q;  // v is one of them
+          ent[o * 32 + lane] = mom_row_entry(spec, m.norm, ni, q, e);
+        } else {
+          mom_row_mark(marks, m.norm, ni, e);
+        }
+        ++o;
+      });
+      if (kFill) diag[i] = dg;
+    }
+    if (kFill) {
+      for (const uint64_t o1 = off[s + 1]; o < o1; ++o) ent[o * 32 + lane] = kMomRowPad;
+    } else {
+      const uint32_t n = __reduce_max_sync(0xffffffffu, (uint32_t)o);
+      if (lane == 0) width[s] = n;
+    }
+  }
+}
+
 // Expectation values in one vector of the sector (the spin-S counterpart of
 // measure.cu's meas_kernel): per site pair p,
 //   kind SZ     sum_s psi_s^2 m_i(s)
@@ -944,6 +996,51 @@ int launch_spin_mom_hv(const SpinParams& p, const MomParams& mp, const SpinDev& 
     spin_mom_hv_kernel<typename decltype(form)::type><<<grid, kSpinThreads, 0, st>>>(p, mp, t, m, xc, yc, alpha_part);
   });
   return check_launch_counted("spin_mom_hv_kernel");
+}
+
+int spin_mom_rows_build(const SpinParams& p, const MomParams& mp, const SpinDev& t, const SpinMomTables& m,
+                        MomRowStore& rs, cudaStream_t st) {
+  rs.rows = MomRows();
+  if (m.dim == 0 || p.n_cls == 0) return AED_OK;
+  MomRowSpec spec;
+  for (int c = 0; c < p.n_cls; ++c)
+    for (int pr = 0; pr < t.d * t.d; ++pr)
+      for (int s = 0; s < kSpinMaxOff && ((p.pk[c][pr] >> (8 * s)) & 255u); ++s) {
+        const double e = p.pov[c][pr][s];
+        if (e != e) return AED_OK;  // not a number: no index for it
+        int v = 0;
+        while (v < spec.n_val && spec.val[v] != e) ++v;
+        if (v < spec.n_val) continue;
+        if (v == kMomRowVals) return AED_OK;
+        spec.val[spec.n_val++] = e;
+      }
+  if (spec.n_val == 0) return AED_OK;
+  if (!rs.diag && mem_dev_alloc_n(&rs.diag, (size_t)m.dim)) return AED_OK;
+  const int64_t want = (m.dim + kSpinThreads - 1) / kSpinThreads, cap = (int64_t)sm_count() * 8;
+  const int grid = (int)(want < cap ? want : cap);
+  int rc = mom_rows_begin(m.norm, m.dim, rs, st);
+  if (!rc) {
+    with_spin_form(p, t, [&](auto form) {
+      using Sh = typename decltype(form)::type;
+      if constexpr (!std::is_same<Sh, SpinShared>::value)
+        spin_mom_row_kernel<Sh, false><<<grid, kSpinThreads, 0, st>>>(p, spec, t, m, rs.marks, rs.width, nullptr,
+                                                                      nullptr, nullptr);
+    });
+    rc = check_launch_counted("spin_mom_row_kernel");
+  }
+  if (!rc) rc = mom_rows_plan(mp, m.dim, spec, rs, st);
+  if (!rc) {
+    with_spin_form(p, t, [&](auto form) {
+      using Sh = typename decltype(form)::type;
+      if constexpr (!std::is_same<Sh, SpinShared>::value)
+        spin_mom_row_kernel<Sh, true><<<grid, kSpinThreads, 0, st>>>(p, spec, t, m, rs.marks, nullptr, rs.off, rs.ent,
+                                                                     rs.diag);
+    });
+    rc = check_launch_counted("spin_mom_row_kernel");
+  }
+  if (rc == kMomRowsNone) return AED_OK;  // the apply walks the representatives
+  if (!rc) mom_rows_done(spec, m.dim, rs.diag, rs);
+  return rc;
 }
 
 size_t spin_lo_table_bytes(const SpinParams& p, SpinDev& t) {

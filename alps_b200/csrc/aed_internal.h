@@ -56,6 +56,7 @@ struct HvParams {
   int N, Nlo, n_up;
   int n_pairs;  // entries in low[] and rise[]
   int n_diag;
+  int finite;  // every flip's coefficient is finite
   uint32_t lomask;
   // pairs in ascending-column order for a row: "low" flips (target < source)
   // sorted by (hi desc, lo asc); "rise" flips (target > source) by (hi asc, lo desc)
@@ -83,13 +84,7 @@ struct BasisTables {
 
 int build_tables(int N, int n_up, BasisTables& t);
 
-// Lo-neighbour table: for every lo state l (rank r within its popcount class
-// k), the flips with both bits in the lo part that apply to l, as
-// (target rank r' = tlo[l ^ flip]) | (flip index << 16), sorted by r' and
-// padded with kEllPad to a common width W.  Entry e of row r of class k sits
-// at W * looff[k] + e * C(Nlo, k) + r (coalesced across consecutive rows).
-constexpr uint32_t kEllPad = 0xffffffffu;
-void build_lo_table(const BasisTables& t, const HvParams& P, std::vector<uint32_t>& ell, int* width);
+constexpr uint32_t kEllPad = 0xffffffffu;  // padding of the lo-neighbour table (launch_lo_table)
 
 // Work tiles over the sector: (hi block h, first row r0 within the block).
 void build_tiles(const BasisTables& t, int tile_rows, std::vector<uint32_t>& th, std::vector<uint32_t>& tr,
@@ -104,7 +99,8 @@ void build_tiles(const BasisTables& t, int tile_rows, std::vector<uint32_t>& th,
 void build_cross_table(const BasisTables& t, std::vector<uint16_t>& xt);
 constexpr int kBundleMax = 4;
 constexpr uint32_t kNoBlockEntry = 0xffffffffu;
-void build_block_list(const BasisTables& t, std::vector<uint32_t>& blk, int* maxrows);
+void build_block_list(const BasisTables& t, const HvParams& P, size_t window, std::vector<uint32_t>& blk,
+                      int* maxrows);
 
 // ---- tridiagonal / Tmatrix (host) ---------------------------------------------
 int tridiag_eigen(int n, double* d, double* e, double* zlast, double* zfull = nullptr);

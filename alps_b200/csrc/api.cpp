@@ -148,7 +148,7 @@ void release(aed_handle* h) {
                   (void*)h->d_reps, (void*)h->d_norm, (void*)h->d_mdiag, (void*)h->d_map, (void*)h->d_sthi,
                   (void*)h->d_stlo, (void*)h->d_slolist, (void*)h->d_slooff, (void*)h->d_sblk_hi,
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
-                  (void*)h->d_slol})
+                  (void*)h->d_slol, (void*)h->d_low_e, (void*)h->d_low_w})
     mem_dev_free(p, h->stream);
   mom_rows_free(h->mrows, h->stream);
   delete h->mp;
@@ -163,25 +163,33 @@ void release(aed_handle* h) {
 
 // (Re)build the lo-neighbour table of the handle's couplings on the device.
 int upload_lo_table(aed_handle* h) {
-  std::vector<uint32_t> ell;
-  int W = 0;
-  build_lo_table(h->tab, h->P, ell, &W);
-  cudaStreamSynchronize(h->stream);  // no apply reads the old table any more
-  if (ell.size() + 1 > h->d_ell_n) {  // grow only: new couplings usually keep the width
+  const int W = h->P.n_lolo;
+  const size_t n = ((size_t)W << h->tab.Nlo) + 1;
+  int rc = AED_OK;
+  if (n > h->d_ell_n) {  // grow only: new couplings usually keep the flips
     mem_dev_free(h->d_ell, h->stream);
     h->d_ell = nullptr;
     h->d_ell_n = 0;
-    const int rc = mem_dev_alloc_n(&h->d_ell, ell.size() + 1);
-    if (rc) return rc;
-    h->d_ell_n = ell.size() + 1;
-  }
-  if (!ell.empty()) {
-    AED_CUDA_TRY(cudaMemcpyAsync(h->d_ell, ell.data(), ell.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    AED_CUDA_TRY(cudaStreamSynchronize(h->stream));  // host vector goes out of scope
+    if ((rc = mem_dev_alloc_n(&h->d_ell, n))) return rc;
+    h->d_ell_n = n;
   }
   h->dt.ell = h->d_ell;
   h->dt.ell_w = W;
-  return AED_OK;
+  if ((rc = launch_lo_table(h->P, h->dt, h->d_ell, h->stream))) return rc;
+  // and in slices of 32 rows for the rows apply
+  const size_t slices = lo_slices(h->tab.Nlo), need = slices * (size_t)lo_slice_pairs(W) * 32;
+  if (need > h->d_low_n) {
+    mem_dev_free(h->d_low_e, h->stream);
+    h->d_low_e = nullptr;
+    h->d_low_n = 0;
+    if ((rc = mem_dev_alloc_n(&h->d_low_e, need))) return rc;
+    h->d_low_n = need;
+  }
+  if (!h->d_low_w && (rc = mem_dev_alloc_n(&h->d_low_w, slices))) return rc;
+  h->dt.low_e = h->d_low_e;
+  h->dt.low_w = h->d_low_w;
+  h->dt.low_st = lo_slice_pairs(W);
+  return launch_lo_slices(h->dt, h->dt.maxrows, h->P.n_lolo, h->d_low_e, h->d_low_w, h->stream);
 }
 
 int check_vec(const aed_handle* h, const void* p, const char* name) {
@@ -304,9 +312,8 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
       return AED_OK;
     }
   }
-  if (D < (1 << 12)) {  // tiny sectors: launch-bound, not worth timing (from L = 16 up the
-                        // bundle apply's 16 CTAs beat the tile apply's 7: 241 against 214 solves/s)
-    *out = 0;
+  if (D < (1 << 12)) {  // tiny sectors: launch-bound, not worth timing
+    *out = hv_small_variant();
     return AED_OK;
   }
   cudaEvent_t e0, e1;
@@ -380,8 +387,9 @@ int handle_hv(aed_handle* h, bool f32, const void* x, void* y, double* alpha_par
   int rc = handle_tune(h, f32, x, y);
   if (rc) return rc;
   rc = launch_variant(h, f32, h->hv_var[f32 ? 1 : 0], x, y, alpha_part);
-  // the tuned variant may not take these vectors (bulk copies need 16-byte
-  // aligned x and y): the tile apply takes any, with the same rows and partials
+  // the variant may not take these vectors or couplings (bulk copies need
+  // 16-byte aligned x and y, the rows apply finite couplings): the tile apply
+  // takes any, with the same rows and partials
   if (rc == kVariantNotApplicable) rc = launch_checked(h, f32, 0, x, y, alpha_part);
   return rc;
 }
@@ -526,7 +534,7 @@ int aed_create(const aed_model_desc* model, int precision, int device, aed_handl
   std::vector<uint16_t> xt;
   int maxrows = 0;
   build_tiles(h->tab, kHvTileRows, th, tr, &tf);
-  build_block_list(h->tab, blk, &maxrows);
+  build_block_list(h->tab, h->P, h->precision == AED_FP32 ? 64 : 1, blk, &maxrows);
   build_cross_table(h->tab, xt);
   const size_t nlo = h->tab.tlo.size(), nhi = h->tab.thi.size();
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {

@@ -1,0 +1,442 @@
+// apply_rows.cuh -- y = H x over bundles of hi blocks whose x lies interleaved
+// in shared memory: the kernel that large sectors take.
+//
+// The bundle apply (apply_blocks.cuh) spends 20 to 30 instructions on every
+// term of a row: bounds and padding tests per term, a coupling look-up and a
+// table entry per term and block, the test for the diagonal's column.  Here
+//   * x of the bundle's B blocks is staged row by row (row r of all B blocks
+//     side by side, 16 or 8 bytes), so that one lo-table entry, one coupling
+//     and one shared load serve the lo-part flip of all B blocks;
+//   * the lo table comes in slices of 32 rows (launch_lo_slices), each as wide
+//     as its longest row, the entries of smaller targets before those of
+//     larger ones: a warp walks its slice with a uniform trip count, the
+//     diagonal falls between the two parts, and a padding entry adds 0 * 0
+//     from a row of zeros (a row's sum is never -0, so that changes no bit);
+//   * an entry holds the byte offsets of its x row and of its coupling.
+// Rows add their terms in the order of the other applies (FP64: the explicit
+// matrix's columns), and the <x, y> partials have their thread order and tree:
+// they are formed from the finished rows, after the bundle.
+//
+// Reference paths are relative to the ALPS source tree.
+#pragma once
+
+#include "apply.cuh"
+
+namespace aed {
+namespace rapply {
+
+using apply::ApplyCtx;
+using apply::kCrossOp;
+using apply::kTileRows;
+using apply::SPair;
+using apply::TileOp;
+
+constexpr int kMaxB = 4;
+constexpr uint32_t kNullOp = 0x80000001u;     // an op that no row takes (no byte offset of an element)
+constexpr uint32_t kCrossTest = 0x80008000u;  // null bit and the required lo-bit value
+constexpr int kMaxItems = 32;  // (block, tile) pairs of a bundle: 4 blocks of at most 7 tiles
+
+template <typename T, int B>
+struct alignas(sizeof(T) * B) RowVec {
+  T v[B];
+};
+
+struct RowsSmem {
+  double lolo_c[kMaxBonds + 1];  // the last: 0, of the padding entries
+  int n1, n2, full;  // ops of the two lists; hi-part ops that all blocks have
+  double red[kMaxItems][kHvThreads / 32];
+};
+
+// The bundle's program: the flips outside the lo part that apply to its blocks,
+// op o of all B blocks side by side.
+//   FP64 (rows in column order): ops[o * B + j], the flips to smaller states in
+//   [0, n1), those to larger ones in [n1, n1 + n2);
+//   FP32: the hi-part flips as nb[o * B + j] and c[o * B + j], o < n1, the
+//   crossing ones at o >= cross0 with their lo bit and required values in bits[o].
+// Lists are as long as the longest block's, rounded up to a multiple of the
+// unrolling (at most 8), filled with null ops.
+struct Program {
+  TileOp* ops;
+  uint32_t* nb;
+  double* c;
+  uint32_t* bits;
+};
+__host__ __device__ inline int prog_ops(int elem, int n_pairs, int n_lolo) {
+  return (elem == 8 ? 2 : 1) * (n_pairs - n_lolo) + 14;
+}
+
+// Dynamic shared memory: x rows (and the row of zeros), the program, the flip pairs.
+__host__ __device__ inline size_t rows_smem_bytes(int row_bytes, int B, int maxrows, int n_pairs, int n_lolo) {
+  return (((size_t)(maxrows + 1) * row_bytes + 15) & ~(size_t)15) +
+         (size_t)prog_ops(row_bytes / B, n_pairs, n_lolo) * (B * sizeof(TileOp) + 16) +
+         2 * (size_t)n_pairs * sizeof(SPair);
+}
+
+// The value at a 32-bit byte offset (an FP32 vector of at most 2^30 rows; the
+// largest sector has 601 M): one add per address.
+template <typename T>
+__device__ __forceinline__ T at_byte(const T* __restrict__ p, uint32_t off) {
+  return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off));
+}
+
+// The lo-part flips of one part of the slice: np pairs of entries.
+template <typename T, typename Acc, int B>
+__device__ __forceinline__ void lo_terms(const uint2* __restrict__ tp, int np, const unsigned char* xs,
+                                         const unsigned char* cs, Acc (&acc)[B]) {
+  constexpr int kShift = sizeof(T) * B == 16 ? 0 : 1;
+  auto term = [&](uint32_t e) {
+    const double c = *reinterpret_cast<const double*>(cs + (e >> 20));
+    const RowVec<T, B> x = *reinterpret_cast<const RowVec<T, B>*>(xs + ((e & 0xfffffu) >> kShift));
+#pragma unroll
+    for (int j = 0; j < B; ++j) acc[j].add(c, x.v[j]);
+  };
+  // two pairs of entries ahead of the terms
+  uint2 a{}, b{};
+  if (np > 0) a = __ldg(tp);
+  if (np > 1) b = __ldg(tp + 32);
+#pragma unroll 1
+  for (int p = 0; p < np; p += 2) {
+    const uint2 e = a, f = b;
+    tp += 64;
+    if (p + 2 < np) a = __ldg(tp);
+    if (p + 3 < np) b = __ldg(tp + 32);
+    term(e.x);
+    term(e.y);
+    if (p + 1 < np) {
+      term(f.x);
+      term(f.y);
+    }
+  }
+}
+
+// FP64: n ops of every block (a multiple of U), U at a time for all B blocks:
+// their loads first, then the terms in order.  A crossing flip that the row
+// does not take adds c * 0, as a null op adds 0 * 0: neither changes a sum that
+// is never -0 (the couplings are finite).
+template <typename T, typename Acc, int B, int U>
+__device__ __forceinline__ void hi_terms(const TileOp* ops, int n, uint32_t r, const uint16_t* __restrict__ xt,
+                                         int Nlo, const T* __restrict__ x, Acc (&acc)[B]) {
+#pragma unroll 1
+  for (int o = 0; o < n; o += U) {
+    T xv[U][B];
+    double c[U][B];
+#pragma unroll
+    for (int v = 0; v < U; ++v)
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        const TileOp e = ops[(o + v) * B + j];
+        c[v][j] = e.c;
+        uint32_t at = r;
+        if (e.mc != 0u) at = __ldg(xt + (((e.mc >> 16) & 0xffu) << Nlo));
+        xv[v][j] = T(0);
+        if (((at ^ e.mc) & kCrossTest) == 0u) xv[v][j] = __ldg(x + (e.nb + at));
+      }
+#pragma unroll
+    for (int v = 0; v < U; ++v)
+#pragma unroll
+      for (int j = 0; j < B; ++j) acc[j].add(c[v][j], xv[v][j]);
+  }
+}
+
+// FP32: hi-part flips [0, n) of every block (n even), of which those below
+// nfull are real for all of them.  rb: the row's rank in bytes.
+template <typename T, typename Acc, int B, int U>
+__device__ __forceinline__ void hihi_terms(const Program& pg, int nfull, int n, uint32_t rb,
+                                           const T* __restrict__ x, Acc (&acc)[B]) {
+  using NB = RowVec<uint32_t, B>;
+  using CB = RowVec<double, B == 1 ? 1 : 2>;
+  auto add = [&](int o, const T (&xv)[B]) {
+    const CB* c = reinterpret_cast<const CB*>(pg.c + o * B);
+#pragma unroll
+    for (int j = 0; j < B; ++j) acc[j].add(c[j / 2].v[j % 2], xv[j]);
+  };
+  int o = 0;
+#pragma unroll 1
+  for (; o + U <= nfull; o += U) {
+    T xv[U][B];
+#pragma unroll
+    for (int v = 0; v < U; ++v) {
+      const NB nb = *reinterpret_cast<const NB*>(pg.nb + (o + v) * B);
+#pragma unroll
+      for (int j = 0; j < B; ++j) xv[v][j] = at_byte(x, nb.v[j] + rb);
+    }
+#pragma unroll
+    for (int v = 0; v < U; ++v) add(o + v, xv[v]);
+  }
+  constexpr int UT = 2;
+#pragma unroll 1
+  for (; o < n; o += UT) {  // null ops among them: 0 * 0
+    T xv[UT][B];
+#pragma unroll
+    for (int v = 0; v < UT; ++v) {
+      const NB nb = *reinterpret_cast<const NB*>(pg.nb + (o + v) * B);
+#pragma unroll
+      for (int j = 0; j < B; ++j) xv[v][j] = nb.v[j] != kNullOp ? at_byte(x, nb.v[j] + rb) : T(0);
+    }
+#pragma unroll
+    for (int v = 0; v < UT; ++v) add(o + v, xv[v]);
+  }
+}
+
+// FP32: crossing flips [o0, o0 + n), n a multiple of U: op o of every block
+// names the same lo bit, so one table load serves them all; the table entries
+// of the next U ops are asked for ahead.  A flip that the row does not take
+// adds c * 0.
+template <typename T, typename Acc, int B, int U>
+__device__ __forceinline__ void cross_terms(const Program& pg, int o0, int n, const uint16_t* __restrict__ xt, int Nlo,
+                                            const T* __restrict__ x, Acc (&acc)[B]) {
+  using NB = RowVec<uint32_t, B>;
+  using CB = RowVec<double, B == 1 ? 1 : 2>;
+  if (n == 0) return;
+  uint32_t at[U], next[U];
+#pragma unroll
+  for (int v = 0; v < U; ++v) next[v] = __ldg(xt + ((pg.bits[o0 + v] >> 16) << Nlo));
+#pragma unroll 1
+  for (int o = o0; o < o0 + n; o += U) {
+    T xv[U][B];
+#pragma unroll
+    for (int v = 0; v < U; ++v) {
+      at[v] = next[v];
+      const uint32_t bits = pg.bits[o + v];  // bit j: block j wants the lo bit set; bit 8 + j: clear
+      const uint32_t m = at[v] & 0x8000u ? bits : bits >> 8;
+      const uint32_t ab = (at[v] & 0x7fffu) * (uint32_t)sizeof(T);
+      const NB nb = *reinterpret_cast<const NB*>(pg.nb + (o + v) * B);
+#pragma unroll
+      for (int j = 0; j < B; ++j) xv[v][j] = m & 1u << j ? at_byte(x, nb.v[j] + ab) : T(0);
+    }
+    if (o + U < o0 + n) {
+#pragma unroll
+      for (int v = 0; v < U; ++v) next[v] = __ldg(xt + ((pg.bits[o + U + v] >> 16) << Nlo));
+    }
+#pragma unroll
+    for (int v = 0; v < U; ++v) {
+      const CB* c = reinterpret_cast<const CB*>(pg.c + (o + v) * B);
+#pragma unroll
+      for (int j = 0; j < B; ++j) acc[j].add(c[j / 2].v[j % 2], xv[v][j]);
+    }
+  }
+}
+
+// One warp: emit(position, pair) for the flips of `list` outside the lo part
+// that apply to some rows of block h, in list order from position n on:
+// kind 0 those with the condition's bits (either kind of flip), 1 the hi-part
+// flips in either direction, 2 the crossing flips in either direction.
+// Returns the position after the last.
+template <class Emit>
+__device__ __forceinline__ int walk_list(const SPair* list, int np, uint32_t h, int Nlo, uint32_t lm, int kind, int n,
+                                         Emit&& emit) {
+  const int lane = threadIdx.x & 31;
+  for (int q0 = 0; q0 < np; q0 += 32) {
+    const int q = q0 + lane;
+    bool on = false;
+    SPair e{};
+    if (q < np) {
+      e = list[q];
+      const uint32_t fhi = e.flip >> Nlo, flo = e.flip & lm;
+      on = kind == 0   ? fhi != 0u && (h & fhi) == e.cond >> Nlo
+           : kind == 1 ? flo == 0u && __popc(h & fhi) == 1
+                       : flo != 0u && fhi != 0u;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) emit(n + __popc(m & ((1u << lane) - 1u)), e);
+    n += __popc(m);
+  }
+  return n;
+}
+
+// One warp compiles block j's (hi part h) column of the program.  FP64: lists
+// of l1 and l2 ops; FP32: l1 hi-part ops, then l2 crossing ones.
+template <int B>
+__device__ __forceinline__ void compile_f64(const ApplyCtx& c, const uint32_t* __restrict__ thi, const SPair* low,
+                                            const SPair* rise, uint32_t h, int j, int l1, int l2, TileOp* ops) {
+  auto emit = [&](int at, const SPair& e) {
+    const uint32_t flo = e.flip & c.lm, nb = __ldg(thi + (h ^ (e.flip >> c.Nlo)));
+    const uint32_t v = (e.cond & c.lm) != 0u ? 1u : 0u;
+    ops[at * B + j] = flo == 0u
+                          ? TileOp{0u, nb, e.c}
+                          : TileOp{kCrossOp | ((uint32_t)(__ffs(flo) - 1) << 16) | (v << 15), nb - (v << 15), e.c};
+  };
+  const int lane = threadIdx.x & 31;
+  int n = walk_list(low, c.np, h, c.Nlo, c.lm, 0, 0, emit);
+  for (int q = n + lane; q < l1; q += 32) ops[q * B + j] = {kNullOp, 0u, 0.0};
+  n = walk_list(rise, c.np, h, c.Nlo, c.lm, 0, l1, emit);
+  for (int q = n + lane; q < l1 + l2; q += 32) ops[q * B + j] = {kNullOp, 0u, 0.0};
+}
+
+template <int B>
+__device__ __forceinline__ void compile_f32(const ApplyCtx& c, const uint32_t* __restrict__ thi, const SPair* low,
+                                            uint32_t h, int j, int l1, int l2, const Program& pg) {
+  const int lane = threadIdx.x & 31;
+  auto put = [&](int at, uint32_t nb, double cc) {  // nb: bytes (a multiple of 4), or kNullOp
+    pg.nb[at * B + j] = nb;
+    pg.c[at * B + j] = cc;
+  };
+  int n = walk_list(low, c.np, h, c.Nlo, c.lm, 1, 0, [&](int at, const SPair& e) {
+    put(at, __ldg(thi + (h ^ (e.flip >> c.Nlo))) * 4u, e.c);
+  });
+  for (int q = n + lane; q < l1; q += 32) put(q, kNullOp, 0.0);
+  n = walk_list(low, c.np, h, c.Nlo, c.lm, 2, l1, [&](int at, const SPair& e) {
+    put(at, __ldg(thi + (h ^ (e.flip >> c.Nlo))) * 4u, e.c);
+    const uint32_t b = (uint32_t)(__ffs(e.flip & c.lm) - 1);
+    // the lo bit must differ from the hi bit: set where h's is clear
+    atomicOr(pg.bits + at, b << 16 | 1u << (h & (e.flip >> c.Nlo) ? 8 + j : j));
+  });
+  for (int q = n + lane; q < l1 + l2; q += 32) put(q, 0u, 0.0);
+}
+
+// Bundle ub of the block list.
+template <typename T, typename Acc, int B, int NT, int U, int UC>
+__device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& t, int64_t ub, const T* __restrict__ x,
+                                            T* y, double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
+                                            const Program& pg, int n_ops, const SPair* low, const SPair* rise) {
+  constexpr bool kOrdered = sizeof(T) == 8;
+  using Row = RowVec<T, B>;
+  Row* rows = reinterpret_cast<Row*>(xs);
+  int nv = 0;
+  uint32_t bj[B], tf[B];
+  uint32_t h0 = 0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    const uint32_t h = __ldg(t.blk_h + ub * B + j);
+    const bool real = h != kNoBlockEntry;  // real blocks come first in a bundle
+    if (j == 0) h0 = h;
+    nv += real ? 1 : 0;
+    bj[j] = real ? __ldg(t.thi + h) : 0u;
+    tf[j] = real ? __ldg(t.tfirst + h) : 0u;
+  }
+  if (nv == 0) return;  // padding of the block list
+  const int k = c.n_up - __popc(h0);
+  const uint32_t lbase = __ldg(t.looff + k);
+  const uint32_t nk = __ldg(t.looff + k + 1) - lbase;
+  __syncthreads();  // the previous bundle is done with the program, x and red
+  if constexpr (!kOrdered) {  // collected by the blocks' warps below
+    for (int q = threadIdx.x; q < n_ops; q += NT) pg.bits[q] = 0u;
+    __syncthreads();
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < B) {
+    // the lists of all blocks are as long as the longest, a multiple of the unrolling
+    auto none = [](int, const SPair&) {};
+    int l1 = 0, l2 = 0, full = 1 << 20;
+    for (int j = 0; j < nv; ++j) {
+      const uint32_t h = __ldg(t.blk_h + ub * B + j);
+      const int n = walk_list(low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 1, 0, none);
+      l1 = max(l1, n);
+      full = min(full, n);
+      if (kOrdered || j == 0)
+        l2 = max(l2, walk_list(kOrdered ? rise : low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 2, 0, none));
+    }
+    if (nv < B) full = 0;
+    l1 = kOrdered ? (l1 + U - 1) / U * U : (l1 + 1) / 2 * 2;
+    l2 = kOrdered ? (l2 + U - 1) / U * U : (l2 + UC - 1) / UC * UC;
+    if (warp == 0 && lane == 0) {
+      sm.n1 = l1;
+      sm.n2 = l2;
+      sm.full = full;
+    }
+    if (warp < nv) {
+      const uint32_t h = __ldg(t.blk_h + ub * B + warp);
+      if constexpr (kOrdered)
+        compile_f64<B>(c, t.thi, low, rise, h, warp, l1, l2, pg.ops);
+      else
+        compile_f32<B>(c, t.thi, low, h, warp, l1, l2, pg);
+    } else {  // no such block in the bundle: null ops
+      for (int q = lane; q < l1 + l2; q += 32) {
+        if constexpr (kOrdered) {
+          pg.ops[q * B + warp] = {kNullOp, 0u, 0.0};
+        } else {
+          pg.nb[q * B + warp] = kNullOp;
+          pg.c[q * B + warp] = 0.0;
+        }
+      }
+    }
+  }
+  // x of the blocks, row by row, two rows in flight per thread
+  for (uint32_t i = threadIdx.x; i < nk; i += 2 * NT) {
+    Row a, b;
+    const bool two = i + NT < nk;
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      a.v[j] = j < nv ? __ldg(x + bj[j] + i) : T(0);
+      b.v[j] = j < nv && two ? __ldg(x + bj[j] + i + NT) : T(0);
+    }
+    rows[i] = a;
+    if (two) rows[i + NT] = b;
+  }
+  __syncthreads();
+  const int n1 = sm.n1, n2 = sm.n2, full = sm.full;
+  const unsigned char* cs = reinterpret_cast<const unsigned char*>(sm.lolo_c);
+  const uint32_t s0 = (lbase >> 5) + (uint32_t)k;
+#pragma unroll 1
+  for (uint32_t r = threadIdx.x; r < nk; r += NT) {
+    const uint16_t* xt = t.xtab + lbase + r;
+    const uint32_t s = s0 + (r >> 5);
+    const uint32_t w = __ldg(t.low_w + s);
+    const uint2* tp = t.low_e + ((size_t)s * t.low_st * 32 + lane);
+    const int wl = (int)(w & 0xffffu), wu = (int)(w >> 16);
+    Acc acc[B];
+    if (kOrdered) {
+      double dg[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) dg[j] = j < nv ? __ldg(t.dg + bj[j] + r) : 0.0;
+      hi_terms<T, Acc, B, U>(pg.ops, n1, r, xt, c.Nlo, x, acc);
+      lo_terms<T, Acc, B>(tp, wl, xs, cs, acc);
+      {
+        const Row own = rows[r];
+#pragma unroll
+        for (int j = 0; j < B; ++j) acc[j].add(dg[j], own.v[j]);
+      }
+      lo_terms<T, Acc, B>(tp + wl * 32, wu, xs, cs, acc);
+      hi_terms<T, Acc, B, U>(pg.ops + n1 * B, n2, r, xt, c.Nlo, x, acc);
+    } else {
+      const Row own = rows[r];
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if (j < nv) acc[j].add(apply::diag_fp32(t, bj[j] + r), own.v[j]);
+      hihi_terms<T, Acc, B, U>(pg, full, n1, r * (uint32_t)sizeof(T), x, acc);
+      cross_terms<T, Acc, B, UC>(pg, n1, n2, xt, c.Nlo, x, acc);
+      lo_terms<T, Acc, B>(tp, wl + wu, xs, cs, acc);
+    }
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      if (j < nv) y[bj[j] + r] = acc[j].value();
+  }
+  if (!alpha_part) return;
+  // <x, y> of every (block, tile): threads of a tile as in the tile apply,
+  // row r0 + thread + 256 i in order of i; groups of 128 threads take the
+  // halves of the tiles in turn
+  __syncthreads();  // the bundle's rows of y are written
+  const uint32_t nt = (nk + kTileRows - 1) / kTileRows;
+  const int items = nv * (int)nt;
+  constexpr int kHalf = kHvThreads / 2;
+  for (int q = threadIdx.x / kHalf; q < 2 * items; q += NT / kHalf) {
+    const int it = q >> 1;
+    const uint32_t th = threadIdx.x % kHalf + (q & 1 ? kHalf : 0);
+    const int j = it / (int)nt;
+    const uint32_t r0 = (uint32_t)(it - j * (int)nt) * kTileRows;
+    uint32_t base = bj[0];
+#pragma unroll
+    for (int b = 1; b < B; ++b) base = j == b ? bj[b] : base;
+    double dot = 0.0;
+#pragma unroll
+    for (int i = 0; i < kTileRows / kHvThreads; ++i) {
+      const uint32_t r = r0 + th + i * kHvThreads;
+      if (r < nk) dot = fma((double)rows[r].v[j], (double)y[base + r], dot);
+    }
+    for (int o = 16; o > 0; o >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, o);
+    if (lane == 0) sm.red[it][th >> 5] = dot;
+  }
+  __syncthreads();
+  for (int it = warp; it < items; it += NT / 32) {
+    const int j = it / (int)nt;
+    uint32_t first = tf[0];
+#pragma unroll
+    for (int b = 1; b < B; ++b) first = j == b ? tf[b] : first;
+    double r = lane < kHvThreads / 32 ? sm.red[it][lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+    if (lane == 0) alpha_part[first + (uint32_t)(it - j * (int)nt)] = r;
+  }
+}
+
+}  // namespace rapply
+}  // namespace aed

@@ -30,6 +30,9 @@ struct aed_handle {
   double* d_dg = nullptr;     // per-row diagonal
   uint32_t* d_ell = nullptr;  // lo-neighbour table
   size_t d_ell_n = 0;         // its capacity (entries), kept across aed_set_couplings
+  uint2* d_low_e = nullptr;   // the same in slices of 32 rows (DevTables::low_e)
+  uint32_t* d_low_w = nullptr;
+  size_t d_low_n = 0;         // pairs allocated
   uint16_t* d_xtab = nullptr;  // crossing-flip table
   double* d_partA = nullptr;  // per-tile partial sums (n_tiles)
   double* d_partB = nullptr;  // per-chunk partial sums (red_chunks(D))

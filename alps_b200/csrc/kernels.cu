@@ -18,7 +18,7 @@
 #include <type_traits>
 
 #include "apply.cuh"
-#include "apply_blocks.cuh"
+#include "apply_rows.cuh"
 #include "apply_stream.cuh"
 #include "kernels.cuh"
 #include "reduce.cuh"
@@ -43,22 +43,105 @@ __global__ void __launch_bounds__(kHvThreads, MINB) hv_kernel(const __grid_const
   for (int64_t it = blockIdx.x; it < t.n_tiles; it += gridDim.x) apply::apply_tile<T, Acc, R>(c, t, it, x, y, alpha_part, sm);
 }
 
-// y = H x over bundles of B hi blocks with x staged in shared memory (dynamic:
-// B * maxrows values).  Bundles are taken in a static round robin; the block
-// list puts the largest blocks first.
-template <typename T, typename Acc, int R, int B, int MINB>
-__global__ void __launch_bounds__(kHvThreads, MINB) hvb_kernel(const __grid_constant__ HvParams P, const DevTables t,
-                                                               const T* __restrict__ x, T* __restrict__ y,
-                                                               double* __restrict__ alpha_part) {
-  extern __shared__ __align__(16) unsigned char hvb_dyn[];
-  __shared__ bapply::BundleSmem<B> sm;
-  T* xs = bapply::carve<T, B>(P, t, hvb_dyn, sm);
-  bapply::stage_pairs<B>(P, sm);
+// y = H x over bundles with x interleaved in shared memory (apply_rows.cuh).
+// U / UC: flips (FP32: hi-part / crossing ones) whose loads go out together.
+template <typename T, typename Acc, int B, int NT, int MINB, int U, int UC>
+__global__ void __launch_bounds__(NT, MINB) hvr_kernel(const __grid_constant__ HvParams P, const DevTables t,
+                                                       const T* __restrict__ x, T* y,
+                                                       double* __restrict__ alpha_part) {
+  extern __shared__ __align__(16) unsigned char hvr_dyn[];
+  __shared__ rapply::RowsSmem sm;
+  constexpr int kRow = sizeof(T) * B;
+  const int n_ops = rapply::prog_ops((int)sizeof(T), P.n_pairs, P.n_lolo);
+  unsigned char* p = hvr_dyn + (((size_t)(t.maxrows + 1) * kRow + 15) & ~(size_t)15);
+  rapply::Program pg;
+  pg.ops = reinterpret_cast<apply::TileOp*>(p);
+  pg.c = reinterpret_cast<double*>(p);
+  p += (size_t)B * n_ops * sizeof(double);
+  pg.nb = reinterpret_cast<uint32_t*>(p);
+  p += (size_t)B * n_ops * (sizeof(apply::TileOp) - sizeof(double));
+  pg.bits = reinterpret_cast<uint32_t*>(p);
+  p += (size_t)n_ops * 16;
+  apply::SPair* low = reinterpret_cast<apply::SPair*>(p);
+  apply::SPair* rise = low + P.n_pairs;
+  for (int q = threadIdx.x; q < P.n_pairs; q += NT) {
+    const PairTerm a = P.low[q], b = P.rise[q];
+    low[q] = {a.mhi | a.mlo, a.mhi, a.c};
+    rise[q] = {b.mhi | b.mlo, b.mlo, b.c};
+  }
+  for (int q = threadIdx.x; q <= P.n_lolo; q += NT) sm.lolo_c[q] = q < P.n_lolo ? P.lolo_c[q] : 0.0;
+  if (threadIdx.x == 0) {
+    rapply::RowVec<T, B> z;
+#pragma unroll
+    for (int j = 0; j < B; ++j) z.v[j] = T(0);
+    reinterpret_cast<rapply::RowVec<T, B>*>(hvr_dyn)[t.maxrows] = z;
+  }
   const apply::ApplyCtx c = apply::ctx_of(P);
   const int64_t nb = t.n_blk / B;
-  int rc = 0;
   for (int64_t ub = blockIdx.x; ub < nb; ub += gridDim.x)
-    bapply::apply_bundle<T, Acc, R, B>(c, t, ub, x, y, alpha_part, sm, xs, rc);
+    rapply::rows_bundle<T, Acc, B, NT, U, UC>(c, t, ub, x, y, alpha_part, sm, hvr_dyn, pg, n_ops, low, rise);
+}
+
+// The lo-neighbour table: one thread per lo state, its flips inserted in order
+// of their target's rank (no two share one).
+__global__ void __launch_bounds__(128) lo_table_kernel(const __grid_constant__ HvParams P, const DevTables t,
+                                                       uint32_t* __restrict__ ell) {
+  const uint32_t i = blockIdx.x * 128u + threadIdx.x;
+  if (i >= 1u << t.Nlo) return;
+  const uint32_t l = t.lolist[i];
+  const int k = __popc(l);
+  const uint32_t base = t.looff[k], nk = t.looff[k + 1] - base;
+  uint32_t* E = ell + (size_t)t.ell_w * base + (i - base);
+  int n = 0;
+  uint32_t q = 0;
+  for (int a = 0; a < P.n_pairs; ++a) {
+    if ((P.low[a].mhi >> t.Nlo) != 0u) continue;
+    const uint32_t f = P.low[a].mhi | P.low[a].mlo, b = l & f;
+    if (b != 0u && b != f) {
+      const uint32_t v = t.tlo[l ^ f];
+      int e = n++;
+      for (; e > 0; --e) {
+        const uint32_t w = E[(size_t)(e - 1) * nk];
+        if ((w & 0xffffu) < v) break;
+        E[(size_t)e * nk] = w;
+      }
+      E[(size_t)e * nk] = v | q << 16;
+    }
+    ++q;
+  }
+  for (; n < t.ell_w; ++n) E[(size_t)n * nk] = kEllPad;
+}
+
+// The sliced lo-neighbour table: one warp per slice of 32 rows of a class.
+__global__ void __launch_bounds__(128) lo_slices_kernel(const DevTables t, uint32_t pad, uint2* __restrict__ e,
+                                                        uint32_t* __restrict__ w) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t s = blockIdx.x * 4u + (threadIdx.x >> 5);
+  int k = t.Nlo;  // the class of slice s
+  while (k > 0 && (t.looff[k] >> 5) + (uint32_t)k > s) --k;
+  const uint32_t base = t.looff[k], nk = t.looff[k + 1] - base;
+  const uint32_t r0 = (s - (base >> 5) - (uint32_t)k) * 32u, r = r0 + lane;
+  if (r0 >= nk) return;  // a slice number that no class uses
+  const uint32_t* E = t.ell + (size_t)t.ell_w * base + r;
+  int nl = 0, nu = 0;
+  if (r < nk)
+    for (int i = 0; i < t.ell_w; ++i) {
+      const uint32_t v = E[(size_t)i * nk];
+      if (v == kEllPad) break;
+      (v & 0xffffu) < r ? ++nl : ++nu;
+    }
+  const int wl = (__reduce_max_sync(0xffffffffu, nl) + 1) / 2, wu = (__reduce_max_sync(0xffffffffu, nu) + 1) / 2;
+  if (lane == 0) w[s] = (uint32_t)wl | (uint32_t)wu << 16;
+  uint32_t* o = reinterpret_cast<uint32_t*>(e + ((size_t)s * t.low_st * 32 + lane));
+  for (int i = 0; i < 2 * (wl + wu); ++i) {  // position i of the slice: entry i & 1 of pair i >> 1
+    const int j = i < 2 * wl ? i : i - 2 * wl + nl;
+    uint32_t v = pad;
+    if (r < nk && (i < 2 * wl ? i < nl : j < nl + nu)) {
+      const uint32_t x = E[(size_t)j * nk];
+      v = (x & 0xffffu) << 4 | ((x >> 16) * 8u) << 20;
+    }
+    o[(size_t)(i >> 1) * 64 + (i & 1)] = v;
+  }
 }
 
 // y = H x with the flips' x segments staged by bulk copies (apply_stream.cuh).
@@ -379,19 +462,23 @@ int launch_ritz_combine(const float* V, int64_t ld, int m, const double* coef, d
 }
 
 // ---- apply variants -------------------------------------------------------------
-// Tile apply (apply.cuh): R rows per thread, MINB CTAs per SM.  Bundle apply
-// (apply_blocks.cuh): B hi blocks per CTA with x in shared memory.
+// Tile apply (apply.cuh), rR rows per thread and bM CTAs per SM: it takes any
+// sector and any vectors.  Stream apply (apply_stream.cuh).  Rows apply
+// (apply_rows.cuh): bytes of an interleaved row (of ROW / sizeof(T) blocks),
+// threads per CTA.  The autotuner times the first tile apply and the rows
+// applies, which won on every sector measured (12 to 30 sites, chains, ladders
+// and square lattices); the other shapes are there to be selected.
 struct HvVariant {
-  int B, R, minb;  // B = 0: tile apply; B = -1: stream apply (R = rows per thread, minb = own-x buffers)
+  int kind;  // 0: tile, 1: stream, 2: rows
   const char* name;
 };
 constexpr HvVariant kVariants[] = {
-    {0, 4, 6, "r4b6"},      {0, 4, 5, "r4b5"},      {0, 4, 4, "r4b4"},      {0, 2, 8, "r2b8"},
-    {0, 2, 6, "r2b6"},      {0, 8, 3, "r8b3"},      {1, 4, 3, "blk1r4b3"},  {2, 2, 4, "blk2r2b4"},
-    {2, 4, 2, "blk2r4b2"},  {2, 2, 3, "blk2r2b3"},  {1, 4, 4, "blk1r4b4"},  {1, 2, 4, "blk1r2b4"},
-    {-1, 14, 2, "str14o2"}, {-1, 14, 1, "str14o1"}, {-1, 26, 2, "str26o2"}, {-1, 26, 1, "str26o1"},
-    {-1, 14, 1, "str14w"},  {-1, 26, 1, "str26w"},  // FP32: own x widened once
+    {0, "r4b6"}, {0, "r4b5"}, {0, "r4b4"}, {0, "r2b8"}, {0, "r2b6"}, {0, "r8b3"},
+    {2, "row16n256"}, {2, "row16n384"}, {2, "row16n512"}, {2, "row16n1024"},
+    {2, "row8n256"}, {2, "row8n512"}, {2, "row8n1024"},
+    {1, "str14o2"}, {1, "str14o1"}, {1, "str26o2"}, {1, "str26o1"}, {1, "str14w"}, {1, "str26w"},
 };
+constexpr int kSmallVariant = 12;  // row8n1024: the most threads on each of the most CTAs
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 
 // Launch shapes are computed once per kernel (and per shared-memory size or
@@ -438,13 +525,19 @@ int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* 
   return check_launch("hv_kernel");
 }
 
-// Bundle apply: grid from the occupancy at this sector's dynamic shared
-// memory (sectors of one process share a few sizes).
-template <typename T, typename Acc, int R, int B, int MINB>
-int launch_bundle(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
-  if (!t.blk_h || t.maxrows <= 0) return kVariantNotApplicable;
-  const size_t dyn = bapply::bundle_smem_bytes<T>(B, t.maxrows, P.n_pairs, P.n_lolo);
-  auto kern = hvb_kernel<T, Acc, R, B, MINB>;
+// Rows apply: bundles of ROW / sizeof(T) blocks; the grid from the occupancy
+// at this sector's dynamic shared memory (sectors of one process share a few
+// sizes).  Not for couplings that are not finite: a flip that a row does not
+// take adds c * 0.
+// Four flips of all blocks in flight (FP32 crossing flips: two) fill the 64
+// registers of 1024 threads per SM without a spill; eight, or four crossing
+// ones, spill and were 5-25 % slower on L=28 and 6x5.
+template <typename T, typename Acc, int ROW, int NT, int MINB>
+int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
+  constexpr int B = ROW / (int)sizeof(T);
+  if (!t.blk_h || !t.low_e || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
+  const size_t dyn = rapply::rows_smem_bytes(ROW, B, t.maxrows, P.n_pairs, P.n_lolo);
+  auto kern = hvr_kernel<T, Acc, B, NT, MINB, 4, 2>;
   static int limit_rc = -1;
   static size_t static_bytes = 0;
   static std::map<size_t, int> grids;  // dyn -> grid (0: does not fit)
@@ -460,7 +553,7 @@ int launch_bundle(const HvParams& P, const DevTables& t, const T* x, T* y, doubl
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
       if (limit_rc == AED_OK && static_bytes + dyn <= (size_t)optin)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHvThreads, dyn);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, dyn);
       it = grids.emplace(dyn, per_sm < 1 ? 0 : num_sms() * per_sm).first;
     }
     grid = it->second;
@@ -470,8 +563,8 @@ int launch_bundle(const HvParams& P, const DevTables& t, const T* x, T* y, doubl
   const int64_t nb = t.n_blk / B;
   if (g > nb) g = nb;
   if (g < 1) return AED_OK;
-  kern<<<(unsigned)g, kHvThreads, dyn, st>>>(P, t, x, y, alpha_part);
-  return check_launch("hvb_kernel");
+  kern<<<(unsigned)g, NT, dyn, st>>>(P, t, x, y, alpha_part);
+  return check_launch("hvr_kernel");
 }
 
 // Stream apply: one CTA per SM with OB own-x buffers and as many ring stages
@@ -479,6 +572,7 @@ int launch_bundle(const HvParams& P, const DevTables& t, const T* x, T* y, doubl
 // sectors whose blocks need more than U rows per thread, to lo parts under
 // 8 bits (the crossing-table rows must be 16-byte multiples), or to vectors
 // that are not 16-byte aligned (bulk copies).
+constexpr size_t align16(size_t n) { return (n + 15) & ~(size_t)15; }
 struct StreamShape {
   sapply::StreamCfg cfg{};
   size_t dyn = 0;
@@ -511,10 +605,10 @@ int launch_stream(int OB, const HvParams& P, const DevTables& t, const T* x, T* 
       int dev = 0, optin = 0;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      n.cfg.own_bytes = (uint32_t)bapply::bundle_align16((size_t)t.maxrows * sizeof(T) + 32);
+      n.cfg.own_bytes = (uint32_t)align16((size_t)t.maxrows * sizeof(T) + 32);
       n.cfg.xoff = n.cfg.own_bytes;
-      n.cfg.stage_bytes = n.cfg.xoff + (uint32_t)bapply::bundle_align16((size_t)t.maxrows * 2 + 32);
-      const uint32_t ownd_bytes = kOwnD ? (uint32_t)bapply::bundle_align16((size_t)t.maxrows * 8 + 32) : 0u;
+      n.cfg.stage_bytes = n.cfg.xoff + (uint32_t)align16((size_t)t.maxrows * 2 + 32);
+      const uint32_t ownd_bytes = kOwnD ? (uint32_t)align16((size_t)t.maxrows * 8 + 32) : 0u;
       n.cfg.ownd_off = (uint32_t)OB * n.cfg.own_bytes;
       n.cfg.ring_off = n.cfg.ownd_off + ownd_bytes;
       const int64_t avail = (int64_t)optin - (int64_t)static_bytes - 1024;
@@ -553,27 +647,26 @@ int launch_hv_t(int v, const HvParams& P, const DevTables& t, const T* x, T* y, 
     case 3: return launch_one<T, Acc, 2, 8>(P, t, x, y, alpha_part, st);
     case 4: return launch_one<T, Acc, 2, 6>(P, t, x, y, alpha_part, st);
     case 5: return launch_one<T, Acc, 8, 3>(P, t, x, y, alpha_part, st);
-    case 6: return launch_bundle<T, Acc, 4, 1, 3>(P, t, x, y, alpha_part, st);
-    case 7: return launch_bundle<T, Acc, 2, 2, 4>(P, t, x, y, alpha_part, st);
-    case 8: return launch_bundle<T, Acc, 4, 2, 2>(P, t, x, y, alpha_part, st);
-    case 9: return launch_bundle<T, Acc, 2, 2, 3>(P, t, x, y, alpha_part, st);
-    case 10: return launch_bundle<T, Acc, 4, 1, 4>(P, t, x, y, alpha_part, st);
-    case 11: return launch_bundle<T, Acc, 2, 1, 4>(P, t, x, y, alpha_part, st);
-    case 12: return launch_stream<T, Acc, 14, false>(2, P, t, x, y, alpha_part, st);
-    case 13: return launch_stream<T, Acc, 14, false>(1, P, t, x, y, alpha_part, st);
-    case 14: return launch_stream<T, Acc, 26, false>(2, P, t, x, y, alpha_part, st);
-    case 15: return launch_stream<T, Acc, 26, false>(1, P, t, x, y, alpha_part, st);
-    case 16: return launch_stream<T, Acc, 14, true>(1, P, t, x, y, alpha_part, st);
-    case 17: return launch_stream<T, Acc, 26, true>(1, P, t, x, y, alpha_part, st);
+    case 6: return launch_rows<T, Acc, 16, 256, 4>(P, t, x, y, alpha_part, st);
+    case 7: return launch_rows<T, Acc, 16, 384, 3>(P, t, x, y, alpha_part, st);
+    case 8: return launch_rows<T, Acc, 16, 512, 2>(P, t, x, y, alpha_part, st);
+    case 9: return launch_rows<T, Acc, 16, 1024, 1>(P, t, x, y, alpha_part, st);
+    case 10: return launch_rows<T, Acc, 8, 256, 4>(P, t, x, y, alpha_part, st);
+    case 11: return launch_rows<T, Acc, 8, 512, 2>(P, t, x, y, alpha_part, st);
+    case 12: return launch_rows<T, Acc, 8, 1024, 1>(P, t, x, y, alpha_part, st);
+    case 13: return launch_stream<T, Acc, 14, false>(2, P, t, x, y, alpha_part, st);
+    case 14: return launch_stream<T, Acc, 14, false>(1, P, t, x, y, alpha_part, st);
+    case 15: return launch_stream<T, Acc, 26, false>(2, P, t, x, y, alpha_part, st);
+    case 16: return launch_stream<T, Acc, 26, false>(1, P, t, x, y, alpha_part, st);
+    case 17: return launch_stream<T, Acc, 14, true>(1, P, t, x, y, alpha_part, st);
+    case 18: return launch_stream<T, Acc, 26, true>(1, P, t, x, y, alpha_part, st);
     default: return fail(AED_ERR_INVALID, "unknown apply variant");
   }
 }
 
 int hv_num_variants() { return kNumVariants; }
-// The stream applies trail the bundle applies on every sector measured (1.9 to
-// 2.3 times slower: one CTA per SM leaves too few warps to issue), so the
-// autotuner does not time them; AED_HV_VARIANT still selects them.
-bool hv_variant_tuned(int v) { return v >= 0 && v < kNumVariants && kVariants[v].B >= 0; }
+bool hv_variant_tuned(int v) { return v == 0 || (v > 0 && v < kNumVariants && kVariants[v].kind == 2); }
+int hv_small_variant() { return kSmallVariant; }
 const char* hv_variant_name(int v) { return (v >= 0 && v < kNumVariants) ? kVariants[v].name : "?"; }
 
 int launch_hv_f64(int variant, const HvParams& P, const DevTables& t, const double* x, double* y,
@@ -589,6 +682,18 @@ int launch_hv_f32(int variant, const HvParams& P, const DevTables& t, const floa
   }();
   if (twosum) return launch_hv_t<float, AccTwoSum32>(variant, P, t, x, y, alpha_part, st);
   return launch_hv_t<float, AccWide32>(variant, P, t, x, y, alpha_part, st);
+}
+
+int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaStream_t st) {
+  if (t.ell_w == 0) return AED_OK;
+  lo_table_kernel<<<((1u << t.Nlo) + 127) / 128, 128, 0, st>>>(P, t, ell);
+  return check_launch("lo_table_kernel");
+}
+
+int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st) {
+  const uint32_t pad = (uint32_t)pad_row << 4 | ((uint32_t)pad_c * 8u) << 20;
+  lo_slices_kernel<<<(unsigned)((lo_slices(t.Nlo) + 3) / 4), 128, 0, st>>>(t, pad, e, w);
+  return check_launch("lo_slices_kernel");
 }
 
 int launch_diag_table(const HvParams& P, const DevTables& t, double* dg, cudaStream_t st) {

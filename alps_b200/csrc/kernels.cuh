@@ -18,13 +18,13 @@ struct DevTables {
   const uint32_t* tile_h;  // n_tiles
   const uint32_t* tile_r;  // n_tiles
   const double* dg;        // D: diagonal M(i,i) of every row
-  const uint32_t* ell;     // lo-neighbour table (build_lo_table), ell_w entries per lo state
+  const uint32_t* ell;     // lo-neighbour table (launch_lo_table), ell_w entries per lo state
   const uint16_t* xtab = nullptr;  // crossing-flip table (build_cross_table), Nlo x 2^Nlo
   int ell_w;
   int64_t n_tiles;
   int64_t D;
   int Nlo, Nhi, n_up;
-  // block list of the bundle apply (build_block_list): hi blocks grouped by
+  // block list of the bundle and rows applies (build_block_list): hi blocks grouped by
   // lo popcount, each group padded with kNoBlock to a multiple of kBundleMax
   const uint32_t* blk_h = nullptr;   // n_blk
   const uint32_t* tfirst = nullptr;  // 2^Nhi: index of the first tile of each hi block
@@ -35,6 +35,14 @@ struct DevTables {
   // FP32 handles: M(i,i) rounded to FP32 (D floats), read by the FP32 applies
   // in place of dg (half its bytes; the FP64 applies keep dg)
   const float* dgf = nullptr;
+  // the lo-neighbour table in slices of 32 rows (launch_lo_slices): slice
+  // (looff[k] >> 5) + k + (r >> 5) of row r of class k holds low_st pairs of
+  // entries per row, pair p of lane l at (slice * low_st + p) * 32 + l;
+  // low_w: pairs to smaller targets | pairs to larger ones << 16.  An entry is
+  // 16 x target rank | (8 x coupling index) << 20
+  const uint2* low_e = nullptr;
+  const uint32_t* low_w = nullptr;
+  int low_st = 0;
 };
 
 constexpr int kHvThreads = 256;
@@ -52,8 +60,25 @@ int launch_hv_f32(int variant, const HvParams& P, const DevTables& t, const floa
 constexpr int kVariantNotApplicable = 2;
 int hv_num_variants();
 const char* hv_variant_name(int v);
-// Whether the autotuner times variant v (the stream applies are left out).
+// The variant of sectors too small to time.
+int hv_small_variant();
+// Whether the autotuner times variant v.
 bool hv_variant_tuned(int v);
+
+// The lo-neighbour table of P's flips into ell (t.ell_w = P.n_lolo entries per
+// lo state): for every lo state l (rank r within its popcount class k), the
+// flips with both bits in the lo part that apply to l, as (target rank r' =
+// tlo[l ^ flip]) | (flip index << 16), sorted by r' and padded with kEllPad.
+// Entry e of row r of class k sits at ell_w * looff[k] + e * C(Nlo, k) + r
+// (coalesced across consecutive rows).
+int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaStream_t st);
+
+// The sliced lo-neighbour table from t.ell (t.low_e, t.low_w, t.low_st name
+// its arrays): pad_row is the rank of padding entries (a staged row of zeros),
+// pad_c their coupling index (0.0).
+inline int lo_slice_pairs(int ell_w) { return 2 * ((ell_w + 1) / 2) + 1; }  // each part at most ell_w entries
+inline size_t lo_slices(int Nlo) { return ((size_t)1 << Nlo) / 32 + (size_t)Nlo + 2; }
+int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st);
 
 // per-row diagonal table (once per handle)
 int launch_diag_table(const HvParams& P, const DevTables& t, double* dg, cudaStream_t st);

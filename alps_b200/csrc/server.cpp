@@ -186,7 +186,8 @@ int sector_acquire(aed_server* s, int N, int n_up, Sector** out) {
   std::vector<uint16_t> xt;
   build_tiles(sec.tab, kHvTileRows, th, tr, &tf);
   build_cross_table(sec.tab, xt);
-  build_block_list(sec.tab, sec.blk, &sec.maxrows);
+  static const HvParams no_pairs{};  // the sector's list serves any couplings
+  build_block_list(sec.tab, no_pairs, 1, sec.blk, &sec.maxrows);
   sec.n_tiles = (int64_t)th.size();
   const size_t nhi = sec.tab.thi.size(), nlo = sec.tab.tlo.size(), nof = sec.tab.looff.size();
   if ((rc = dmalloc(s, (void**)&sec.thi, nhi * 4)) || (rc = dmalloc(s, (void**)&sec.tlo, nlo * 2)) ||
@@ -314,17 +315,11 @@ int admit(aed_server* s, int k, const std::shared_ptr<Request>& r) {
   t.n_up = sec->tab.n_up;
   t.dg = (const double*)pdg;
   {
-    std::vector<uint32_t> ell;
-    int W = 0;
-    build_lo_table(sec->tab, P, ell, &W);
     void* pe = nullptr;
-    if ((rc = take(&pe, ell.size() * 4 + 4))) return rc;
-    if (!ell.empty()) {
-      cudaMemcpyAsync(pe, ell.data(), ell.size() * 4, cudaMemcpyHostToDevice, s->stream);
-      AED_CUDA_TRY(cudaStreamSynchronize(s->stream));  // host vector goes out of scope
-    }
+    t.ell_w = P.n_lolo;
+    if ((rc = take(&pe, ((size_t)t.ell_w << t.Nlo) * 4 + 4))) return rc;
     t.ell = (const uint32_t*)pe;
-    t.ell_w = W;
+    if ((rc = launch_lo_table(P, t, (uint32_t*)pe, s->stream))) return rc;
   }
   if ((rc = launch_diag_table(P, t, (double*)pdg, s->stream))) return rc;
   I.D = D;

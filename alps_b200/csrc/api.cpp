@@ -148,7 +148,9 @@ void release(aed_handle* h) {
                   (void*)h->d_reps, (void*)h->d_norm, (void*)h->d_mdiag, (void*)h->d_map, (void*)h->d_sthi,
                   (void*)h->d_stlo, (void*)h->d_slolist, (void*)h->d_slooff, (void*)h->d_sblk_hi,
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
-                  (void*)h->d_slol, (void*)h->d_low_e, (void*)h->d_low_w})
+                  (void*)h->d_slol, (void*)h->d_srblk, (void*)h->d_stfirst, (void*)h->d_slow_w, (void*)h->d_sxtab,
+                  (void*)h->d_slow_e, (void*)h->d_slokey, (void*)h->d_srprog, (void*)h->d_slodiag, (void*)h->d_sxoff, (void*)h->d_sxdiag, (void*)h->d_scross,
+                  (void*)h->d_low_e, (void*)h->d_low_w})
     mem_dev_free(p, h->stream);
   mom_rows_free(h->mrows, h->stream);
   delete h->mp;
@@ -381,6 +383,10 @@ int handle_hv(aed_handle* h, bool f32, const void* x, void* y, double* alpha_par
   if (h->gen && h->mom)
     return launch_spin_mom_hv(*h->sp, *h->mp, h->sdev, h->spin_mom_tables(), (const double*)x, (double*)y,
                               alpha_part, h->stream);
+  if (h->gen && h->sdev.rblk) {
+    const int rc = launch_spin_rows(*h->sp, h->sdev, h->srow_vals, (const double*)x, (double*)y, alpha_part, h->stream);
+    if (rc != kSpinRowsNone) return rc;
+  }
   if (h->gen) return launch_spin_hv(*h->sp, h->sdev, (const double*)x, (double*)y, alpha_part, h->stream);
   if (h->mom)
     return launch_mom_hv(*h->mp, h->dt, h->mom_tables(), (const double*)x, (double*)y, alpha_part, h->stream);
@@ -768,14 +774,87 @@ void spin_couplings(const Model& m, SpinParams& p) {
   spin_set_couplings(m.s1, m.s2, m.jz, m.jxy, m.kq, m.site_h, m.site_d, m.N, p);
 }
 
+// The tables of the rows apply of a spin-S Sz-sector handle for its current
+// couplings; *built false: the form has none, or there is no memory for them
+// (the tile apply then walks the bonds).  Filled on the handle's stream and
+// waited for.
+int spin_rows_tables(aed_handle* h, bool* built) {
+  SpinDev& t = h->sdev;
+  *built = false;
+  t.rblk = nullptr;
+  // AED_SPIN_ROWS=0 keeps the tile apply (a test compares the two)
+  if (const char* e = std::getenv("AED_SPIN_ROWS"); e && e[0] == '0') return AED_OK;
+  SpinRowsPlan r;
+  if (!spin_rows_plan(*h->sp, t, r)) return AED_OK;
+  const size_t slices = spin_low_slices(t), pairs = slices * (size_t)t.low_st * 32;
+  const size_t xt = (size_t)t.n_xtab * (2 * t.d - 1) * t.n_lo;
+  auto grow = [&](auto** p, size_t n) {
+    mem_dev_free(*p, h->stream);
+    *p = nullptr;
+    return mem_dev_alloc_n(p, n) == AED_OK;
+  };
+  bool ok = h->d_srblk && h->d_stfirst;
+  if (ok && (!h->d_slow_w || pairs > h->slow_n)) {
+    h->slow_n = 0;
+    ok = grow(&h->d_slow_e, pairs) && grow(&h->d_slow_w, slices) && grow(&h->d_slodiag, (size_t)t.n_lo) &&
+         grow(&h->d_slokey, (size_t)t.n_lo);
+    if (ok) h->slow_n = pairs;
+  }
+  if (ok && xt > h->sxtab_n) {
+    h->sxtab_n = 0;
+    ok = grow(&h->d_sxtab, xt);
+    if (ok) h->sxtab_n = xt;
+  }
+  if (ok && r.cross.size() > h->scross_n) {
+    h->scross_n = 0;
+    ok = grow(&h->d_scross, r.cross.size()) && grow(&h->d_sxoff, r.xoff.size()) && grow(&h->d_sxdiag, r.xdiag.size());
+    if (ok) h->scross_n = r.cross.size();
+  }
+  const size_t progs = spin_prog_bytes(t);
+  if (ok && progs > h->srprog_n) {
+    h->srprog_n = 0;
+    ok = grow(&h->d_srprog, progs);
+    if (ok) h->srprog_n = progs;
+  }
+  if (!ok) return AED_OK;
+  if (!r.cross.empty()) {
+    AED_CUDA_TRY(cudaMemcpyAsync(h->d_scross, r.cross.data(), r.cross.size() * sizeof(SpinCross),
+                                 cudaMemcpyHostToDevice, h->stream));
+    AED_CUDA_TRY(cudaMemcpyAsync(h->d_sxoff, r.xoff.data(), r.xoff.size() * 8, cudaMemcpyHostToDevice, h->stream));
+    AED_CUDA_TRY(cudaMemcpyAsync(h->d_sxdiag, r.xdiag.data(), r.xdiag.size() * 8, cudaMemcpyHostToDevice, h->stream));
+  }
+  int rc = launch_spin_rows_tables(*h->sp, t, r, h->d_slow_e, h->d_slow_w, h->d_slodiag, h->d_slokey, h->d_sxtab,
+                                         h->stream);
+  if (rc) return rc;
+  t.rblk = h->d_srblk;
+  t.tfirst = h->d_stfirst;
+  t.low_e = h->d_slow_e;
+  t.low_w = h->d_slow_w;
+  t.lodiag = h->d_slodiag;
+  t.lokey = h->d_slokey;
+  t.cross = h->d_scross;
+  t.xtab = h->d_sxtab;
+  t.xoff = h->d_sxoff;
+  t.xdiag = h->d_sxdiag;
+  t.rprog = h->d_srprog;
+  h->srow_vals = r.vals;
+  if ((rc = launch_spin_progs(*h->sp, t, h->d_srprog, h->stream))) return rc;
+  AED_CUDA_TRY(cudaStreamSynchronize(h->stream));  // r goes out of scope
+  *built = true;
+  return AED_OK;
+}
+
 // The lo table of a spin-S Sz-sector handle for its current couplings (none
 // for a momentum sector, whose apply walks representatives, or a form
 // without one); filled on the handle's stream and waited for.
 int spin_lo_table(aed_handle* h) {
   SpinDev& t = h->sdev;
+  t.lol = nullptr;
+  bool rows = false;
+  if (int rc = h->mom ? AED_OK : spin_rows_tables(h, &rows)) return rc;
+  if (rows) return AED_OK;  // the rows apply takes the sector
   size_t bytes = h->mom ? 0 : spin_lo_table_bytes(*h->sp, t);
   if (bytes > (size_t(1) << 30)) bytes = 0;  // a bond list this long walks the lo words instead
-  t.lol = nullptr;
   if (bytes == 0) return AED_OK;
   if (bytes > h->slol_bytes) {
     mem_dev_free(h->d_slol, h->stream);
@@ -792,7 +871,9 @@ int spin_lo_table(aed_handle* h) {
 
 }  // namespace
 
-int aed_create_spin(const aed_model_desc* model, int32_t two_s, int device, aed_handle** out) {
+namespace {
+// sz_apply false: a momentum sector's handle, which takes no product of the Sz sector.
+int create_spin(const aed_model_desc* model, int32_t two_s, int device, bool sz_apply, aed_handle** out) {
   if (!out || !model) return fail(AED_ERR_INVALID, "NULL argument");
   *out = nullptr;
   int ndev = 0;
@@ -824,6 +905,7 @@ int aed_create_spin(const aed_model_desc* model, int32_t two_s, int device, aed_
   h->sp = new SpinParams();
   spin_transitions(two_s, *h->sp);
   spin_couplings(h->model, *h->sp);
+  if (sz_apply) spin_block_list(*h->sp, tb);
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     release(h);
@@ -834,7 +916,8 @@ int aed_create_spin(const aed_model_desc* model, int32_t two_s, int device, aed_
     const std::vector<uint32_t>* v;
   } ups[] = {{&h->d_sthi, &tb.thi},         {&h->d_stlo, &tb.tlo},         {&h->d_slolist, &tb.lolist},
              {&h->d_slooff, &tb.looff},     {&h->d_sblk_hi, &tb.blk_hi},   {&h->d_sblk_off, &tb.blk_off},
-             {&h->d_stile_blk, &tb.tile_blk}, {&h->d_stile_r, &tb.tile_r}};
+             {&h->d_stile_blk, &tb.tile_blk}, {&h->d_stile_r, &tb.tile_r}, {&h->d_srblk, &tb.rblk},
+             {&h->d_stfirst, &tb.tfirst}};
   for (auto& u : ups) {
     if ((rc = mem_dev_alloc_n(u.d, u.v->size() + 1))) {
       release(h);
@@ -875,13 +958,20 @@ int aed_create_spin(const aed_model_desc* model, int32_t two_s, int device, aed_
   t.d = tb.d;
   t.T = tb.T;
   t.n_lo = (int64_t)tb.lolist.size();
+  t.n_rblk = (int64_t)tb.rblk.size();
+  t.maxrows = tb.maxrows;
   h->dim = h->vlen = D;
-  if ((rc = spin_lo_table(h))) {
+  if (sz_apply && (rc = spin_lo_table(h))) {
     release(h);
     return rc;
   }
   *out = h;
   return AED_OK;
+}
+}  // namespace
+
+int aed_create_spin(const aed_model_desc* model, int32_t two_s, int device, aed_handle** out) {
+  return create_spin(model, two_s, device, true, out);
 }
 
 int aed_create_spin_momentum(const aed_model_desc* model, int32_t two_s, const aed_translations* tr, int device,
@@ -892,7 +982,7 @@ int aed_create_spin_momentum(const aed_model_desc* model, int32_t two_s, const a
   int rc = momentum_params(model->n_sites, tr, *mpp);
   if (rc) return rc;
   aed_handle* h = nullptr;
-  if ((rc = aed_create_spin(model, two_s, device, &h))) return rc;
+  if ((rc = create_spin(model, two_s, device, false, &h))) return rc;
   {
     std::vector<int> maps(tr->site_map, tr->site_map + (size_t)tr->n_trans * model->n_sites);
     if ((rc = translation_invariant(h->model, tr->n_trans, maps.data()))) {
@@ -903,10 +993,6 @@ int aed_create_spin_momentum(const aed_model_desc* model, int32_t two_s, const a
   DeviceGuard g(device);
   h->mom = true;
   h->mp = mpp.release();
-  h->sdev.lol = nullptr;  // the momentum apply walks representatives, not tiles
-  mem_dev_free(h->d_slol, h->stream);
-  h->d_slol = nullptr;
-  h->slol_bytes = 0;
   // the Sz sector's partial-sum arrays give way to the momentum sector's
   mem_dev_free(h->d_partA, h->stream);
   mem_dev_free(h->d_partB, h->stream);

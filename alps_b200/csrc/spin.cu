@@ -16,6 +16,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -261,6 +263,7 @@ struct SpinShared {
 // word looks up one table and only a bond across the split looks up both.
 template <int D, int MO>
 struct SpinTabShared {
+  static constexpr int kD = D, kMO = MO;
   double dg[kSpinMaxCls * D * D];
   double ov[kSpinMaxCls * D * D * MO];
   uint32_t pk[kSpinMaxCls * D * D];
@@ -289,6 +292,12 @@ struct TileHiOf<SpinTabShared<D, MO>> {
 
 // Bond record flags: bit 0 site i in hi, bit 1 site j in hi.
 __device__ __forceinline__ int bond_side(const int4& b) { return (b.y >> 16) & 3; }
+
+}  // namespace
+}  // namespace aed
+#include "spin_rows.cuh"
+namespace aed {
+namespace {
 
 __device__ __forceinline__ int stage_site_terms(const SpinParams& p, int N, int d, double* sdg) {
   int nz = 0;
@@ -601,6 +610,108 @@ __global__ void __launch_bounds__(kSpinThreads) spin_hv_kernel(const __grid_cons
       if (threadIdx.x == 0) alpha_part[it] = tot;
     }
   }
+}
+
+// The rows apply (spin_rows.cuh).
+template <int D, int B, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) spin_rows_kernel(const SpinDev t, const __grid_constant__ SpinRowVals vals,
+                                                             const double* __restrict__ x, double* y,
+                                                             double* __restrict__ alpha_part) {
+  extern __shared__ __align__(16) unsigned char spin_dyn[];
+  __shared__ SpinRowsSmem sm;
+  const size_t pb = spin_block_prog_bytes(D, t.n_hh, t.n_x, t.n_key);
+  unsigned char* prog = spin_dyn + (((size_t)(t.maxrows + 1) * 8 * B + 15) & ~(size_t)15);
+  const int64_t nb = t.n_rblk / B;
+  if ((int64_t)blockIdx.x < nb) spin_fetch<NT>(t, blockIdx.x, prog, (size_t)B * pb);
+  for (int q = threadIdx.x; q <= vals.n; q += NT) sm.val[q] = q < vals.n ? vals.v[q] : 0.0;
+  if (threadIdx.x < B) reinterpret_cast<double*>(spin_dyn)[(size_t)t.maxrows * B + threadIdx.x] = 0.0;
+  int w = 0;
+  for (int64_t ub = blockIdx.x; ub < nb; ub += gridDim.x, w ^= 1)
+    spin_rows_bundle<D, B, NT>(t, ub + gridDim.x < nb ? ub + gridDim.x : -1, x, y, alpha_part, sm, spin_dyn,
+                               prog + (size_t)w * B * pb, prog + (size_t)(w ^ 1) * B * pb, pb);
+}
+
+// The blocks' programs: one warp per entry of the block list.
+template <class Sh, int D, int MO>
+__global__ void __launch_bounds__(kSpinThreads) spin_prog_kernel(const __grid_constant__ SpinParams p, const SpinDev t,
+                                                                 unsigned char* __restrict__ out) {
+  __shared__ Sh sh;
+  const bool has_site = __syncthreads_or(stage_spin(p, t, sh)) != 0;
+  const size_t pb = spin_block_prog_bytes(D, t.n_hh, t.n_x, t.n_key);
+  for (int64_t at = (blockIdx.x * (int64_t)kSpinThreads + threadIdx.x) / 32; at < t.n_rblk;
+       at += (int64_t)gridDim.x * kSpinThreads / 32)
+    spin_compile<Sh, D, MO>(sh, p, t, has_site, at, out + at * pb);
+}
+
+struct SpinXSites {
+  int n;
+  int shift[kSpinMaxSites];
+};
+
+// Its lo table and lo diagonal: one warp per slice of 32 lo codes of one digit sum.
+template <class Sh, int D, int MO>
+__global__ void __launch_bounds__(128) spin_low_kernel(const __grid_constant__ SpinParams p, const SpinDev t,
+                                                       const __grid_constant__ SpinRowVals vals,
+                                                       const __grid_constant__ SpinXSites xs,
+                                                       uint2* __restrict__ low_e, uint32_t* __restrict__ low_w,
+                                                       double* __restrict__ lodiag, uint8_t* __restrict__ lokey) {
+  constexpr int BITS = D <= 2 ? 1 : D <= 4 ? 2 : 3;
+  constexpr uint32_t dm = (1u << BITS) - 1u;
+  __shared__ Sh sh;
+  __syncthreads_or(stage_spin(p, t, sh));
+  const int lane = threadIdx.x & 31, Nh = t.N - t.Nl;
+  const uint32_t s = blockIdx.x * 4u + (threadIdx.x >> 5);
+  int k = (D - 1) * t.Nl;  // the digit sum of slice s
+  while (k > 0 && (t.looff[k] >> 5) + (uint32_t)k > s) --k;
+  const uint32_t base = t.looff[k], nk = t.looff[k + 1] - base;
+  const uint32_t r0 = (s - (base >> 5) - (uint32_t)k) * 32u, r = r0 + lane;
+  if (r0 >= nk) return;  // a slice number that no digit sum uses
+  const uint32_t lo = r < nk ? t.lolist[base + r] : 0u;
+  uint32_t* o = reinterpret_cast<uint32_t*>(low_e + ((size_t)s * t.low_st * 32 + lane));
+  double dg = 0.0;
+  int n = 0;
+  if (r < nk) {
+    for (int i = Nh; i < t.N; ++i) dg += sh.sdg[i * D + (int)((lo >> (BITS * (t.N - 1 - i))) & dm)];
+    for (int q = 0; q < p.n_bonds; ++q) {
+      const int4 b = sh.bond[q];
+      if (bond_side(b) != 0) continue;
+      const int pr = b.x + (int)((lo >> (b.y & 255)) & dm) * D + (int)((lo >> ((b.y >> 8) & 255)) & dm);
+      dg += sh.dg[pr];
+      const uint32_t kp = sh.pk[pr];
+#pragma unroll
+      for (int c = 0; c < MO; ++c) {
+        const int kk = (int)(int8_t)(uint8_t)(kp >> (8 * c));
+        if (kk == 0) continue;
+        int v = 0;
+        while (vals.v[v] != sh.ov[pr * MO + c]) ++v;  // one of them
+        o[(size_t)(n >> 1) * 64 + (n & 1)] = t.tlo[lo + (uint32_t)(kk * b.w)] << 4 | (uint32_t)(v * 8) << 20;
+        ++n;
+      }
+    }
+    lodiag[base + r] = dg;
+    if (t.n_key) {
+      int key = 0;
+      for (int c = xs.n - 1; c >= 0; --c) key = key * D + (int)((lo >> xs.shift[c]) & dm);
+      lokey[base + r] = (uint8_t)key;
+    }
+  }
+  const int w = (__reduce_max_sync(0xffffffffu, n) + 1) / 2;
+  if (lane == 0) low_w[s] = (uint32_t)w;
+  for (; n < 2 * w; ++n) o[(size_t)(n >> 1) * 64 + (n & 1)] = (uint32_t)t.maxrows << 4 | (uint32_t)(vals.n * 8) << 20;
+}
+
+// Its crossing table: one thread per (lo site, change q, lo code).
+__global__ void __launch_bounds__(256) spin_xtab_kernel(const SpinDev t, const __grid_constant__ SpinXSites xs,
+                                                        uint32_t* __restrict__ xtab) {
+  const int64_t n = blockIdx.x * 256ll + threadIdx.x;
+  const int nq = 2 * t.d - 1;
+  if (n >= xs.n * nq * t.n_lo) return;
+  const int64_t row = n / t.n_lo;
+  const uint32_t u = (uint32_t)(n - row * t.n_lo);
+  const int q = (int)(row % nq) - (t.d - 1), w = xs.shift[row / nq];
+  const uint32_t lo = t.lolist[u];
+  const int ld = (int)((lo >> w) & ((1u << t.bits) - 1u));
+  xtab[n] = ld - q >= 0 && ld - q < t.d ? t.tlo[lo - (uint32_t)(q * (1 << w))] | (uint32_t)ld << 24 : kSpinNone;
 }
 
 // y = H x on a momentum sector of a spin-S model, interleaved complex: row i
@@ -1071,6 +1182,231 @@ int launch_spin_lo_table(const SpinParams& p, const SpinDev& t, uint2* dst, cuda
       break;
   }
   return check_launch_counted("spin_lo_table_kernel");
+}
+
+void spin_block_list(const SpinParams& p, SpinTables& t) {
+  const int Nh = t.Nh, bits = t.bits, d = t.d, maxlo = (d - 1) * t.Nl;
+  const uint32_t dm = (1u << bits) - 1u;
+  const size_t nb = t.blk_hi.size();
+  // the hi-hi bonds (digit shifts, terms by digit pair) and the crossing bonds' hi digits
+  struct HiBond {
+    int wi, wj;
+    uint8_t terms[kSpinMaxPairs];
+  };
+  std::vector<HiBond> hb;
+  uint32_t hx = 0;
+  for (int q = 0; q < (p.n_cls ? p.n_bonds : 0); ++q) {
+    const int i = p.s1[q], j = p.s2[q];
+    if ((i < Nh) != (j < Nh)) hx |= dm << (bits * (Nh - 1 - std::min(i, j)));
+    if (i >= Nh || j >= Nh) continue;
+    HiBond b{bits * (Nh - 1 - i), bits * (Nh - 1 - j), {}};
+    for (int pr = 0; pr < d * d; ++pr)
+      for (uint32_t k = p.pk[p.cls[q]][pr]; k & 255u; k >>= 8) ++b.terms[pr];
+    hb.push_back(b);
+  }
+  // keys (crossing digits, block) by lo digit sum
+  std::vector<std::vector<uint64_t>> by(maxlo + 1);
+  std::vector<uint8_t> n_hh(nb, 0);
+  t.tfirst.resize(nb);
+  for (uint32_t b = 0, tile = 0; b < (uint32_t)nb; ++b) {
+    const uint32_t h = t.blk_hi[b];
+    int k = t.T;
+    for (uint32_t w = h; w; w >>= bits) k -= (int)(w & dm);
+    by[k].push_back((uint64_t)(h & hx) << 32 | b);
+    const int rows = (int)(t.looff[k + 1] - t.looff[k]);
+    t.tfirst[b] = tile;
+    tile += (uint32_t)(rows + kSpinTileRows - 1) / kSpinTileRows;
+    t.maxrows = std::max(t.maxrows, rows);
+    for (const HiBond& q : hb) n_hh[b] += q.terms[(h >> q.wi & dm) * d + (h >> q.wj & dm)];
+  }
+  std::vector<int> order(maxlo + 1);
+  for (int k = 0; k <= maxlo; ++k) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return t.looff[a + 1] - t.looff[a] > t.looff[b + 1] - t.looff[b];
+  });
+  constexpr size_t window = 32;
+  for (int k : order) {
+    std::vector<uint64_t>& key = by[k];
+    std::sort(key.begin(), key.end());
+    for (size_t i = 0; i < key.size();) {
+      size_t e = i;
+      while (e < key.size() && e - i < window && key[e] >> 32 == key[i] >> 32) ++e;
+      std::stable_sort(key.begin() + i, key.begin() + e,
+                       [&](uint64_t u, uint64_t v) { return n_hh[(uint32_t)u] > n_hh[(uint32_t)v]; });
+      i = e;
+    }
+    for (uint64_t v : key) t.rblk.push_back((uint32_t)v);
+    if (t.rblk.size() & 1) t.rblk.push_back(kSpinNone);
+  }
+}
+
+bool spin_rows_plan(const SpinParams& p, SpinDev& t, SpinRowsPlan& r) {
+  r = SpinRowsPlan();
+  if (p.n_cls == 0 || t.n_lo == 0) return false;
+  const int d = t.d, N = t.N, Nh = N - t.Nl, bits = t.bits, nq = 2 * d - 1;
+  r.vals.n = 0;
+  int n_hh = 0, n_ll = 0;
+  for (int c = 0; c < p.n_cls; ++c)
+    for (int pr = 0; pr < d * d; ++pr)
+      for (int s = 0; s < kSpinMaxOff && ((p.pk[c][pr] >> (8 * s)) & 255u); ++s) {
+        const double e = p.pov[c][pr][s];
+        if (!std::isfinite(e)) return false;
+        int v = 0;
+        while (v < r.vals.n && r.vals.v[v] != e) ++v;
+        if (v < r.vals.n) continue;
+        if (v == kSpinRowVals) return false;
+        r.vals.v[r.vals.n++] = e;
+      }
+  for (int q = 0; q < p.n_bonds; ++q) {
+    const int i = p.s1[q], j = p.s2[q];
+    const bool li = i >= Nh, lj = j >= Nh;
+    n_hh += !li && !lj;
+    n_ll += li && lj;
+    if (li == lj) continue;
+    SpinCross x{};
+    const int hs = li ? j : i, ls = li ? i : j;
+    x.hshift = bits * (Nh - 1 - hs);
+    x.lshift = bits * (N - 1 - ls);
+    size_t k = 0;
+    while (k < r.xsite.size() && r.xsite[k] != ls) ++k;
+    if (k == r.xsite.size()) r.xsite.push_back(ls);
+    x.tab = (int)k;
+    const size_t o0 = r.xoff.size(), d0 = r.xdiag.size();
+    r.xoff.resize(o0 + (size_t)d * nq * d, 0.0);
+    r.xdiag.resize(d0 + (size_t)d * d, 0.0);
+    for (int hd = 0; hd < d; ++hd)
+      for (int ld = 0; ld < d; ++ld) {
+        const int pr = li ? ld * d + hd : hd * d + ld;  // (digit of s1, digit of s2)
+        r.xdiag[d0 + hd * d + ld] = p.pdg[p.cls[q]][pr];
+        const uint32_t pk = p.pk[p.cls[q]][pr];
+        for (int s = 0; s < kSpinMaxOff && ((pk >> (8 * s)) & 255u); ++s) {
+          const int kk = (int)(int8_t)(uint8_t)(pk >> (8 * s));  // s1's digit rises by kk, s2's falls
+          const int dq = li ? -kk : kk;
+          r.xoff[o0 + ((size_t)hd * nq + dq + d - 1) * d + ld] = p.pov[p.cls[q]][pr][s];
+          x.mask |= 1ull << (hd * nq + dq + d - 1);
+        }
+      }
+    r.cross.push_back(x);
+  }
+  t.n_hh = n_hh * std::max(1, p.pmo);
+  t.n_x = (int)r.cross.size();
+  t.n_xtab = (int)r.xsite.size();
+  t.n_key = 0;
+  int keys = 1;
+  for (int k = 0; k < t.n_xtab && keys <= kSpinKeys; ++k) keys *= d;
+  if (t.n_xtab > 0 && keys <= kSpinKeys) t.n_key = keys;
+  t.hxmask = 0;
+  for (const SpinCross& c : r.cross) t.hxmask |= ((1u << bits) - 1u) << c.hshift;
+  t.low_st = (n_ll * std::max(1, p.pmo) + 1) / 2;
+  if ((int64_t)t.n_xtab * nq * t.n_lo > ((int64_t)1 << 26) ||
+      (int64_t)spin_low_slices(t) * t.low_st * 32 > ((int64_t)1 << 27))
+    return false;  // tables of at most 256 MB and 1 GB
+  return t.maxrows < (1 << 16) && spin_rows_smem_bytes(1, d, t.maxrows, t.n_hh, t.n_x, t.n_key) <= (size_t)200 << 10;
+}
+
+template <class F>
+void with_rows_form(const SpinParams& p, const SpinDev& t, F&& f) {
+  with_spin_form(p, t, [&](auto form) {
+    using Sh = typename decltype(form)::type;
+    if constexpr (!std::is_same<Sh, SpinShared>::value) f(form);
+  });
+}
+
+int launch_spin_rows_tables(const SpinParams& p, const SpinDev& t, const SpinRowsPlan& r, uint2* low_e,
+                            uint32_t* low_w, double* lodiag, uint8_t* lokey, uint32_t* xtab, cudaStream_t st) {
+  const unsigned grid = (unsigned)((spin_low_slices(t) + 3) / 4);
+  SpinXSites xs{};
+  xs.n = t.n_xtab;
+  for (int k = 0; k < xs.n; ++k) xs.shift[k] = t.bits * (t.N - 1 - r.xsite[k]);
+  with_rows_form(p, t, [&](auto form) {
+    using Sh = typename decltype(form)::type;
+    spin_low_kernel<Sh, Sh::kD, Sh::kMO><<<grid, 128, 0, st>>>(p, t, r.vals, xs, low_e, low_w, lodiag, lokey);
+  });
+  int rc = check_launch_counted("spin_low_kernel");
+  if (rc || t.n_xtab == 0) return rc;
+  const int64_t n = (int64_t)xs.n * (2 * t.d - 1) * t.n_lo;
+  spin_xtab_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(t, xs, xtab);
+  return check_launch_counted("spin_xtab_kernel");
+}
+
+size_t spin_prog_bytes(const SpinDev& t) {
+  return (size_t)t.n_rblk * spin_block_prog_bytes(t.d, t.n_hh, t.n_x, t.n_key);
+}
+
+int launch_spin_progs(const SpinParams& p, const SpinDev& t, unsigned char* out, cudaStream_t st) {
+  const int64_t want = (t.n_rblk + 7) / 8, cap = (int64_t)sm_count() * 8;
+  if (want < 1) return AED_OK;
+  with_rows_form(p, t, [&](auto form) {
+    using Sh = typename decltype(form)::type;
+    spin_prog_kernel<Sh, Sh::kD, Sh::kMO><<<(unsigned)(want < cap ? want : cap), kSpinThreads, 0, st>>>(p, t, out);
+  });
+  return check_launch_counted("spin_prog_kernel");
+}
+
+template <int D, int B, int NT, int MINB>
+int spin_rows_go(const SpinDev& t, const SpinRowVals& vals, const double* x, double* y, double* alpha_part,
+                 cudaStream_t st) {
+  auto kern = spin_rows_kernel<D, B, NT, MINB>;
+  const size_t dyn = spin_rows_smem_bytes(B, t.d, t.maxrows, t.n_hh, t.n_x, t.n_key);
+  static std::mutex mu;
+  static std::map<size_t, int> grids;  // shared memory -> CTAs per SM
+  static bool raised = false;
+  int per_sm = 0;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!raised) {
+      int dev = 0, optin = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+      cudaFuncAttributes fa{};
+      AED_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
+      AED_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        optin - (int)fa.sharedSizeBytes));
+      raised = true;
+    }
+    auto it = grids.find(dyn);
+    if (it == grids.end()) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, dyn);
+      cudaGetLastError();
+      it = grids.emplace(dyn, per_sm).first;
+    }
+    per_sm = it->second;
+  }
+  if (per_sm < 1) return kSpinRowsNone;
+  const int64_t nb = t.n_rblk / B, cap = (int64_t)sm_count() * per_sm;
+  kern<<<(unsigned)(nb < cap ? nb : cap), NT, dyn, st>>>(t, vals, x, y, alpha_part);
+  return check_launch_counted("spin_rows_kernel");
+}
+
+// 1024 threads per SM (64 registers), in as many CTAs as the x rows of two
+// blocks leave room for, so that one bundle's staging runs beside another's
+// rows; blocks of up to 640 rows in CTAs of 128 threads, which waste fewer
+// threads on their last rows; with few bundles 256 threads that cover a block at
+// once, and single blocks where two would leave SMs empty.  Measured (us, chains,
+// Sz = 0; against the tile apply): spin 1, L=18 833 (512 threads 894, single
+// blocks 1103; 1610), L=16 90 (96, 110; 200), L=12 8.3 (128 threads 12.5; 15.2),
+// L=10 6.1 (8.3 with two blocks; 14.7); S = 3/2, L=13 105 (256 threads 120; 233);
+// S = 2, L=11 70 (84; 155).
+int launch_spin_rows(const SpinParams& p, const SpinDev& t, const SpinRowVals& vals, const double* x, double* y,
+                     double* alpha_part, cudaStream_t st) {
+  if (t.n_tiles == 0) return AED_OK;
+  int rc = kSpinRowsNone;
+  with_rows_form(p, t, [&](auto form) {
+    constexpr int D = decltype(form)::type::kD;
+    const int64_t bundles = t.n_rblk / 2, sms = sm_count();
+    if (bundles < sms)
+      rc = spin_rows_go<D, 1, 256, 4>(t, vals, x, y, alpha_part, st);
+    else if (t.maxrows <= 640 && bundles > 4 * sms)
+      rc = spin_rows_go<D, 2, 128, 8>(t, vals, x, y, alpha_part, st);
+    else if (t.maxrows <= 3300)
+      rc = spin_rows_go<D, 2, 256, 4>(t, vals, x, y, alpha_part, st);
+    else if (t.maxrows <= 6600)
+      rc = spin_rows_go<D, 2, 512, 2>(t, vals, x, y, alpha_part, st);
+    else
+      rc = spin_rows_go<D, 2, 1024, 1>(t, vals, x, y, alpha_part, st);
+    if (rc == kSpinRowsNone) rc = spin_rows_go<D, 1, 1024, 1>(t, vals, x, y, alpha_part, st);
+  });
+  return rc;
 }
 
 int launch_spin_basis(const SpinDev& t, uint64_t* out, int64_t offset, int64_t count, cudaStream_t st) {

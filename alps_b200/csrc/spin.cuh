@@ -27,6 +27,16 @@ constexpr int kSpinMaxPairs = kSpinMaxDim * kSpinMaxDim;
 constexpr int kSpinMaxTrans = kSpinMaxPairs * kSpinMaxDim;
 constexpr int kSpinTileRows = 1024;                // rows per <x, y> partial of the apply
 
+constexpr int kSpinRowVals = 126;  // distinct elements of the rows apply's lo-lo terms
+
+// A bond across the hi and lo words: bit offsets of its digits, its lo site's
+// index among those with a crossing table, and per hi digit and its change q
+// (bit hd (2 d - 1) + q + d - 1) whether any lo digit has an element.
+struct SpinCross {
+  int hshift, lshift, tab;
+  unsigned long long mask;
+};
+
 // Host tables of one sector.
 struct SpinTables {
   int N = 0, twoS = 0, d = 0, bits = 0, Nh = 0, Nl = 0, T = 0;
@@ -38,8 +48,11 @@ struct SpinTables {
   std::vector<uint32_t> blk_hi;   // hi code of every block (ascending = basis order)
   std::vector<uint32_t> blk_off;  // first row of every block
   std::vector<uint32_t> tile_blk, tile_r;  // work tiles: (block, first row within it)
+  std::vector<uint32_t> rblk, tfirst;      // the rows apply's block list; first tile of every block
+  int maxrows = 0;                         // rows of the largest block
 };
 constexpr uint32_t kSpinNone = 0xffffffffu;
+constexpr int kSpinRowsNone = 1;  // launch_spin_rows: the blocks do not fit, nothing launched
 int build_spin_tables(int N, int twoS, int T, SpinTables& t);
 
 struct SpinDev {
@@ -54,6 +67,31 @@ struct SpinDev {
   const uint2* lol;
   int64_t n_lo;
   int n_ll;
+  // the rows apply (spin_rows.cuh; rblk == nullptr: none): blocks grouped by lo
+  // digit sum, each group padded with kSpinNone to an even number; the first
+  // tile of every block; the lo-lo terms in slices of 32 rows (slice
+  // (looff[k] >> 5) + k + (r >> 5) of row r of digit sum k; low_w pairs of
+  // entries, pair q of lane l at (slice * low_st + q) * 32 + l, an entry 16 x
+  // target rank | 8 x element index << 20); the diagonal of every lo code over
+  // the lo word; the crossing bonds with their tables: xtab[(tab (2 d - 1) + q +
+  // d - 1) n_lo + u] = rank of lo code u with the site's digit lowered by q |
+  // digit << 24, xoff / xdiag the elements by bond, hd, (q,) ld
+  const uint32_t* rblk = nullptr;
+  const uint32_t* tfirst = nullptr;
+  const uint2* low_e = nullptr;
+  const uint32_t* low_w = nullptr;
+  const double* lodiag = nullptr;
+  const SpinCross* cross = nullptr;
+  const uint32_t* xtab = nullptr;
+  const double *xoff = nullptr, *xdiag = nullptr;
+  int64_t n_rblk = 0;
+  int low_st = 0, maxrows = 0, n_hh = 0, n_x = 0, n_xtab = 0;
+  // n_key > 0: key of every lo code over its digits at the sites with a
+  // crossing table (d^n_xtab keys); hxmask the hi word's bits of crossing bonds
+  const uint8_t* lokey = nullptr;
+  const unsigned char* rprog = nullptr;  // the blocks' programs, in list order
+  int n_key = 0;
+  uint32_t hxmask = 0;
 };
 constexpr uint32_t kSpinLoNone = (1u << 26) - 1u;
 
@@ -89,6 +127,10 @@ struct SpinParams {
   uint32_t pk[kSpinMaxCls][kSpinMaxPairs];
   double sdiag[kSpinMaxSites][kSpinMaxDim];  // -h m + D m^2 of every site and digit
 };
+struct SpinRowVals {
+  int n;
+  double v[kSpinRowVals];
+};
 // The local operators of the spin model (models.xml.in:24-36, 282-300): the
 // transitions of Sz Sz, exchange_xy and biquadratic for spin S = twoS / 2.
 void spin_transitions(int twoS, SpinParams& p);
@@ -105,6 +147,28 @@ int launch_spin_hv(const SpinParams& p, const SpinDev& t, const double* x, doubl
 // fill (the table at dst, t.n_lo set); t.n_ll is set by the first call.
 size_t spin_lo_table_bytes(const SpinParams& p, SpinDev& t);
 int launch_spin_lo_table(const SpinParams& p, const SpinDev& t, uint2* dst, cudaStream_t st);
+// The rows apply's block list, ordered for p's bonds: largest blocks first,
+// within a digit sum by the digits of the crossing bonds, so that the blocks of
+// a bundle share their crossing terms, then by their number of hi-hi terms.
+void spin_block_list(const SpinParams& p, SpinTables& t);
+// Host plan of the rows apply for p's couplings: false when the form has none
+// (untabulated couplings, too many elements, or blocks too large for shared
+// memory).  Fills the counts of t and the arrays to upload.
+struct SpinRowsPlan {
+  std::vector<SpinCross> cross;
+  std::vector<double> xoff, xdiag;
+  std::vector<int> xsite;  // lo sites with a crossing table
+  SpinRowVals vals;
+};
+bool spin_rows_plan(const SpinParams& p, SpinDev& t, SpinRowsPlan& r);
+inline size_t spin_low_slices(const SpinDev& t) { return (size_t)t.n_lo / 32 + (size_t)(t.d - 1) * t.Nl + 2; }
+// Fill low_e / low_w / lodiag and the crossing table (device arrays).
+int launch_spin_rows_tables(const SpinParams& p, const SpinDev& t, const SpinRowsPlan& r, uint2* low_e,
+                            uint32_t* low_w, double* lodiag, uint8_t* lokey, uint32_t* xtab, cudaStream_t st);
+size_t spin_prog_bytes(const SpinDev& t);  // of all blocks' programs
+int launch_spin_progs(const SpinParams& p, const SpinDev& t, unsigned char* out, cudaStream_t st);
+int launch_spin_rows(const SpinParams& p, const SpinDev& t, const SpinRowVals& vals, const double* x, double* y,
+                     double* alpha_part, cudaStream_t st);
 __host__ __device__ inline int64_t spin_tiles_of(const SpinDev& t) { return t.n_tiles; }
 
 }  // namespace aed

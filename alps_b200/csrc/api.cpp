@@ -150,7 +150,8 @@ void release(aed_handle* h) {
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
                   (void*)h->d_slol, (void*)h->d_srblk, (void*)h->d_stfirst, (void*)h->d_slow_w, (void*)h->d_sxtab,
                   (void*)h->d_slow_e, (void*)h->d_slokey, (void*)h->d_srprog, (void*)h->d_slodiag, (void*)h->d_sxoff, (void*)h->d_sxdiag, (void*)h->d_scross,
-                  (void*)h->d_low_e, (void*)h->d_low_w})
+                  (void*)h->d_low_e, (void*)h->d_low_w, (void*)h->d_rprog[0][0], (void*)h->d_rprog[0][1],
+                  (void*)h->d_rprog[1][0], (void*)h->d_rprog[1][1], (void*)h->d_lolo})
     mem_dev_free(p, h->stream);
   mom_rows_free(h->mrows, h->stream);
   delete h->mp;
@@ -191,7 +192,40 @@ int upload_lo_table(aed_handle* h) {
   h->dt.low_e = h->d_low_e;
   h->dt.low_w = h->d_low_w;
   h->dt.low_st = lo_slice_pairs(W);
-  return launch_lo_slices(h->dt, h->dt.maxrows, h->P.n_lolo, h->d_low_e, h->d_low_w, h->stream);
+  if ((rc = launch_lo_slices(h->dt, h->dt.maxrows, h->P.n_lolo, h->d_low_e, h->d_low_w, h->stream))) return rc;
+  // and the rows apply's programs (an FP32 handle's refinement applies H to
+  // FP64 vectors too); without memory for them the tile apply serves the handle
+  DevTables& t = h->dt;
+  for (auto& e : t.rprog) e[0] = e[1] = nullptr;
+  t.n_lolo = h->P.n_lolo;
+  if (t.n_blk == 0 || !h->P.finite) return AED_OK;
+  if (!h->d_lolo && mem_dev_alloc_n(&h->d_lolo, (size_t)kMaxBonds)) return AED_OK;
+  t.lolo_c = h->d_lolo;
+  const int n_elem = h->precision == AED_FP32 ? 2 : 1;
+  int* d_ops = reinterpret_cast<int*>(h->d_scal);  // free between calls
+  int ops[4] = {};
+  AED_CUDA_TRY(cudaMemsetAsync(d_ops, 0, sizeof ops, h->stream));
+  for (int e = 0; e < n_elem; ++e)
+    if ((rc = launch_row_need(h->P, t, e == 0 ? 8 : 4, d_ops + 2 * e, h->stream))) return rc;
+  AED_CUDA_TRY(cudaMemcpyAsync(ops, d_ops, sizeof ops, cudaMemcpyDeviceToHost, h->stream));
+  AED_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  for (int e = 0; e < n_elem; ++e)
+    for (int row = 0; row < 2; ++row) {
+      const int elem = e == 0 ? 8 : 4;
+      t.rcap[e][row] = std::max(2, (ops[2 * e + row] + 1) & ~1);
+      t.rstride[e][row] = row_prog_stride(elem, row, t.rcap[e][row]);
+      const size_t bytes = (size_t)(t.n_blk / row_blocks(elem, row)) * (size_t)t.rstride[e][row];
+      if (bytes > h->d_rprog_n[e][row]) {
+        mem_dev_free(h->d_rprog[e][row], h->stream);
+        h->d_rprog[e][row] = nullptr;
+        h->d_rprog_n[e][row] = 0;
+        if (mem_dev_alloc_n(&h->d_rprog[e][row], bytes)) return AED_OK;
+        h->d_rprog_n[e][row] = bytes;
+      }
+      if ((rc = launch_row_progs(h->P, t, elem, row, h->d_rprog[e][row], h->d_lolo, h->stream))) return rc;
+      t.rprog[e][row] = h->d_rprog[e][row];
+    }
+  return AED_OK;
 }
 
 int check_vec(const aed_handle* h, const void* p, const char* name) {

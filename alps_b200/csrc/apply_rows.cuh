@@ -32,6 +32,10 @@ using apply::SPair;
 using apply::TileOp;
 
 constexpr int kMaxB = 4;
+// Flips (of all blocks; FP32: hi-part / crossing ones) whose loads go out
+// together.  They fill the 64 registers of 1024 threads per SM without a spill;
+// eight, or four crossing ones, spill and were 5-25 % slower on L=28 and 6x5.
+constexpr int kU = 4, kUC = 2;
 constexpr uint32_t kNullOp = 0x80000001u;     // an op that no row takes (no byte offset of an element)
 constexpr uint32_t kCrossTest = 0x80008000u;  // null bit and the required lo-bit value
 constexpr int kMaxItems = 32;  // (block, tile) pairs of a bundle: 4 blocks of at most 7 tiles
@@ -43,33 +47,52 @@ struct alignas(sizeof(T) * B) RowVec {
 
 struct RowsSmem {
   double lolo_c[kMaxBonds + 1];  // the last: 0, of the padding entries
-  int n1, n2, full;  // ops of the two lists; hi-part ops that all blocks have
   double red[kMaxItems][kHvThreads / 32];
 };
 
-// The bundle's program: the flips outside the lo part that apply to its blocks,
-// op o of all B blocks side by side.
+// A bundle's program: a head, then the flips outside the lo part that apply to
+// its blocks, op o of all B blocks side by side.
 //   FP64 (rows in column order): ops[o * B + j], the flips to smaller states in
 //   [0, n1), those to larger ones in [n1, n1 + n2);
-//   FP32: the hi-part flips as nb[o * B + j] and c[o * B + j], o < n1, the
-//   crossing ones at o >= cross0 with their lo bit and required values in bits[o].
+//   FP32: c[o * B + j] and nb[o * B + j], the hi-part flips at o < n1, the
+//   crossing ones in [n1, n1 + n2) with their lo bit and required values in bits[o].
 // Lists are as long as the longest block's, rounded up to a multiple of the
-// unrolling (at most 8), filled with null ops.
+// unrolling, filled with null ops.  Programs depend on the couplings alone: a
+// handle forms them once (launch_row_progs), `cap` ops each, and a CTA copies
+// the next bundle's while it runs one.  (Listed in the apply, by a warp per
+// block while the others staged x, they put a chain of dependent loads and a
+// barrier before every bundle.)
+struct RowHead {
+  uint32_t first[kMaxB], tile[kMaxB];  // first row and tile of each block
+  uint32_t lbase, nk;                  // lo class offset and rows per block
+  int32_t k, nv;                       // lo popcount, blocks (0: none)
+  int32_t n1, n2, full, pad;           // ops of the lists; FP32 hi-part ops that every block has
+};
+static_assert(sizeof(RowHead) == 64, "a multiple of 16 bytes");
 struct Program {
   TileOp* ops;
   uint32_t* nb;
   double* c;
   uint32_t* bits;
 };
-__host__ __device__ inline int prog_ops(int elem, int n_pairs, int n_lolo) {
-  return (elem == 8 ? 2 : 1) * (n_pairs - n_lolo) + 14;
+template <int B>
+__host__ __device__ inline Program program_at(unsigned char* p, int cap) {
+  Program g;
+  g.ops = reinterpret_cast<TileOp*>(p + sizeof(RowHead));
+  g.c = reinterpret_cast<double*>(p + sizeof(RowHead));
+  g.nb = reinterpret_cast<uint32_t*>(g.c + (size_t)cap * B);
+  g.bits = g.nb + (size_t)cap * B;
+  return g;
+}
+// Bytes of one program of `cap` ops (cap even).
+__host__ __device__ inline int prog_stride(int B, int elem, int cap) {
+  const int b = (int)sizeof(RowHead) + cap * (elem == 8 ? B * 16 : B * 12 + 4);
+  return (b + 15) & ~15;
 }
 
-// Dynamic shared memory: x rows (and the row of zeros), the program, the flip pairs.
-__host__ __device__ inline size_t rows_smem_bytes(int row_bytes, int B, int maxrows, int n_pairs, int n_lolo) {
-  return (((size_t)(maxrows + 1) * row_bytes + 15) & ~(size_t)15) +
-         (size_t)prog_ops(row_bytes / B, n_pairs, n_lolo) * (B * sizeof(TileOp) + 16) +
-         2 * (size_t)n_pairs * sizeof(SPair);
+// Dynamic shared memory: x rows (and the row of zeros) and two programs.
+__host__ __device__ inline size_t rows_smem_bytes(int row_bytes, int maxrows, int stride) {
+  return (((size_t)(maxrows + 1) * row_bytes + 15) & ~(size_t)15) + 2 * (size_t)stride;
 }
 
 // The value at a 32-bit byte offset (an FP32 vector of at most 2^30 rows; the
@@ -279,78 +302,117 @@ __device__ __forceinline__ void compile_f32(const ApplyCtx& c, const uint32_t* _
     put(at, __ldg(thi + (h ^ (e.flip >> c.Nlo))) * 4u, e.c);
     const uint32_t b = (uint32_t)(__ffs(e.flip & c.lm) - 1);
     // the lo bit must differ from the hi bit: set where h's is clear
-    atomicOr(pg.bits + at, b << 16 | 1u << (h & (e.flip >> c.Nlo) ? 8 + j : j));
+    const uint32_t want = b << 16 | 1u << (h & (e.flip >> c.Nlo) ? 8 + j : j);
+    pg.bits[at] = j == 0 ? want : pg.bits[at] | want;
   });
-  for (int q = n + lane; q < l1 + l2; q += 32) put(q, 0u, 0.0);
+  for (int q = n + lane; q < l1 + l2; q += 32) {
+    put(q, 0u, 0.0);
+    pg.bits[q] = 0u;
+  }
 }
 
-// Bundle ub of the block list.
-template <typename T, typename Acc, int B, int NT, int U, int UC>
-__device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& t, int64_t ub, const T* __restrict__ x,
-                                            T* y, double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
-                                            const Program& pg, int n_ops, const SPair* low, const SPair* rise) {
+// One warp: lengths of the lists of bundle ub (rounded up) and, FP32, the
+// hi-part ops that every block has.
+template <typename T, int B, int U, int UC>
+__device__ __forceinline__ int list_lengths(const ApplyCtx& c, const DevTables& t, int64_t ub, const SPair* low,
+                                            const SPair* rise, int* n1, int* n2, int* full) {
   constexpr bool kOrdered = sizeof(T) == 8;
-  using Row = RowVec<T, B>;
-  Row* rows = reinterpret_cast<Row*>(xs);
-  int nv = 0;
-  uint32_t bj[B], tf[B];
-  uint32_t h0 = 0;
-#pragma unroll
+  auto none = [](int, const SPair&) {};
+  int nv = 0, l1 = 0, l2 = 0, f = 1 << 20;
   for (int j = 0; j < B; ++j) {
     const uint32_t h = __ldg(t.blk_h + ub * B + j);
-    const bool real = h != kNoBlockEntry;  // real blocks come first in a bundle
-    if (j == 0) h0 = h;
-    nv += real ? 1 : 0;
-    bj[j] = real ? __ldg(t.thi + h) : 0u;
-    tf[j] = real ? __ldg(t.tfirst + h) : 0u;
+    if (h == kNoBlockEntry) break;  // real blocks come first in a bundle
+    ++nv;
+    const int n = walk_list(low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 1, 0, none);
+    l1 = max(l1, n);
+    f = min(f, n);
+    if (kOrdered || j == 0)
+      l2 = max(l2, walk_list(kOrdered ? rise : low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 2, 0, none));
   }
-  if (nv == 0) return;  // padding of the block list
-  const int k = c.n_up - __popc(h0);
-  const uint32_t lbase = __ldg(t.looff + k);
-  const uint32_t nk = __ldg(t.looff + k + 1) - lbase;
-  __syncthreads();  // the previous bundle is done with the program, x and red
-  if constexpr (!kOrdered) {  // collected by the blocks' warps below
-    for (int q = threadIdx.x; q < n_ops; q += NT) pg.bits[q] = 0u;
-    __syncthreads();
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < B) {
-    // the lists of all blocks are as long as the longest, a multiple of the unrolling
-    auto none = [](int, const SPair&) {};
-    int l1 = 0, l2 = 0, full = 1 << 20;
-    for (int j = 0; j < nv; ++j) {
+  *n1 = kOrdered ? (l1 + U - 1) / U * U : (l1 + 1) / 2 * 2;
+  *n2 = kOrdered ? (l2 + U - 1) / U * U : (l2 + UC - 1) / UC * UC;
+  *full = nv == B ? f : 0;
+  return nv;
+}
+
+// One warp forms the program of bundle ub at `out` (cap ops; cap 0: only the
+// length it needs, which it returns).
+template <typename T, int B, int U, int UC>
+__device__ __forceinline__ int form_program(const ApplyCtx& c, const DevTables& t, int64_t ub, const SPair* low,
+                                            const SPair* rise, unsigned char* out, int cap) {
+  constexpr bool kOrdered = sizeof(T) == 8;
+  int n1, n2, full;
+  const int nv = list_lengths<T, B, U, UC>(c, t, ub, low, rise, &n1, &n2, &full);
+  if (cap == 0) return n1 + n2;
+  const int lane = threadIdx.x & 31;
+  const Program pg = program_at<B>(out, cap);
+  RowHead hd{};
+  hd.nv = nv;
+  hd.n1 = n1;
+  hd.n2 = n2;
+  hd.full = full;
+  for (int j = 0; j < B; ++j) {
+    if (j < nv) {
       const uint32_t h = __ldg(t.blk_h + ub * B + j);
-      const int n = walk_list(low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 1, 0, none);
-      l1 = max(l1, n);
-      full = min(full, n);
-      if (kOrdered || j == 0)
-        l2 = max(l2, walk_list(kOrdered ? rise : low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 2, 0, none));
-    }
-    if (nv < B) full = 0;
-    l1 = kOrdered ? (l1 + U - 1) / U * U : (l1 + 1) / 2 * 2;
-    l2 = kOrdered ? (l2 + U - 1) / U * U : (l2 + UC - 1) / UC * UC;
-    if (warp == 0 && lane == 0) {
-      sm.n1 = l1;
-      sm.n2 = l2;
-      sm.full = full;
-    }
-    if (warp < nv) {
-      const uint32_t h = __ldg(t.blk_h + ub * B + warp);
+      if (j == 0) {
+        hd.k = c.n_up - __popc(h);
+        hd.lbase = __ldg(t.looff + hd.k);
+        hd.nk = __ldg(t.looff + hd.k + 1) - hd.lbase;
+      }
+      hd.first[j] = __ldg(t.thi + h);
+      hd.tile[j] = __ldg(t.tfirst + h);
       if constexpr (kOrdered)
-        compile_f64<B>(c, t.thi, low, rise, h, warp, l1, l2, pg.ops);
+        compile_f64<B>(c, t.thi, low, rise, h, j, n1, n2, pg.ops);
       else
-        compile_f32<B>(c, t.thi, low, h, warp, l1, l2, pg);
+        compile_f32<B>(c, t.thi, low, h, j, n1, n2, pg);
+      __syncwarp();
     } else {  // no such block in the bundle: null ops
-      for (int q = lane; q < l1 + l2; q += 32) {
+      for (int q = lane; q < n1 + n2; q += 32) {
         if constexpr (kOrdered) {
-          pg.ops[q * B + warp] = {kNullOp, 0u, 0.0};
+          pg.ops[q * B + j] = {kNullOp, 0u, 0.0};
         } else {
-          pg.nb[q * B + warp] = kNullOp;
-          pg.c[q * B + warp] = 0.0;
+          pg.nb[q * B + j] = kNullOp;
+          pg.c[q * B + j] = 0.0;
         }
       }
     }
   }
+  if (lane == 0) *reinterpret_cast<RowHead*>(out) = hd;
+  return n1 + n2;
+}
+
+// A program on its way from `src` into shared memory (every thread; waited for
+// by the next rows_bundle).
+template <int NT>
+__device__ __forceinline__ void fetch_program(const unsigned char* src, unsigned char* dst, int bytes) {
+  for (int i = (int)threadIdx.x * 16; i < bytes; i += NT * 16) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + i);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + i) : "memory");
+  }
+}
+
+// The bundle whose program is in (or on its way into) prog; the next one's
+// (next == nullptr: none) goes to `other` while this one runs.
+template <typename T, typename Acc, int B, int NT, int U, int UC>
+__device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restrict__ x, T* y,
+                                            double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
+                                            unsigned char* prog, unsigned char* other,
+                                            const unsigned char* __restrict__ next, int stride, int cap) {
+  constexpr bool kOrdered = sizeof(T) == 8;
+  using Row = RowVec<T, B>;
+  Row* rows = reinterpret_cast<Row*>(xs);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();  // this program is here; the previous bundle is done with x, red and `other`
+  if (next) fetch_program<NT>(next, other, stride);
+  const RowHead& hd = *reinterpret_cast<const RowHead*>(prog);
+  const Program pg = program_at<B>(prog, cap);
+  const int nv = hd.nv;
+  if (nv == 0) return;  // padding of the block list
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t lbase = hd.lbase, nk = hd.nk;
+  uint32_t bj[B];
+#pragma unroll
+  for (int j = 0; j < B; ++j) bj[j] = hd.first[j];
   // x of the blocks, row by row, two rows in flight per thread
   for (uint32_t i = threadIdx.x; i < nk; i += 2 * NT) {
     Row a, b;
@@ -364,9 +426,9 @@ __device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& 
     if (two) rows[i + NT] = b;
   }
   __syncthreads();
-  const int n1 = sm.n1, n2 = sm.n2, full = sm.full;
+  const int n1 = hd.n1, n2 = hd.n2, full = hd.full, Nlo = t.Nlo;
   const unsigned char* cs = reinterpret_cast<const unsigned char*>(sm.lolo_c);
-  const uint32_t s0 = (lbase >> 5) + (uint32_t)k;
+  const uint32_t s0 = (lbase >> 5) + (uint32_t)hd.k;
 #pragma unroll 1
   for (uint32_t r = threadIdx.x; r < nk; r += NT) {
     const uint16_t* xt = t.xtab + lbase + r;
@@ -379,7 +441,7 @@ __device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& 
       double dg[B];
 #pragma unroll
       for (int j = 0; j < B; ++j) dg[j] = j < nv ? __ldg(t.dg + bj[j] + r) : 0.0;
-      hi_terms<T, Acc, B, U>(pg.ops, n1, r, xt, c.Nlo, x, acc);
+      hi_terms<T, Acc, B, U>(pg.ops, n1, r, xt, Nlo, x, acc);
       lo_terms<T, Acc, B>(tp, wl, xs, cs, acc);
       {
         const Row own = rows[r];
@@ -387,14 +449,14 @@ __device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& 
         for (int j = 0; j < B; ++j) acc[j].add(dg[j], own.v[j]);
       }
       lo_terms<T, Acc, B>(tp + wl * 32, wu, xs, cs, acc);
-      hi_terms<T, Acc, B, U>(pg.ops + n1 * B, n2, r, xt, c.Nlo, x, acc);
+      hi_terms<T, Acc, B, U>(pg.ops + n1 * B, n2, r, xt, Nlo, x, acc);
     } else {
       const Row own = rows[r];
 #pragma unroll
       for (int j = 0; j < B; ++j)
         if (j < nv) acc[j].add(apply::diag_fp32(t, bj[j] + r), own.v[j]);
       hihi_terms<T, Acc, B, U>(pg, full, n1, r * (uint32_t)sizeof(T), x, acc);
-      cross_terms<T, Acc, B, UC>(pg, n1, n2, xt, c.Nlo, x, acc);
+      cross_terms<T, Acc, B, UC>(pg, n1, n2, xt, Nlo, x, acc);
       lo_terms<T, Acc, B>(tp, wl + wu, xs, cs, acc);
     }
 #pragma unroll
@@ -414,9 +476,7 @@ __device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& 
     const uint32_t th = threadIdx.x % kHalf + (q & 1 ? kHalf : 0);
     const int j = it / (int)nt;
     const uint32_t r0 = (uint32_t)(it - j * (int)nt) * kTileRows;
-    uint32_t base = bj[0];
-#pragma unroll
-    for (int b = 1; b < B; ++b) base = j == b ? bj[b] : base;
+    const uint32_t base = hd.first[j];
     double dot = 0.0;
 #pragma unroll
     for (int i = 0; i < kTileRows / kHvThreads; ++i) {
@@ -429,9 +489,7 @@ __device__ __forceinline__ void rows_bundle(const ApplyCtx& c, const DevTables& 
   __syncthreads();
   for (int it = warp; it < items; it += NT / 32) {
     const int j = it / (int)nt;
-    uint32_t first = tf[0];
-#pragma unroll
-    for (int b = 1; b < B; ++b) first = j == b ? tf[b] : first;
+    const uint32_t first = hd.tile[j];
     double r = lane < kHvThreads / 32 ? sm.red[it][lane] : 0.0;
     for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
     if (lane == 0) alpha_part[first + (uint32_t)(it - j * (int)nt)] = r;

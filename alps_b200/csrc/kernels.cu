@@ -44,42 +44,72 @@ __global__ void __launch_bounds__(kHvThreads, MINB) hv_kernel(const __grid_const
 }
 
 // y = H x over bundles with x interleaved in shared memory (apply_rows.cuh).
-// U / UC: flips (FP32: hi-part / crossing ones) whose loads go out together.
-template <typename T, typename Acc, int B, int NT, int MINB, int U, int UC>
-__global__ void __launch_bounds__(NT, MINB) hvr_kernel(const __grid_constant__ HvParams P, const DevTables t,
-                                                       const T* __restrict__ x, T* y,
+template <typename T, typename Acc, int B, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const T* __restrict__ x, T* y,
                                                        double* __restrict__ alpha_part) {
   extern __shared__ __align__(16) unsigned char hvr_dyn[];
   __shared__ rapply::RowsSmem sm;
-  constexpr int kRow = sizeof(T) * B;
-  const int n_ops = rapply::prog_ops((int)sizeof(T), P.n_pairs, P.n_lolo);
-  unsigned char* p = hvr_dyn + (((size_t)(t.maxrows + 1) * kRow + 15) & ~(size_t)15);
-  rapply::Program pg;
-  pg.ops = reinterpret_cast<apply::TileOp*>(p);
-  pg.c = reinterpret_cast<double*>(p);
-  p += (size_t)B * n_ops * sizeof(double);
-  pg.nb = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)B * n_ops * (sizeof(apply::TileOp) - sizeof(double));
-  pg.bits = reinterpret_cast<uint32_t*>(p);
-  p += (size_t)n_ops * 16;
-  apply::SPair* low = reinterpret_cast<apply::SPair*>(p);
-  apply::SPair* rise = low + P.n_pairs;
-  for (int q = threadIdx.x; q < P.n_pairs; q += NT) {
-    const PairTerm a = P.low[q], b = P.rise[q];
-    low[q] = {a.mhi | a.mlo, a.mhi, a.c};
-    rise[q] = {b.mhi | b.mlo, b.mlo, b.c};
-  }
-  for (int q = threadIdx.x; q <= P.n_lolo; q += NT) sm.lolo_c[q] = q < P.n_lolo ? P.lolo_c[q] : 0.0;
-  if (threadIdx.x == 0) {
-    rapply::RowVec<T, B> z;
-#pragma unroll
-    for (int j = 0; j < B; ++j) z.v[j] = T(0);
-    reinterpret_cast<rapply::RowVec<T, B>*>(hvr_dyn)[t.maxrows] = z;
-  }
-  const apply::ApplyCtx c = apply::ctx_of(P);
+  constexpr int kRow = sizeof(T) * B, kTab = kRow == 16 ? 0 : 1;
+  constexpr int kEl = sizeof(T) == 8 ? 0 : 1;
+  const int stride = t.rstride[kEl][kTab], cap = t.rcap[kEl][kTab];
+  unsigned char* prog = hvr_dyn + (((size_t)(t.maxrows + 1) * kRow + 15) & ~(size_t)15);
+  const unsigned char* src = t.rprog[kEl][kTab];
   const int64_t nb = t.n_blk / B;
-  for (int64_t ub = blockIdx.x; ub < nb; ub += gridDim.x)
-    rapply::rows_bundle<T, Acc, B, NT, U, UC>(c, t, ub, x, y, alpha_part, sm, hvr_dyn, pg, n_ops, low, rise);
+  int64_t ub = blockIdx.x;
+  if (ub < nb) rapply::fetch_program<NT>(src + ub * stride, prog, stride);
+  for (int q = threadIdx.x; q <= t.n_lolo; q += NT) sm.lolo_c[q] = q < t.n_lolo ? __ldg(t.lolo_c + q) : 0.0;
+  if (threadIdx.x < B) reinterpret_cast<T*>(hvr_dyn)[(size_t)t.maxrows * B + threadIdx.x] = T(0);
+  int w = 0;
+  for (; ub < nb; ub += gridDim.x, w ^= 1)
+    rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(
+        t, x, y, alpha_part, sm, hvr_dyn, prog + w * stride, prog + (w ^ 1) * stride,
+        ub + gridDim.x < nb ? src + (ub + gridDim.x) * stride : nullptr, stride, cap);
+}
+
+// The rows apply's programs, one warp per bundle.
+struct PairSmem {
+  apply::SPair low[kMaxBonds], rise[kMaxBonds];
+};
+__device__ __forceinline__ void stage_flips(const HvParams& P, PairSmem& sm) {
+  for (int q = threadIdx.x; q < P.n_pairs; q += blockDim.x) {
+    const PairTerm a = P.low[q], b = P.rise[q];
+    sm.low[q] = {a.mhi | a.mlo, a.mhi, a.c};
+    sm.rise[q] = {b.mhi | b.mlo, b.mlo, b.c};
+  }
+  __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) row_need_kernel(const __grid_constant__ HvParams P, const DevTables t,
+                                                       int* __restrict__ need) {
+  __shared__ PairSmem sm;
+  stage_flips(P, sm);
+  const apply::ApplyCtx c = apply::ctx_of(P);
+  constexpr int B = 16 / sizeof(T);
+  int n16 = 0, n8 = 0;
+  for (int64_t ub = blockIdx.x * 8 + (threadIdx.x >> 5); ub < t.n_blk / B; ub += (int64_t)gridDim.x * 8) {
+    n16 = max(n16, rapply::form_program<T, B, rapply::kU, rapply::kUC>(c, t, ub, sm.low, sm.rise, nullptr, 0));
+    for (int q = 0; q < 2; ++q)
+      n8 = max(n8, rapply::form_program<T, B / 2, rapply::kU, rapply::kUC>(c, t, 2 * ub + q, sm.low, sm.rise, nullptr,
+                                                                            0));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(need, n16);
+    atomicMax(need + 1, n8);
+  }
+}
+
+template <typename T, int B>
+__global__ void __launch_bounds__(256) row_prog_kernel(const __grid_constant__ HvParams P, const DevTables t,
+                                                       unsigned char* __restrict__ out, int stride, int cap,
+                                                       double* __restrict__ lolo_c) {
+  __shared__ PairSmem sm;
+  stage_flips(P, sm);
+  const apply::ApplyCtx c = apply::ctx_of(P);
+  if (blockIdx.x == 0)
+    for (int q = threadIdx.x; q < P.n_lolo; q += 256) lolo_c[q] = P.lolo_c[q];
+  for (int64_t ub = blockIdx.x * 8 + (threadIdx.x >> 5); ub < t.n_blk / B; ub += (int64_t)gridDim.x * 8)
+    rapply::form_program<T, B, rapply::kU, rapply::kUC>(c, t, ub, sm.low, sm.rise, out + ub * stride, cap);
 }
 
 // The lo-neighbour table: one thread per lo state, its flips inserted in order
@@ -529,15 +559,12 @@ int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* 
 // at this sector's dynamic shared memory (sectors of one process share a few
 // sizes).  Not for couplings that are not finite: a flip that a row does not
 // take adds c * 0.
-// Four flips of all blocks in flight (FP32 crossing flips: two) fill the 64
-// registers of 1024 threads per SM without a spill; eight, or four crossing
-// ones, spill and were 5-25 % slower on L=28 and 6x5.
 template <typename T, typename Acc, int ROW, int NT, int MINB>
 int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
-  constexpr int B = ROW / (int)sizeof(T);
-  if (!t.blk_h || !t.low_e || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
-  const size_t dyn = rapply::rows_smem_bytes(ROW, B, t.maxrows, P.n_pairs, P.n_lolo);
-  auto kern = hvr_kernel<T, Acc, B, NT, MINB, 4, 2>;
+  constexpr int B = ROW / (int)sizeof(T), kTab = ROW == 16 ? 0 : 1, kEl = sizeof(T) == 8 ? 0 : 1;
+  if (!t.low_e || !t.rprog[kEl][kTab] || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
+  const size_t dyn = rapply::rows_smem_bytes(ROW, t.maxrows, t.rstride[kEl][kTab]);
+  auto kern = hvr_kernel<T, Acc, B, NT, MINB>;
   static int limit_rc = -1;
   static size_t static_bytes = 0;
   static std::map<size_t, int> grids;  // dyn -> grid (0: does not fit)
@@ -563,7 +590,7 @@ int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double*
   const int64_t nb = t.n_blk / B;
   if (g > nb) g = nb;
   if (g < 1) return AED_OK;
-  kern<<<(unsigned)g, NT, dyn, st>>>(P, t, x, y, alpha_part);
+  kern<<<(unsigned)g, NT, dyn, st>>>(t, x, y, alpha_part);
   return check_launch("hvr_kernel");
 }
 
@@ -688,6 +715,35 @@ int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaSt
   if (t.ell_w == 0) return AED_OK;
   lo_table_kernel<<<((1u << t.Nlo) + 127) / 128, 128, 0, st>>>(P, t, ell);
   return check_launch("lo_table_kernel");
+}
+
+int row_blocks(int elem, int row) { return (row == 0 ? 16 : 8) / elem; }
+int row_prog_stride(int elem, int row, int cap) { return rapply::prog_stride(row_blocks(elem, row), elem, cap); }
+
+int launch_row_need(const HvParams& P, const DevTables& t, int elem, int* need, cudaStream_t st) {
+  const int64_t want = (t.n_blk / row_blocks(elem, 0) + 7) / 8, cap = (int64_t)num_sms() * 4;
+  const unsigned grid = (unsigned)(want < 1 ? 1 : want < cap ? want : cap);
+  if (elem == 8)
+    row_need_kernel<double><<<grid, 256, 0, st>>>(P, t, need);
+  else
+    row_need_kernel<float><<<grid, 256, 0, st>>>(P, t, need);
+  return check_launch("row_need_kernel");
+}
+
+int launch_row_progs(const HvParams& P, const DevTables& t, int elem, int row, unsigned char* out, double* lolo_c,
+                     cudaStream_t st) {
+  const int64_t want = (t.n_blk / row_blocks(elem, row) + 7) / 8, lim = (int64_t)num_sms() * 4;
+  const unsigned grid = (unsigned)(want < 1 ? 1 : want < lim ? want : lim);
+  const int e = elem == 8 ? 0 : 1, stride = t.rstride[e][row], cap = t.rcap[e][row];
+  if (elem == 8 && row == 0)
+    row_prog_kernel<double, 2><<<grid, 256, 0, st>>>(P, t, out, stride, cap, lolo_c);
+  else if (elem == 8)
+    row_prog_kernel<double, 1><<<grid, 256, 0, st>>>(P, t, out, stride, cap, lolo_c);
+  else if (row == 0)
+    row_prog_kernel<float, 4><<<grid, 256, 0, st>>>(P, t, out, stride, cap, lolo_c);
+  else
+    row_prog_kernel<float, 2><<<grid, 256, 0, st>>>(P, t, out, stride, cap, lolo_c);
+  return check_launch("row_prog_kernel");
 }
 
 int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st) {

@@ -43,6 +43,13 @@ struct DevTables {
   const uint2* low_e = nullptr;
   const uint32_t* low_w = nullptr;
   int low_st = 0;
+  // the rows apply's programs (apply_rows.cuh), one per bundle of the block
+  // list, for FP64 [0] and FP32 [1] vectors and rows of 16 [0] and 8 [1] bytes
+  // (nullptr: none); couplings of the lo-part flips
+  const unsigned char* rprog[2][2] = {};
+  int rstride[2][2] = {}, rcap[2][2] = {};
+  const double* lolo_c = nullptr;
+  int n_lolo = 0;
 };
 
 constexpr int kHvThreads = 256;
@@ -79,6 +86,16 @@ int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaSt
 inline int lo_slice_pairs(int ell_w) { return 2 * ((ell_w + 1) / 2) + 1; }  // each part at most ell_w entries
 inline size_t lo_slices(int Nlo) { return ((size_t)1 << Nlo) / 32 + (size_t)Nlo + 2; }
 int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st);
+
+// The rows apply's programs of P for vectors of `elem` bytes an element: `need`
+// (two device ints, zeroed) gets the ops per program for rows of 16 and 8 bytes;
+// then the programs into out (row = 0: 16 bytes, 1: 8 bytes; t.rstride / t.rcap
+// set) and P's lo-part couplings into lolo_c.
+int row_blocks(int elem, int row);                 // blocks of a bundle
+int row_prog_stride(int elem, int row, int cap);   // bytes of a program
+int launch_row_need(const HvParams& P, const DevTables& t, int elem, int* need, cudaStream_t st);
+int launch_row_progs(const HvParams& P, const DevTables& t, int elem, int row, unsigned char* out, double* lolo_c,
+                     cudaStream_t st);
 
 // per-row diagonal table (once per handle)
 int launch_diag_table(const HvParams& P, const DevTables& t, double* dg, cudaStream_t st);

@@ -192,7 +192,7 @@ int upload_lo_table(aed_handle* h) {
   h->dt.low_e = h->d_low_e;
   h->dt.low_w = h->d_low_w;
   h->dt.low_st = lo_slice_pairs(W);
-  if ((rc = launch_lo_slices(h->dt, h->dt.maxrows, h->P.n_lolo, h->d_low_e, h->d_low_w, h->stream))) return rc;
+  if ((rc = launch_lo_slices(h->P, h->dt, h->d_low_e, h->d_low_w, h->stream))) return rc;
   // and the rows apply's programs (an FP32 handle's refinement applies H to
   // FP64 vectors too); without memory for them the tile apply serves the handle
   DevTables& t = h->dt;

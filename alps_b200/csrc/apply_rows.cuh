@@ -1,9 +1,9 @@
 // apply_rows.cuh -- y = H x over bundles of hi blocks whose x lies interleaved
-// in shared memory: the kernel that large sectors take.
+// in shared memory: the apply of the single-instance and of the batched engine.
 //
-// The bundle apply (apply_blocks.cuh) spends 20 to 30 instructions on every
-// term of a row: bounds and padding tests per term, a coupling look-up and a
-// table entry per term and block, the test for the diagonal's column.  Here
+// The tile apply (apply.cuh) spends 20 to 30 instructions on every term of a
+// row: bounds and padding tests per term, a table entry and a coupling per term
+// and block, the test for the diagonal's column.  Here
 //   * x of the bundle's B blocks is staged row by row (row r of all B blocks
 //     side by side, 16 or 8 bytes), so that one lo-table entry, one coupling
 //     and one shared load serve the lo-part flip of all B blocks;
@@ -12,10 +12,21 @@
 //     larger ones: a warp walks its slice with a uniform trip count, the
 //     diagonal falls between the two parts, and a padding entry adds 0 * 0
 //     from a row of zeros (a row's sum is never -0, so that changes no bit);
-//   * an entry holds the byte offsets of its x row and of its coupling.
-// Rows add their terms in the order of the other applies (FP64: the explicit
+//   * an entry holds the byte offsets of its x row and of its coupling;
+//   * the flips outside the lo part come from a program formed once per handle,
+//     their loads out together for all blocks.
+// Rows add their terms in the order of the tile apply (FP64: the explicit
 // matrix's columns), and the <x, y> partials have their thread order and tree:
 // they are formed from the finished rows, after the bundle.
+//
+// Bound by the latency of the x loads outside the lo part (L2 and, above its
+// size, DRAM) behind 32 warps per SM; part costs on 6x5 FP32 (3.93 ms, a copy
+// with one part left out): hi-part flips 1.15 ms, crossing 1.48, lo-part 0.83;
+// L=28 FP64 (1.34 ms): outside the lo part 0.83, lo-part 0.29.
+// Measured (one box, with partials, us; the bundle apply before: one block of x
+// in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1396 (1684), FP32
+// 786 (1102); 6x5 FP64 6930 (8730), FP32 3970 (5570); L=24 FP64 92 (133), FP32
+// 60 (88); L=16 FP64 8.4 (18.4).
 //
 // Reference paths are relative to the ALPS source tree.
 #pragma once
@@ -397,13 +408,13 @@ template <typename T, typename Acc, int B, int NT, int U, int UC>
 __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restrict__ x, T* y,
                                             double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
                                             unsigned char* prog, unsigned char* other,
-                                            const unsigned char* __restrict__ next, int stride, int cap) {
+                                            const unsigned char* __restrict__ next, int next_bytes, int cap) {
   constexpr bool kOrdered = sizeof(T) == 8;
   using Row = RowVec<T, B>;
   Row* rows = reinterpret_cast<Row*>(xs);
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();  // this program is here; the previous bundle is done with x, red and `other`
-  if (next) fetch_program<NT>(next, other, stride);
+  if (next) fetch_program<NT>(next, other, next_bytes);
   const RowHead& hd = *reinterpret_cast<const RowHead*>(prog);
   const Program pg = program_at<B>(prog, cap);
   const int nv = hd.nv;

@@ -16,7 +16,7 @@
 // longer stall on dependent global loads.
 //
 // Each row adds its terms in the same order as the tile and bundle applies
-// (apply.cuh, apply_blocks.cuh), so FP64 rows are bit-identical to
+// (apply.cuh, apply_rows.cuh), so FP64 rows are bit-identical to
 // y = prod(M, x) of the reference's explicit matrix
 // (src/ietl/interface/ublas.h:57-63 over hamiltonian_matrix.hpp:307-345),
 // FP32 rows are identical to the other variants', and the <x, y> partials

@@ -19,7 +19,7 @@
 #include <cfloat>
 
 #include "apply.cuh"
-#include "apply_blocks.cuh"
+#include "apply_rows.cuh"
 #include "batch.cuh"
 #include "reduce.cuh"
 #include "rr_core.h"
@@ -30,8 +30,6 @@ namespace {
 
 using apply::AccExact64;
 using apply::AccWide32;
-using apply::ApplyCtx;
-using apply::ApplySmem;
 
 
 __device__ __forceinline__ bool stepping(const BInst& I) {
@@ -45,68 +43,81 @@ __device__ __forceinline__ float* low_vec(const BInst& I, int j) {
 }
 __device__ __forceinline__ double* high_vec(const BInst& I, int j) { return I.v64[j % 3]; }
 
-// The apply of every stepping instance over its (instance, bundle) items: the
-// bundle apply (apply_blocks.cuh) with the instance's tables; the staged
-// pairs and the shared-memory layout change with the instance.  FP32 vectors:
-// one kernel per sector-size bucket (the rows of the largest hi block,
-// maxrows in (mr_lo, mr_hi]), each a template instance picked for its bucket
-// by the autotuner (batch_tune_bucket): R rows per thread, MINB CTAs per SM,
-// B = 1 (the item's hi blocks one at a time) or kBatchBundle (both at once).
-// FP64 vectors (b_hv64): 4 rows per thread, 3 CTAs per SM.
-template <int R, int MINB, int B>
-__global__ void __launch_bounds__(kHvThreads, MINB) b_hv32(BatchArgs a, int bucket, int mr_lo, int mr_hi) {
-  static_assert(B == 1 || B == kBatchBundle, "an item is one bundle or its blocks one by one");
-  extern __shared__ __align__(16) unsigned char b_dyn[];
-  __shared__ bapply::BundleSmem<B> sm;
-  const int i0 = a.tile_start[bucket], i1 = a.tile_start[bucket + 1];  // this bucket's items
-  int cur = -1, rc = 0;
-  float* xs = nullptr;
-  for (int it = i0 + (int)blockIdx.x; it < i1; it += gridDim.x) {
-    const BItem w = a.tiles[it];
-    const BInst& I = a.inst[w.inst];
-    if (I.phase != kPhLow || !stepping(I) || I.t.maxrows <= mr_lo || I.t.maxrows > mr_hi)
-      continue;  // same for every thread of the CTA
-    const int j = I.j;
-    if (w.inst != cur) {
-      __syncthreads();  // the previous block is done with the staged pairs
-      xs = bapply::carve<float, B>(*I.P, I.t, b_dyn, sm);
-      bapply::stage_pairs<B>(*I.P, sm);
-      cur = w.inst;
+// The applies over the (instance, bundle) items: the rows apply (apply_rows.cuh)
+// with the instance's tables.  A CTA walks the items that `valid` takes; the
+// next item's program is on its way while one runs, and the tables, the
+// couplings and the row of zeros are staged when the instance changes.
+// Shared memory: two programs of at most `prog` bytes, then the x rows.
+// run(I, t, apply) calls apply(x, y, alpha_part) for every vector pair.
+struct RowsCta {
+  rapply::RowsSmem rows;
+  __align__(16) unsigned char tables[sizeof(DevTables)];
+};
+
+template <typename T, typename Acc, int NT, class Valid, class Run>
+__device__ __forceinline__ void rows_items(const BatchArgs& a, int i0, int i1, int prog, unsigned char* dyn,
+                                           RowsCta& sm, Valid&& valid, Run&& run) {
+  constexpr int B = kBatchBundle, kEl = sizeof(T) == 8 ? 0 : 1, kTab = sizeof(T) * B == 16 ? 0 : 1;
+  auto find = [&](int it) {  // same for every thread of the CTA
+    while (it < i1 && !valid(a.inst[a.tiles[it].inst])) it += gridDim.x;
+    return it;
+  };
+  unsigned char* xs = dyn + 2 * (size_t)prog;
+  DevTables& t = *reinterpret_cast<DevTables*>(sm.tables);
+  int it = find(i0 + (int)blockIdx.x), cur = -1, w = 0;
+  if (it < i1) {
+    const BItem q = a.tiles[it];
+    const DevTables& ti = a.inst[q.inst].t;
+    rapply::fetch_program<NT>(ti.rprog[kEl][kTab] + (int64_t)q.idx * ti.rstride[kEl][kTab], dyn, ti.rstride[kEl][kTab]);
+  }
+  while (it < i1) {
+    const BInst& I = a.inst[a.tiles[it].inst];
+    const int nit = find(it + (int)gridDim.x);
+    const unsigned char* next = nullptr;
+    int next_bytes = 0;
+    if (nit < i1) {
+      const BItem q = a.tiles[nit];
+      const DevTables& tn = a.inst[q.inst].t;
+      next_bytes = tn.rstride[kEl][kTab];
+      next = tn.rprog[kEl][kTab] + (int64_t)q.idx * next_bytes;
     }
-    const ApplyCtx c = apply::ctx_of(*I.P);
-    if (B == kBatchBundle) {  // both blocks of the item at once
-      bapply::apply_bundle<float, AccWide32, R, B>(c, I.t, w.idx, low_vec(I, j), low_vec(I, j + 1), I.partA, sm, xs,
-                                                   rc);
-    } else {
-      for (int q = 0; q < kBatchBundle; ++q)  // the item's blocks one at a time (block-list entries)
-        bapply::apply_bundle<float, AccWide32, R, B>(c, I.t, (int64_t)w.idx * kBatchBundle + q, low_vec(I, j),
-                                                     low_vec(I, j + 1), I.partA, sm, xs, rc);
+    if (a.tiles[it].inst != cur) {
+      cur = a.tiles[it].inst;
+      __syncthreads();  // the previous item is done with the tables, the couplings and x
+      for (int q = threadIdx.x; q < (int)(sizeof(DevTables) / 4); q += NT)
+        reinterpret_cast<uint32_t*>(sm.tables)[q] = reinterpret_cast<const uint32_t*>(&I.t)[q];
+      for (int q = threadIdx.x; q <= I.t.n_lolo; q += NT) sm.rows.lolo_c[q] = q < I.t.n_lolo ? I.t.lolo_c[q] : 0.0;
+      if (threadIdx.x < B) reinterpret_cast<T*>(xs)[(size_t)I.t.maxrows * B + threadIdx.x] = T(0);
     }
+    run(I, [&](const T* x, T* y, double* alpha_part, bool last) {
+      rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(t, x, y, alpha_part, sm.rows, xs, dyn + w * prog,
+                                                                  dyn + (w ^ 1) * prog, last ? next : nullptr,
+                                                                  next_bytes, I.t.rcap[kEl][kTab]);
+    });
+    it = nit;
+    w ^= 1;
   }
 }
 
-__global__ void __launch_bounds__(kHvThreads, 3) b_hv64(BatchArgs a) {
+// FP32 vectors: one kernel per sector-size bucket (the rows of the largest hi
+// block, maxrows in (mr_lo, mr_hi]), each a template instance picked for its
+// bucket by the autotuner (batch_tune_bucket).
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) b_hv32(BatchArgs a, int bucket, int mr_lo, int mr_hi) {
   extern __shared__ __align__(16) unsigned char b_dyn[];
-  __shared__ bapply::BundleSmem<1> sm;
-  const int n = *a.n_tiles;
-  int cur = -1, rc = 0;
-  double* xs = nullptr;
-  for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    const BItem w = a.tiles[it];
-    const BInst& I = a.inst[w.inst];
-    if (I.phase != kPhHigh || !stepping(I)) continue;
-    const int j = I.j;
-    if (w.inst != cur) {
-      __syncthreads();
-      xs = bapply::carve<double, 1>(*I.P, I.t, b_dyn, sm);
-      bapply::stage_pairs<1>(*I.P, sm);
-      cur = w.inst;
-    }
-    const ApplyCtx c = apply::ctx_of(*I.P);
-    for (int q = 0; q < kBatchBundle; ++q)  // the item's blocks one at a time (block-list entries)
-      bapply::apply_bundle<double, AccExact64, 4, 1>(c, I.t, (int64_t)w.idx * kBatchBundle + q, high_vec(I, j),
-                                                     high_vec(I, j + 1), I.partA, sm, xs, rc);
-  }
+  __shared__ RowsCta sm;
+  rows_items<float, AccWide32, NT>(
+      a, a.tile_start[bucket], a.tile_start[bucket + 1], a.prog32, b_dyn, sm,
+      [&](const BInst& I) { return I.phase == kPhLow && stepping(I) && I.t.maxrows > mr_lo && I.t.maxrows <= mr_hi; },
+      [](const BInst& I, auto&& apply) { apply(low_vec(I, I.j), low_vec(I, I.j + 1), I.partA, true); });
+}
+
+__global__ void __launch_bounds__(kHvThreads, 4) b_hv64(BatchArgs a) {
+  extern __shared__ __align__(16) unsigned char b_dyn[];
+  __shared__ RowsCta sm;
+  rows_items<double, AccExact64, kHvThreads>(
+      a, 0, *a.n_tiles, a.prog64, b_dyn, sm, [](const BInst& I) { return I.phase == kPhHigh && stepping(I); },
+      [](const BInst& I, auto&& apply) { apply(high_vec(I, I.j), high_vec(I, I.j + 1), I.partA, true); });
 }
 
 __global__ void __launch_bounds__(256) b_alpha(BatchArgs a) {
@@ -475,7 +486,7 @@ __global__ void __launch_bounds__(32) b_check(BatchArgs a) {
 // The single-instance refinement of lanczos.cpp (rayleigh_ritz) for every
 // request whose FP32 phase ended at this graph launch: the K Ritz vectors of
 // T that span its nev lowest clusters are formed in FP64 from the stored
-// basis, H is applied to each (the FP64 bundle apply), the Gram matrices
+// basis, H is applied to each (the FP64 rows apply), the Gram matrices
 // Psi^T Psi and Psi^T H Psi are summed per chunk and finished per request,
 // one thread per request solves the K x K pencil (rr_core.h), the residuals
 // of the pairs below the FP32 phase's gap bound are summed, and the block
@@ -523,29 +534,15 @@ __global__ void __launch_bounds__(kRedThreads) b_rr_combine(BatchArgs a) {
   }
 }
 
-// H Psi_k for k < K over the request's (bundle) items: the FP64 bundle apply.
-__global__ void __launch_bounds__(kHvThreads, 3) b_rr_apply(BatchArgs a) {
+// H Psi_k for k < K over the request's (bundle) items: the FP64 rows apply.
+__global__ void __launch_bounds__(kHvThreads, 4) b_rr_apply(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char b_dyn[];
-  __shared__ bapply::BundleSmem<1> sm;
-  const int n = *a.n_tiles;
-  int cur = -1, rc = 0;
-  double* xs = nullptr;
-  for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    const BItem w = a.tiles[it];
-    const BInst& I = a.inst[w.inst];
-    if (I.phase != kPhRR) continue;
-    if (w.inst != cur) {
-      __syncthreads();
-      xs = bapply::carve<double, 1>(*I.P, I.t, b_dyn, sm);
-      bapply::stage_pairs<1>(*I.P, sm);
-      cur = w.inst;
-    }
-    const ApplyCtx c = apply::ctx_of(*I.P);
-    for (int k = 0; k < I.rr_k; ++k)
-      for (int q = 0; q < kBatchBundle; ++q)
-        bapply::apply_bundle<double, AccExact64, 4, 1>(c, I.t, (int64_t)w.idx * kBatchBundle + q, rr_psi(I, k),
-                                                       rr_img(I, k), nullptr, sm, xs, rc);
-  }
+  __shared__ RowsCta sm;
+  rows_items<double, AccExact64, kHvThreads>(
+      a, 0, *a.n_tiles, a.prog64, b_dyn, sm, [](const BInst& I) { return I.phase == kPhRR && I.rr_k > 0; },
+      [](const BInst& I, auto&& apply) {
+        for (int k = 0; k < I.rr_k; ++k) apply(rr_psi(I, k), rr_img(I, k), nullptr, k + 1 == I.rr_k);
+      });
 }
 
 // Chunk partials of the Gram matrices: G(a, b), a <= b, then A(a, b) =
@@ -850,27 +847,30 @@ int sms() {
 }
 
 // The FP32 apply candidates of the autotuner.  Every candidate adds each
-// row's terms in the same order (apply_blocks.cuh), so the choice changes the
+// row's terms in the same order (apply_rows.cuh), so the choice changes the
 // speed, not the results.
 struct Cand32 {
   void (*kern)(BatchArgs, int, int, int);
+  int threads;
   const char* name;
 };
 const Cand32 kCand32[kBatchCand32] = {
-    {b_hv32<1, 6, 1>, "r1b6"},          {b_hv32<2, 4, kBatchBundle>, "blk2r2b4"}, {b_hv32<2, 4, 1>, "r2b4"},
-    {b_hv32<1, 4, kBatchBundle>, "blk2r1b4"}, {b_hv32<4, 3, 1>, "r4b3"},
+    {b_hv32<128, 8>, 128, "n128"},
+    {b_hv32<256, 4>, 256, "n256"},
+    {b_hv32<512, 2>, 512, "n512"},
+    {b_hv32<1024, 1>, 1024, "n1024"},
 };
-int g_c32[kBatchCand32] = {}, g_c32_smem[kBatchCand32] = {-1, -1, -1, -1, -1};
+int g_c32[kBatchCand32] = {}, g_c32_smem[kBatchCand32] = {-1, -1, -1, -1};
 int g_hv64 = 0, g_hv64_smem = -1;
 int g_rr = 0, g_rr_smem = -1;
 
 // Grid of an apply kernel for `smem` bytes of dynamic shared memory (cached per size).
 template <typename K>
-int hv_grid(K kern, int smem, int* g, int* g_smem) {
+int hv_grid(K kern, int threads, int smem, int* g, int* g_smem) {
   if (smem != *g_smem) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kHvThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem);
     *g = sms() * (per < 1 ? 1 : per);
     *g_smem = smem;
   }
@@ -885,10 +885,8 @@ int check(const char* what) {
 
 }  // namespace
 
-size_t batch_hv_smem_bytes(int maxrows, const HvParams& P) {
-  const size_t f64 = bapply::bundle_smem_bytes<double>(1, maxrows, P.n_pairs, P.n_lolo);
-  const size_t f32 = bapply::bundle_smem_bytes<float>(kBatchBundle, maxrows, P.n_pairs, P.n_lolo);
-  return f64 > f32 ? f64 : f32;
+size_t batch_hv_smem_bytes(int elem, int maxrows, int prog) {
+  return 2 * (size_t)prog + (((size_t)(maxrows + 1) * elem * kBatchBundle + 15) & ~(size_t)15);
 }
 
 size_t batch_hv_smem_limit() {
@@ -907,9 +905,10 @@ size_t batch_hv_smem_limit() {
 }
 
 int batch_prepare(const BatchArgs& a) {
-  for (int c = 0; c < kBatchCand32; ++c) hv_grid(kCand32[c].kern, a.hv_smem, &g_c32[c], &g_c32_smem[c]);
-  hv_grid(b_hv64, a.hv_smem, &g_hv64, &g_hv64_smem);
-  hv_grid(b_rr_apply, a.hv_smem, &g_rr, &g_rr_smem);
+  for (int c = 0; c < kBatchCand32; ++c)
+    hv_grid(kCand32[c].kern, kCand32[c].threads, a.hv_smem, &g_c32[c], &g_c32_smem[c]);
+  hv_grid(b_hv64, kHvThreads, a.hv_smem64, &g_hv64, &g_hv64_smem);
+  hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, &g_rr, &g_rr_smem);
   return check("batched apply attributes");
 }
 
@@ -926,8 +925,9 @@ int batch_launch_hv32(const BatchArgs& a, int cand, int bucket, cudaStream_t st)
     return fail(AED_ERR_INVALID, "batched apply: bad candidate or bucket");
   const int lo = bucket == 0 ? -1 : kBatchBucketHi[bucket - 1];
   const int hi = bucket + 1 == kBatchBuckets ? 0x7fffffff : kBatchBucketHi[bucket];
-  kCand32[cand].kern<<<hv_grid(kCand32[cand].kern, a.hv_smem, &g_c32[cand], &g_c32_smem[cand]), kHvThreads,
-                       a.hv_smem, st>>>(a, bucket, lo, hi);
+  const Cand32& k = kCand32[cand];
+  k.kern<<<hv_grid(k.kern, k.threads, a.hv_smem, &g_c32[cand], &g_c32_smem[cand]), k.threads, a.hv_smem, st>>>(
+      a, bucket, lo, hi);
   return check("batched FP32 apply");
 }
 
@@ -973,7 +973,7 @@ int batch_record_step(const BatchArgs& a, const int* choice32, cudaStream_t st) 
     const int rc = batch_launch_hv32(a, choice32[b], b, st);
     if (rc) return rc;
   }
-  b_hv64<<<hv_grid(b_hv64, a.hv_smem, &g_hv64, &g_hv64_smem), kHvThreads, a.hv_smem, st>>>(a);
+  b_hv64<<<hv_grid(b_hv64, kHvThreads, a.hv_smem64, &g_hv64, &g_hv64_smem), kHvThreads, a.hv_smem64, st>>>(a);
   b_alpha<<<ni, 256, 0, st>>>(a);
   b_update<<<gchunk, kRedThreads, 0, st>>>(a);
   b_beta<<<ni, 256, 0, st>>>(a);
@@ -987,7 +987,7 @@ int batch_record_check(const BatchArgs& a, cudaStream_t st) {
   const int gchunk = sms() * 8;
   b_check<<<ni, 32, 0, st>>>(a);
   b_rr_combine<<<gchunk, kRedThreads, 0, st>>>(a);
-  b_rr_apply<<<hv_grid(b_rr_apply, a.hv_smem, &g_rr, &g_rr_smem), kHvThreads, a.hv_smem, st>>>(a);
+  b_rr_apply<<<hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, &g_rr, &g_rr_smem), kHvThreads, a.hv_smem64, st>>>(a);
   b_rr_gram<<<gchunk, kRedThreads, 0, st>>>(a);
   b_rr_finish<<<ni, 256, 0, st>>>(a, 0);
   b_rr_solve<<<(ni + 127) / 128, 128, 0, st>>>(a);

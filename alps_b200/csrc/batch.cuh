@@ -112,21 +112,24 @@ struct BatchArgs {
   BItem* chunks;
   int32_t* n_chunks;
   int max_inst;
-  int hv_smem;         // dynamic shared memory of the apply (batch_hv_smem_bytes, max over residents)
+  // dynamic shared memory of the FP32 and FP64 applies and the bytes of a
+  // program in it (batch_hv_smem_bytes, max over residents)
+  int hv_smem, hv_smem64, prog32, prog64;
   // tiles are ordered by FP32 size bucket: bucket b's items are [tile_start[b], tile_start[b + 1])
   // (kBatchBuckets + 1 offsets, device), so each bucket's apply walks only its own items
   int32_t* tile_start;
 };
 
-// Hi blocks per work item of the batched apply (entries ub * kBatchBundle ..
-// of a sector's block list, applied one block at a time).
+// Hi blocks per work item of the batched apply: entries ub * kBatchBundle .. of
+// a sector's block list, one bundle of the rows apply (FP32 vectors: rows of 8
+// bytes, FP64: 16).
 constexpr int kBatchBundle = 2;
-// Dynamic shared memory the batched apply needs for one instance (the larger
-// of its FP64 layout, one block, and its FP32 layout, two blocks).
-size_t batch_hv_smem_bytes(int maxrows, const HvParams& P);
+// Dynamic shared memory of the apply of vectors of `elem` bytes an element for
+// a sector of `maxrows` rows in its largest block and programs of `prog` bytes.
+size_t batch_hv_smem_bytes(int elem, int maxrows, int prog);
 // Largest dynamic shared memory a CTA of the batched apply may take on this device.
 size_t batch_hv_smem_limit();
-// Set the apply kernels' shared-memory limits for a.hv_smem; call before capturing.
+// Set the apply kernels' shared-memory limits for a.hv_smem and a.hv_smem64; call before capturing.
 int batch_prepare(const BatchArgs& a);
 // The FP32 apply is tuned per sector-size bucket: bucket b holds the sectors
 // whose largest hi block has maxrows in (kBatchBucketHi[b-1], kBatchBucketHi[b]]
@@ -134,8 +137,8 @@ int batch_prepare(const BatchArgs& a);
 // choice32[b] is bucket b's.  Untuned: kBatchDefault32[b].
 constexpr int kBatchBuckets = 4;
 constexpr int kBatchBucketHi[kBatchBuckets] = {300, 1000, 4000, 0x7fffffff};
-constexpr int kBatchCand32 = 5;
-constexpr int kBatchDefault32[kBatchBuckets] = {0, 1, 1, 1};
+constexpr int kBatchCand32 = 4;
+constexpr int kBatchDefault32[kBatchBuckets] = {0, 1, 2, 2};
 int batch_bucket_of(int maxrows);
 const char* batch_cand32_name(int c);
 int batch_launch_hv32(const BatchArgs& a, int cand, int bucket, cudaStream_t st);

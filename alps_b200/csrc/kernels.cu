@@ -112,10 +112,50 @@ __global__ void __launch_bounds__(256) row_prog_kernel(const __grid_constant__ H
     rapply::form_program<T, B, rapply::kU, rapply::kUC>(c, t, ub, sm.low, sm.rise, out + ub * stride, cap);
 }
 
-// The lo-neighbour table: one thread per lo state, its flips inserted in order
-// of their target's rank (no two share one).
+// The flips of P inside the lo part, in P's order: low[] to smaller states
+// (hi bit set), rise[] to larger ones (lo bit set) with their index in low[].
+// Each list's targets ascend, and no two flips of a state share one.
+struct LoFlips {
+  uint32_t low[kMaxBonds], hi[kMaxBonds], rise[kMaxBonds], lo[kMaxBonds];
+  uint16_t idx[kMaxBonds];
+  int n;
+};
+__device__ __forceinline__ void stage_lo_flips(const HvParams& P, LoFlips& f) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    int n = 0, m = 0;
+    for (int a0 = 0; a0 < P.n_pairs; a0 += 32) {
+      const int a = a0 + lane;
+      const bool l = a < P.n_pairs && (P.low[a].mhi >> P.Nlo) == 0u, r = a < P.n_pairs && (P.rise[a].mhi >> P.Nlo) == 0u;
+      const unsigned ml = __ballot_sync(0xffffffffu, l), mr = __ballot_sync(0xffffffffu, r);
+      const unsigned below = (1u << lane) - 1u;
+      if (l) {
+        f.low[n + __popc(ml & below)] = P.low[a].mhi | P.low[a].mlo;
+        f.hi[n + __popc(ml & below)] = P.low[a].mhi;
+      }
+      if (r) {
+        f.rise[m + __popc(mr & below)] = P.rise[a].mhi | P.rise[a].mlo;
+        f.lo[m + __popc(mr & below)] = P.rise[a].mlo;
+      }
+      n += __popc(ml);
+      m += __popc(mr);
+    }
+    if (lane == 0) f.n = n;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < f.n; q += blockDim.x) {
+    int k = 0;
+    while (f.low[k] != f.rise[q]) ++k;  // the lists hold the same flips
+    f.idx[q] = (uint16_t)k;
+  }
+  __syncthreads();
+}
+
+// The lo-neighbour table: one thread per lo state.
 __global__ void __launch_bounds__(128) lo_table_kernel(const __grid_constant__ HvParams P, const DevTables t,
                                                        uint32_t* __restrict__ ell) {
+  __shared__ LoFlips f;
+  stage_lo_flips(P, f);
   const uint32_t i = blockIdx.x * 128u + threadIdx.x;
   if (i >= 1u << t.Nlo) return;
   const uint32_t l = t.lolist[i];
@@ -123,28 +163,19 @@ __global__ void __launch_bounds__(128) lo_table_kernel(const __grid_constant__ H
   const uint32_t base = t.looff[k], nk = t.looff[k + 1] - base;
   uint32_t* E = ell + (size_t)t.ell_w * base + (i - base);
   int n = 0;
-  uint32_t q = 0;
-  for (int a = 0; a < P.n_pairs; ++a) {
-    if ((P.low[a].mhi >> t.Nlo) != 0u) continue;
-    const uint32_t f = P.low[a].mhi | P.low[a].mlo, b = l & f;
-    if (b != 0u && b != f) {
-      const uint32_t v = t.tlo[l ^ f];
-      int e = n++;
-      for (; e > 0; --e) {
-        const uint32_t w = E[(size_t)(e - 1) * nk];
-        if ((w & 0xffffu) < v) break;
-        E[(size_t)e * nk] = w;
-      }
-      E[(size_t)e * nk] = v | q << 16;
-    }
-    ++q;
-  }
+  for (int q = 0; q < f.n; ++q)
+    if ((l & f.low[q]) == f.hi[q]) E[(size_t)n++ * nk] = (uint32_t)t.tlo[l ^ f.low[q]] | (uint32_t)q << 16;
+  for (int q = 0; q < f.n; ++q)
+    if ((l & f.rise[q]) == f.lo[q]) E[(size_t)n++ * nk] = (uint32_t)t.tlo[l ^ f.rise[q]] | (uint32_t)f.idx[q] << 16;
   for (; n < t.ell_w; ++n) E[(size_t)n * nk] = kEllPad;
 }
 
 // The sliced lo-neighbour table: one warp per slice of 32 rows of a class.
-__global__ void __launch_bounds__(128) lo_slices_kernel(const DevTables t, uint32_t pad, uint2* __restrict__ e,
+__global__ void __launch_bounds__(128) lo_slices_kernel(const __grid_constant__ HvParams P, const DevTables t,
+                                                        uint32_t pad, uint2* __restrict__ e,
                                                         uint32_t* __restrict__ w) {
+  __shared__ LoFlips f;
+  stage_lo_flips(P, f);
   const int lane = threadIdx.x & 31;
   const uint32_t s = blockIdx.x * 4u + (threadIdx.x >> 5);
   int k = t.Nlo;  // the class of slice s
@@ -152,26 +183,26 @@ __global__ void __launch_bounds__(128) lo_slices_kernel(const DevTables t, uint3
   const uint32_t base = t.looff[k], nk = t.looff[k + 1] - base;
   const uint32_t r0 = (s - (base >> 5) - (uint32_t)k) * 32u, r = r0 + lane;
   if (r0 >= nk) return;  // a slice number that no class uses
-  const uint32_t* E = t.ell + (size_t)t.ell_w * base + r;
+  const uint32_t l = r < nk ? t.lolist[base + r] : 0u;  // no flip applies to 0
   int nl = 0, nu = 0;
-  if (r < nk)
-    for (int i = 0; i < t.ell_w; ++i) {
-      const uint32_t v = E[(size_t)i * nk];
-      if (v == kEllPad) break;
-      (v & 0xffffu) < r ? ++nl : ++nu;
-    }
+  for (int q = 0; q < f.n; ++q) {
+    nl += (l & f.low[q]) == f.hi[q] ? 1 : 0;
+    nu += (l & f.rise[q]) == f.lo[q] ? 1 : 0;
+  }
   const int wl = (__reduce_max_sync(0xffffffffu, nl) + 1) / 2, wu = (__reduce_max_sync(0xffffffffu, nu) + 1) / 2;
   if (lane == 0) w[s] = (uint32_t)wl | (uint32_t)wu << 16;
   uint32_t* o = reinterpret_cast<uint32_t*>(e + ((size_t)s * t.low_st * 32 + lane));
-  for (int i = 0; i < 2 * (wl + wu); ++i) {  // position i of the slice: entry i & 1 of pair i >> 1
-    const int j = i < 2 * wl ? i : i - 2 * wl + nl;
-    uint32_t v = pad;
-    if (r < nk && (i < 2 * wl ? i < nl : j < nl + nu)) {
-      const uint32_t x = E[(size_t)j * nk];
-      v = (x & 0xffffu) << 4 | ((x >> 16) * 8u) << 20;
-    }
-    o[(size_t)(i >> 1) * 64 + (i & 1)] = v;
-  }
+  int n = 0;  // position i of the slice: entry i & 1 of pair i >> 1
+  auto put = [&](uint32_t v) {
+    o[(size_t)(n >> 1) * 64 + (n & 1)] = v;
+    ++n;
+  };
+  for (int q = 0; q < f.n; ++q)
+    if ((l & f.low[q]) == f.hi[q]) put((uint32_t)t.tlo[l ^ f.low[q]] << 4 | (uint32_t)(q * 8) << 20);
+  while (n < 2 * wl) put(pad);
+  for (int q = 0; q < f.n; ++q)
+    if ((l & f.rise[q]) == f.lo[q]) put((uint32_t)t.tlo[l ^ f.rise[q]] << 4 | (uint32_t)(f.idx[q] * 8) << 20);
+  while (n < 2 * (wl + wu)) put(pad);
 }
 
 // y = H x with the flips' x segments staged by bulk copies (apply_stream.cuh).
@@ -720,6 +751,11 @@ int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaSt
 int row_blocks(int elem, int row) { return (row == 0 ? 16 : 8) / elem; }
 int row_prog_stride(int elem, int row, int cap) { return rapply::prog_stride(row_blocks(elem, row), elem, cap); }
 
+int row_cap_bound(int elem, const HvParams& P) {
+  const int n = P.n_pairs - P.n_lolo;  // FP64: two lists of either direction; FP32: the hi-part and the crossing flips
+  return ((elem == 8 ? 2 : 1) * n + 2 * rapply::kU + 1) & ~1;
+}
+
 int launch_row_need(const HvParams& P, const DevTables& t, int elem, int* need, cudaStream_t st) {
   const int64_t want = (t.n_blk / row_blocks(elem, 0) + 7) / 8, cap = (int64_t)num_sms() * 4;
   const unsigned grid = (unsigned)(want < 1 ? 1 : want < cap ? want : cap);
@@ -746,9 +782,9 @@ int launch_row_progs(const HvParams& P, const DevTables& t, int elem, int row, u
   return check_launch("row_prog_kernel");
 }
 
-int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st) {
-  const uint32_t pad = (uint32_t)pad_row << 4 | ((uint32_t)pad_c * 8u) << 20;
-  lo_slices_kernel<<<(unsigned)((lo_slices(t.Nlo) + 3) / 4), 128, 0, st>>>(t, pad, e, w);
+int launch_lo_slices(const HvParams& P, const DevTables& t, uint2* e, uint32_t* w, cudaStream_t st) {
+  const uint32_t pad = (uint32_t)t.maxrows << 4 | (uint32_t)(P.n_lolo * 8) << 20;  // the staged row of zeros, 0.0
+  lo_slices_kernel<<<(unsigned)((lo_slices(t.Nlo) + 3) / 4), 128, 0, st>>>(P, t, pad, e, w);
   return check_launch("lo_slices_kernel");
 }
 

@@ -80,12 +80,11 @@ bool hv_variant_tuned(int v);
 // (coalesced across consecutive rows).
 int launch_lo_table(const HvParams& P, const DevTables& t, uint32_t* ell, cudaStream_t st);
 
-// The sliced lo-neighbour table from t.ell (t.low_e, t.low_w, t.low_st name
-// its arrays): pad_row is the rank of padding entries (a staged row of zeros),
-// pad_c their coupling index (0.0).
+// The sliced lo-neighbour table of P's flips (DevTables::low_e, low_w; t.low_st
+// = lo_slice_pairs(P.n_lolo) and t.maxrows set).
 inline int lo_slice_pairs(int ell_w) { return 2 * ((ell_w + 1) / 2) + 1; }  // each part at most ell_w entries
 inline size_t lo_slices(int Nlo) { return ((size_t)1 << Nlo) / 32 + (size_t)Nlo + 2; }
-int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint32_t* w, cudaStream_t st);
+int launch_lo_slices(const HvParams& P, const DevTables& t, uint2* e, uint32_t* w, cudaStream_t st);
 
 // The rows apply's programs of P for vectors of `elem` bytes an element: `need`
 // (two device ints, zeroed) gets the ops per program for rows of 16 and 8 bytes;
@@ -93,6 +92,7 @@ int launch_lo_slices(const DevTables& t, int pad_row, int pad_c, uint2* e, uint3
 // set) and P's lo-part couplings into lolo_c.
 int row_blocks(int elem, int row);                 // blocks of a bundle
 int row_prog_stride(int elem, int row, int cap);   // bytes of a program
+int row_cap_bound(int elem, const HvParams& P);    // ops that hold any program of P
 int launch_row_need(const HvParams& P, const DevTables& t, int elem, int* need, cudaStream_t st);
 int launch_row_progs(const HvParams& P, const DevTables& t, int elem, int row, unsigned char* out, double* lolo_c,
                      cudaStream_t st);

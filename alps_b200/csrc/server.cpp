@@ -37,7 +37,7 @@ struct Sector {
   BasisTables tab;
   uint32_t *thi = nullptr, *looff = nullptr, *tile_h = nullptr, *tile_r = nullptr;
   uint16_t* xtab = nullptr;  // crossing-flip table
-  uint32_t *blk_h = nullptr, *tfirst = nullptr;  // block list of the bundle apply, first tile per hi block
+  uint32_t *blk_h = nullptr, *tfirst = nullptr;  // block list of the rows apply, first tile per hi block
   std::vector<uint32_t> blk;                     // host copy of the block list (work items)
   int maxrows = 0;
   uint16_t *tlo = nullptr, *lolist = nullptr;
@@ -111,7 +111,7 @@ struct aed_server {
   bool dirty = true;
   cudaGraphExec_t graph = nullptr;
   bool graph_stale = true;
-  int hv_smem = 0;  // dynamic shared memory of the apply in the graph
+  int hv_smem = 0, hv_smem64 = 0, prog32 = 0, prog64 = 0;  // shared memory of the applies in the graph (batch.cuh)
   int64_t launches = 0;
   // the FP32 apply kernel of each sector-size bucket (batch.cuh), tuned on
   // the first resident work of the bucket unless AED_BATCH_VARIANT forces one
@@ -146,7 +146,7 @@ int dmalloc(aed_server* s, void** p, size_t bytes) {
 int rr_kmax_of(int nev) { return std::min(kMaxRR, nev + 3); }
 
 // Bytes a request holds while resident (the admission footprint).
-size_t request_bytes(const aed_server* s, int N, int64_t D, int nev, int cap, int n_store) {
+size_t request_bytes(const aed_server* s, int N, int n_bonds, int64_t D, int nev, int cap, int n_store) {
   const size_t ldv = ((size_t)D * 4 + 255) & ~(size_t)255;
   size_t b = (size_t)D * 8;                      // diagonal
   b += 3 * (((size_t)D * 8 + 255) & ~(size_t)255);  // FP64 vectors
@@ -154,7 +154,9 @@ size_t request_bytes(const aed_server* s, int N, int64_t D, int nev, int cap, in
   b += (size_t)sector_tiles_est(D) * 8 + (size_t)red_chunks(D) * 8;  // partials
   b += (size_t)cap * 8 * (2 + kCheckScratch + 1);                               // alpha/beta, scratch, coefficients
   b += sizeof(HvParams) + 4096;
-  b += (size_t)40 * ((size_t)1 << ((N + 1) / 2)) * 4;  // lo-neighbour table (width <= 40)
+  const int nlo = std::max((N + 1) / 2, std::min(12, N - 2)), pairs = std::min(n_bonds, kMaxBonds);
+  b += lo_slices(nlo) * ((size_t)lo_slice_pairs(pairs) * 256 + 4);  // lo-neighbour table
+  b += ((size_t)1 << (N - nlo)) * (2 * sizeof(double) * 2 * (size_t)(pairs + 8) + 128);  // the applies' programs
   if (s->precision == AED_FP32) {  // the Rayleigh-Ritz hand-over: K vectors and their images, sums
     const size_t k = (size_t)rr_kmax_of(nev);
     b += 2 * k * (((size_t)D * 8 + 255) & ~(size_t)255) + k * (size_t)cap * 8 +
@@ -253,12 +255,29 @@ int admit(aed_server* s, int k, const std::shared_ptr<Request>& r) {
   I = BInst{};
   HvParams P;
   if ((rc = build_hv_params(r->model, sec->tab.Nlo, P))) return rc;
-  const size_t smem = batch_hv_smem_bytes(sec->maxrows, P);
-  if (smem > batch_hv_smem_limit())
-    return fail(AED_ERR_INVALID, "sector too large for the batched apply's shared memory");
-  if ((int)smem > s->hv_smem) {  // the graph's apply needs more shared memory: capture again
-    s->hv_smem = (int)((smem + 1023) & ~(size_t)1023);
-    s->graph_stale = true;
+  DevTables& t = I.t;
+  for (int e = 0; e < 2; ++e) {  // the applies' programs: FP64 rows of 16 bytes, FP32 rows of 8 (kBatchBundle blocks)
+    const int elem = e == 0 ? 8 : 4;
+    t.rcap[e][e] = row_cap_bound(elem, P);
+    t.rstride[e][e] = row_prog_stride(elem, e, t.rcap[e][e]);
+  }
+  {  // the graph's applies need more shared memory: capture again
+    const int p64 = std::max(s->prog64, t.rstride[0][0]), p32 = std::max(s->prog32, t.rstride[1][1]);
+    const size_t m64 = batch_hv_smem_bytes(8, sec->maxrows, p64), m32 = batch_hv_smem_bytes(4, sec->maxrows, p32);
+    if (std::max(m64, m32) > batch_hv_smem_limit())
+      return fail(AED_ERR_INVALID, "sector too large for the batched apply's shared memory");
+    const size_t grow64 = 2 * (size_t)(p64 - s->prog64), grow32 = 2 * (size_t)(p32 - s->prog32);
+    const size_t n64 = std::max(m64, s->hv_smem64 + grow64), n32 = std::max(m32, s->hv_smem + grow32);
+    if (p64 > s->prog64 || p32 > s->prog32 || n64 > (size_t)s->hv_smem64 || n32 > (size_t)s->hv_smem) {
+      const size_t lim = batch_hv_smem_limit();
+      if (std::max(n64, n32) > lim)
+        return fail(AED_ERR_INVALID, "sector too large for the batched apply's shared memory");
+      s->prog64 = p64;
+      s->prog32 = p32;
+      s->hv_smem64 = (int)std::min(lim, (n64 + 1023) & ~(size_t)1023);
+      s->hv_smem = (int)std::min(lim, (n32 + 1023) & ~(size_t)1023);
+      s->graph_stale = true;
+    }
   }
   const int cap = cap_of(*r, D);
   const int n_store = s->precision == AED_FP32 ? std::min(kServerStore, std::min(cap + 1, kBatchMaxChunks * kStoreChunkB)) : 0;
@@ -296,7 +315,6 @@ int admit(aed_server* s, int k, const std::shared_ptr<Request>& r) {
     if ((rc = take((void**)&I.chunk[c], vb * kStoreChunkB))) return rc;
   cudaMemcpyAsync(pP, &P, sizeof(HvParams), cudaMemcpyHostToDevice, s->stream);
   I.P = (const HvParams*)pP;
-  DevTables& t = I.t;
   t.thi = sec->thi;
   t.tlo = sec->tlo;
   t.lolist = sec->lolist;
@@ -315,11 +333,22 @@ int admit(aed_server* s, int k, const std::shared_ptr<Request>& r) {
   t.n_up = sec->tab.n_up;
   t.dg = (const double*)pdg;
   {
-    void* pe = nullptr;
-    t.ell_w = P.n_lolo;
-    if ((rc = take(&pe, ((size_t)t.ell_w << t.Nlo) * 4 + 4))) return rc;
-    t.ell = (const uint32_t*)pe;
-    if ((rc = launch_lo_table(P, t, (uint32_t*)pe, s->stream))) return rc;
+    void *pe = nullptr, *pw = nullptr, *pp = nullptr;
+    t.low_st = lo_slice_pairs(P.n_lolo);
+    const size_t slices = lo_slices(t.Nlo);
+    if ((rc = take(&pe, slices * (size_t)t.low_st * 32 * sizeof(uint2))) || (rc = take(&pw, slices * 4))) return rc;
+    t.low_e = (const uint2*)pe;
+    t.low_w = (const uint32_t*)pw;
+    if ((rc = launch_lo_slices(P, t, (uint2*)pe, (uint32_t*)pw, s->stream))) return rc;
+    t.n_lolo = P.n_lolo;
+    double* lolo = (double*)((char*)pP + offsetof(HvParams, lolo_c));  // of the device copy
+    t.lolo_c = lolo;
+    for (int e = 0; e < 2; ++e) {
+      if (e == 1 && s->precision != AED_FP32) continue;
+      if ((rc = take(&pp, (size_t)(t.n_blk / kBatchBundle) * (size_t)t.rstride[e][e]))) return rc;
+      t.rprog[e][e] = (const unsigned char*)pp;
+      if ((rc = launch_row_progs(P, t, e == 0 ? 8 : 4, e, (unsigned char*)pp, lolo, s->stream))) return rc;
+    }
   }
   if ((rc = launch_diag_table(P, t, (double*)pdg, s->stream))) return rc;
   I.D = D;
@@ -437,7 +466,7 @@ int tune_buckets(aed_server* s) {
   for (const Slot& sl : s->slots)
     if (sl.used && sl.inst.phase == kPhLow) want[batch_bucket_of(sl.inst.t.maxrows)] = true;
   BatchArgs a{s->d_inst, s->d_counts, s->d_tiles, s->d_counts + 1, s->d_chunks, s->d_counts + 2, s->max_slots,
-              s->hv_smem, s->d_counts + kBucketStarts};
+              s->hv_smem, s->hv_smem64, s->prog32, s->prog64, s->d_counts + kBucketStarts};
   for (int b = 0; b < kBatchBuckets; ++b) {
     if (!want[b] || s->tuned32[b]) continue;
     int rc = batch_prepare(a);
@@ -514,7 +543,7 @@ int capture_graph(aed_server* s) {
     s->graph = nullptr;
   }
   BatchArgs a{s->d_inst, s->d_counts, s->d_tiles, s->d_counts + 1, s->d_chunks, s->d_counts + 2, s->max_slots,
-              s->hv_smem, s->d_counts + kBucketStarts};
+              s->hv_smem, s->hv_smem64, s->prog32, s->prog64, s->d_counts + kBucketStarts};
   cudaGraph_t g = nullptr;
   const int rp = batch_prepare(a);
   if (rp) return rp;
@@ -678,7 +707,7 @@ int aed_server_submit(aed_server* s, const aed_model_desc* model, const aed_solv
   r->dim = t.D;
   const int cap = cap_of(*r, t.D);
   const int n_store = s->precision == AED_FP32 ? std::min(kServerStore, cap + 1) : 0;
-  r->footprint = request_bytes(s, r->model.N, t.D, opts->nev, cap, n_store);
+  r->footprint = request_bytes(s, r->model.N, (int)r->model.s1.size(), t.D, opts->nev, cap, n_store);
   if (r->footprint + sector_bytes(r->model.N, r->model.n_up) > s->budget)
     return fail(AED_ERR_ADMISSION, "request footprint (" + std::to_string(r->footprint) +
                                        " bytes) exceeds the server's HBM budget (" + std::to_string(s->budget) + ")");

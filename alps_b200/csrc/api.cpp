@@ -1489,11 +1489,8 @@ int aed_lanczos_step(aed_handle* h, const void* v_prev, const void* v_cur, void*
     return fail(AED_ERR_INVALID, "Lanczos vectors must not alias");
   DeviceGuard g(h->device);
   const bool f32 = h->precision == AED_FP32;
-  h->h_scal[4] = beta_prev;
-  AED_CUDA_TRY(cudaMemcpyAsync(h->d_scal + 4, h->h_scal + 4, 8, cudaMemcpyHostToDevice, h->stream));
-  rc = lanczos_step_kernels(h, f32, v_prev, v_cur, v_next, h->d_scal + 4, h->d_scal + 0, h->d_scal + 1);
+  rc = lanczos_step_kernels(h, f32, v_prev, v_cur, v_next, beta_prev);
   if (rc) return rc;
-  AED_CUDA_TRY(cudaMemcpyAsync(h->h_scal, h->d_scal, 16, cudaMemcpyDeviceToHost, h->stream));
   AED_CUDA_TRY(cudaStreamSynchronize(h->stream));
   if (alpha) *alpha = h->h_scal[0];
   if (beta) *beta = h->h_scal[1];

@@ -191,9 +191,10 @@ int eigenvectors(aed_handle* h, const aed_solve_opts* o, int k, void* const* vec
 int64_t lanczos_state_bytes(const aed_handle* h);
 int lanczos_save(aed_handle* h, void* buf, int64_t bytes);
 int lanczos_load(aed_handle* h, const void* buf, int64_t bytes);
-// One make_step on device vectors: apply, alpha, update, beta, normalise.
-// beta_prev / alpha / beta are device scalars; v_prev may be NULL.
+// One make_step on device vectors: apply, alpha, update, beta, normalise;
+// alpha and beta end up in h_scal[0] and [1] (read after the stream).  v_prev
+// may be NULL.
 int lanczos_step_kernels(aed_handle* h, bool f32, const void* v_prev, const void* v_cur, void* v_next,
-                         const double* beta_prev, double* alpha, double* beta);
+                         double beta_prev);
 
 }  // namespace aed

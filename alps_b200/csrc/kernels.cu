@@ -347,12 +347,28 @@ __device__ __forceinline__ double update_chunk(double alpha, double b, const T* 
       return acc;
     }
   }
-  for (int64_t i = e0 + threadIdx.x; i < e1; i += kRedThreads) {
-    double w = __dsub_rn((double)y[i], __dmul_rn(alpha, (double)x[i]));
-    if (vprev) w = __dsub_rn(w, __dmul_rn(b, (double)vprev[i]));
-    const T wt = (T)w;
-    y[i] = wt;
-    acc = fma((double)wt, (double)wt, acc);
+  // eight elements' loads before their arithmetic: a small sector's few CTAs
+  // wait for memory twice per chunk instead of sixteen times
+  constexpr int U = 8;
+  for (int64_t i0 = e0 + threadIdx.x; i0 < e1; i0 += U * kRedThreads) {
+    T yv[U], xv[U], pv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * kRedThreads;
+      yv[u] = i < e1 ? y[i] : T(0);
+      xv[u] = i < e1 ? x[i] : T(0);
+      pv[u] = vprev && i < e1 ? vprev[i] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * kRedThreads;
+      if (i >= e1) break;
+      double w = __dsub_rn((double)yv[u], __dmul_rn(alpha, (double)xv[u]));
+      if (vprev) w = __dsub_rn(w, __dmul_rn(b, (double)pv[u]));
+      const T wt = (T)w;
+      y[i] = wt;
+      acc = fma((double)wt, (double)wt, acc);
+    }
   }
   return acc;
 }
@@ -421,17 +437,22 @@ __global__ void __launch_bounds__(kRedThreads) lanczos_update_kernel(const doubl
 
 // The update with alpha's finishing sum folded in: every CTA sums the
 // apply's tile partials itself (the order of finish_sum, so the same alpha to
-// the bit) and CTA 0 stores it.  For sectors with few tiles, where this saves
-// a launch per step.
+// the bit) and CTA 0 stores it, also at alpha_host (pinned host memory, may be
+// null): the host reads it there after the step's event, without a copy on the
+// stream.  beta_prev null: beta_val.  For sectors with few tiles, where this
+// saves a launch per step.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) lanczos_update_fin_kernel(
-    const double* __restrict__ alpha_part, int64_t n_apart, double* __restrict__ alpha_out, const T* __restrict__ x,
-    const T* __restrict__ vprev, const double* __restrict__ beta_prev, T* __restrict__ y, int64_t n,
-    double* __restrict__ partB) {
+    const double* __restrict__ alpha_part, int64_t n_apart, double* __restrict__ alpha_out, double* alpha_host,
+    const T* __restrict__ x, const T* __restrict__ vprev, const double* __restrict__ beta_prev, double beta_val,
+    T* __restrict__ y, int64_t n, double* __restrict__ partB) {
   __shared__ double sm[33];
   const double alpha = finish_sum_in_cta<kRedThreads>(alpha_part, n_apart, sm);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *alpha_out = alpha;
-  const double b = vprev ? *beta_prev : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *alpha_out = alpha;
+    if (alpha_host) *alpha_host = alpha;
+  }
+  const double b = vprev ? (beta_prev ? *beta_prev : beta_val) : 0.0;
   const int64_t nch = (n + kRedChunk - 1) / kRedChunk;
   for (int64_t c = blockIdx.x; c < nch; c += gridDim.x) {
     const int64_t e0 = c * kRedChunk, e1 = min(n, e0 + kRedChunk);
@@ -446,10 +467,14 @@ template <typename T>
 __global__ void __launch_bounds__(kRedThreads) lanczos_normalize_fin_kernel(const double* __restrict__ beta_part,
                                                                            int64_t n_bpart,
                                                                            double* __restrict__ beta_out,
-                                                                           T* __restrict__ y, int64_t n) {
+                                                                           double* beta_host, T* __restrict__ y,
+                                                                           int64_t n) {
   __shared__ double sm[33];
   const double beta = sqrt(finish_sum_in_cta<kRedThreads>(beta_part, n_bpart, sm));
-  if (blockIdx.x == 0 && threadIdx.x == 0) *beta_out = beta;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *beta_out = beta;
+    if (beta_host) *beta_host = beta;
+  }
   normalize_elems(beta, y, n);
 }
 
@@ -860,19 +885,20 @@ int launch_lanczos_update(const double* alpha, const T* x, const T* vprev, const
 }
 
 template <typename T>
-int launch_lanczos_update_fin(const double* alpha_part, int64_t n_apart, double* alpha, const T* x, const T* vprev,
-                              const double* beta_prev, T* y, int64_t n, double* partB, cudaStream_t st) {
+int launch_lanczos_update_fin(const double* alpha_part, int64_t n_apart, double* alpha, double* alpha_host, const T* x,
+                              const T* vprev, const double* beta_prev, double beta_val, T* y, int64_t n, double* partB,
+                              cudaStream_t st) {
   const int64_t nch = red_chunks(n);
   const int grid = (int)(nch < (int64_t)num_sms() * 8 ? nch : (int64_t)num_sms() * 8);
-  lanczos_update_fin_kernel<T><<<grid < 1 ? 1 : grid, kRedThreads, 0, st>>>(alpha_part, n_apart, alpha, x, vprev,
-                                                                           beta_prev, y, n, partB);
+  lanczos_update_fin_kernel<T><<<grid < 1 ? 1 : grid, kRedThreads, 0, st>>>(
+      alpha_part, n_apart, alpha, alpha_host, x, vprev, beta_prev, beta_val, y, n, partB);
   return check_launch("lanczos_update_fin_kernel");
 }
 
 template <typename T>
-int launch_lanczos_normalize_fin(const double* beta_part, int64_t n_bpart, double* beta, T* y, int64_t n,
-                                 cudaStream_t st) {
-  lanczos_normalize_fin_kernel<T><<<elem_grid(n), kRedThreads, 0, st>>>(beta_part, n_bpart, beta, y, n);
+int launch_lanczos_normalize_fin(const double* beta_part, int64_t n_bpart, double* beta, double* beta_host, T* y,
+                                 int64_t n, cudaStream_t st) {
+  lanczos_normalize_fin_kernel<T><<<elem_grid(n), kRedThreads, 0, st>>>(beta_part, n_bpart, beta, beta_host, y, n);
   return check_launch("lanczos_normalize_fin_kernel");
 }
 
@@ -891,9 +917,9 @@ int launch_lanczos_normalize(const double* beta, T* y, int64_t n, cudaStream_t s
   template int launch_lanczos_update<T>(const double*, const T*, const T*, const double*, T*, int64_t,      \
                                         double*, cudaStream_t);                                              \
   template int launch_lanczos_normalize<T>(const double*, T*, int64_t, cudaStream_t);                          \
-  template int launch_lanczos_update_fin<T>(const double*, int64_t, double*, const T*, const T*, const double*, T*, \
-                                            int64_t, double*, cudaStream_t);                                      \
-  template int launch_lanczos_normalize_fin<T>(const double*, int64_t, double*, T*, int64_t, cudaStream_t);
+  template int launch_lanczos_update_fin<T>(const double*, int64_t, double*, double*, const T*, const T*,    \
+                                            const double*, double, T*, int64_t, double*, cudaStream_t);      \
+  template int launch_lanczos_normalize_fin<T>(const double*, int64_t, double*, double*, T*, int64_t, cudaStream_t);
 AED_INST(double)
 AED_INST(float)
 #undef AED_INST

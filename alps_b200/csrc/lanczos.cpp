@@ -162,31 +162,40 @@ double diag_of_state(const HvParams& P, uint32_t s) {
   return d;
 }
 
-// After the apply x -> y (per-tile partials in h->d_partA): alpha, update,
-// beta, normalise (lanczos.h:398-402).
-int lanczos_step_tail(aed_handle* h, bool f32, const void* vprev, const void* x, void* y, const double* beta_prev,
-                      double* alpha, double* beta) {
-  const int64_t D = h->vlen;
-  const int64_t na = h->alpha_tiles(), nb = red_chunks(D);
+// Whether a step's finishing sums go into its update and normalisation.
+bool fold_finish(const aed_handle* h) {
   // AED_FOLD_FINISH=0 keeps the separate finishing kernels (a test compares
   // the two paths bit for bit)
   static const bool fold = [] {
     const char* e = std::getenv("AED_FOLD_FINISH");
     return !(e && e[0] == '0');
   }();
-  if (fold && na <= kFoldFinishMax && nb <= kFoldFinishMax) {
+  return fold && h->alpha_tiles() <= kFoldFinishMax && red_chunks(h->vlen) <= kFoldFinishMax;
+}
+
+// After the apply x -> y (per-tile partials in h->d_partA): alpha, update,
+// beta, normalise (lanczos.h:398-402).  host (pinned, may be null): receives
+// (alpha, beta), by the kernels themselves where the finishing sums are folded
+// in, by a copy on the stream otherwise.  beta_prev null: beta_val (folded
+// steps only).
+int lanczos_step_tail(aed_handle* h, bool f32, const void* vprev, const void* x, void* y, const double* beta_prev,
+                      double beta_val, double* alpha, double* beta, double* host) {
+  const int64_t D = h->vlen;
+  if (fold_finish(h)) {
     // short partial lists: the finishing sums inside the update and the
     // normalisation (same alpha and beta to the bit, two launches fewer)
+    const int64_t na = h->alpha_tiles(), nb = red_chunks(D);
+    double *ha = host, *hb = host ? host + 1 : nullptr;
     int rc;
     if (f32)
-      rc = launch_lanczos_update_fin(h->d_partA, na, alpha, (const float*)x, (const float*)vprev, beta_prev,
-                                     (float*)y, D, h->d_partB, h->stream);
+      rc = launch_lanczos_update_fin(h->d_partA, na, alpha, ha, (const float*)x, (const float*)vprev, beta_prev,
+                                     beta_val, (float*)y, D, h->d_partB, h->stream);
     else
-      rc = launch_lanczos_update_fin(h->d_partA, na, alpha, (const double*)x, (const double*)vprev, beta_prev,
-                                     (double*)y, D, h->d_partB, h->stream);
+      rc = launch_lanczos_update_fin(h->d_partA, na, alpha, ha, (const double*)x, (const double*)vprev, beta_prev,
+                                     beta_val, (double*)y, D, h->d_partB, h->stream);
     if (rc) return rc;
-    if (f32) return launch_lanczos_normalize_fin(h->d_partB, nb, beta, (float*)y, D, h->stream);
-    return launch_lanczos_normalize_fin(h->d_partB, nb, beta, (double*)y, D, h->stream);
+    if (f32) return launch_lanczos_normalize_fin(h->d_partB, nb, beta, hb, (float*)y, D, h->stream);
+    return launch_lanczos_normalize_fin(h->d_partB, nb, beta, hb, (double*)y, D, h->stream);
   }
   int rc = launch_finish_sum(h->d_partA, h->alpha_tiles(), alpha, false, h->stream);
   if (rc) return rc;
@@ -198,8 +207,16 @@ int lanczos_step_tail(aed_handle* h, bool f32, const void* vprev, const void* x,
                                h->stream);
   if (!rc) rc = launch_finish_sum(h->d_partB, red_chunks(D), beta, true, h->stream);
   if (rc) return rc;
-  if (f32) return launch_lanczos_normalize(beta, (float*)y, D, h->stream);
-  return launch_lanczos_normalize(beta, (double*)y, D, h->stream);
+  rc = f32 ? launch_lanczos_normalize(beta, (float*)y, D, h->stream)
+           : launch_lanczos_normalize(beta, (double*)y, D, h->stream);
+  if (rc || !host) return rc;
+  if (beta == alpha + 1) {
+    AED_CUDA_TRY(cudaMemcpyAsync(host, alpha, 16, cudaMemcpyDeviceToHost, h->stream));
+  } else {
+    AED_CUDA_TRY(cudaMemcpyAsync(host, alpha, 8, cudaMemcpyDeviceToHost, h->stream));
+    AED_CUDA_TRY(cudaMemcpyAsync(host + 1, beta, 8, cudaMemcpyDeviceToHost, h->stream));
+  }
+  return AED_OK;
 }
 
 // Steps the device runs ahead of the host's T-matrix analysis.  A step of a
@@ -314,11 +331,11 @@ struct Recurrence {
       if (!rc) rc = launch_dot_partials((const float*)y, (const float*)y, D, h->d_partB, true, h->stream);
       if (!rc) rc = launch_finish_sum(h->d_partB, red_chunks(D), beta, true, h->stream);
       if (!rc) rc = launch_lanczos_normalize(beta, (float*)y, D, h->stream);
+      if (!rc) AED_CUDA_TRY(cudaMemcpyAsync(h_ab + 2 * j, alpha, 16, cudaMemcpyDeviceToHost, h->stream));
     } else {
-      rc = lanczos_step_tail(h, f32, vprev, x, y, bprev, d_ab + 2 * j, d_ab + 2 * j + 1);
+      rc = lanczos_step_tail(h, f32, vprev, x, y, bprev, 0.0, d_ab + 2 * j, d_ab + 2 * j + 1, h_ab + 2 * j);
     }
     if (rc) return rc;
-    AED_CUDA_TRY(cudaMemcpyAsync(h_ab + 2 * j, d_ab + 2 * j, 16, cudaMemcpyDeviceToHost, h->stream));
     AED_CUDA_TRY(cudaEventRecord(ring->ev[j % EventRing::kN], h->stream));
     return AED_OK;
   }
@@ -880,10 +897,16 @@ int solve_mixed(aed_handle* h, const double* start_host, uint64_t seed, int nev,
 }  // namespace
 
 int lanczos_step_kernels(aed_handle* h, bool f32, const void* v_prev, const void* v_cur, void* v_next,
-                         const double* beta_prev, double* alpha, double* beta) {
+                         double beta_prev) {
   int rc = handle_hv(h, f32, v_cur, v_next, h->d_partA);
   if (rc) return rc;
-  return lanczos_step_tail(h, f32, v_prev, v_cur, v_next, v_prev ? beta_prev : nullptr, alpha, beta);
+  const double* b = nullptr;
+  if (v_prev && !fold_finish(h)) {  // the separate update reads it from device memory
+    h->h_scal[4] = beta_prev;
+    AED_CUDA_TRY(cudaMemcpyAsync(h->d_scal + 4, h->h_scal + 4, 8, cudaMemcpyHostToDevice, h->stream));
+    b = h->d_scal + 4;
+  }
+  return lanczos_step_tail(h, f32, v_prev, v_cur, v_next, b, beta_prev, h->d_scal, h->d_scal + 1, h->h_scal);
 }
 
 int solve(aed_handle* h, const aed_solve_opts* o, aed_solve_result* r) {
@@ -1111,8 +1134,8 @@ int eigenvectors(aed_handle* h, const aed_solve_opts* o, int k, void* const* vec
       double* w = buf[(j + 1) % 3];
       const double* vp = j > 0 ? buf[(j + 2) % 3] : nullptr;
       if ((rc = handle_hv(h, false, vj, w, h->d_partA))) return rc;
-      if ((rc = lanczos_step_tail(h, false, vp, vj, w, j > 0 ? d_ab + 2 * (j - 1) + 1 : nullptr, d_ab + 2 * j,
-                                  d_ab + 2 * j + 1)))
+      if ((rc = lanczos_step_tail(h, false, vp, vj, w, j > 0 ? d_ab + 2 * (j - 1) + 1 : nullptr, 0.0, d_ab + 2 * j,
+                                  d_ab + 2 * j + 1, nullptr)))
         return rc;
     }
   }

@@ -77,13 +77,24 @@ __device__ __forceinline__ double finish_sum_in_cta(const double* __restrict__ p
   static_assert(NT % 32 == 0 && kFinishThreads % NT == 0, "block size");
   constexpr int kVirt = kFinishThreads / NT;  // virtual warps per real warp
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double v[kVirt];  // one load per virtual thread in flight
+#pragma unroll
+  for (int q = 0; q < kVirt; ++q) v[q] = 0.0;
+  for (int64_t i0 = 0; i0 < n; i0 += kFinishThreads) {
+    double p[kVirt];
+#pragma unroll
+    for (int q = 0; q < kVirt; ++q) {
+      const int64_t i = i0 + (w + q * (NT / 32)) * 32 + l;  // of virtual warp w + q NT / 32
+      p[q] = i < n ? part[i] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kVirt; ++q)
+      if (i0 + (w + q * (NT / 32)) * 32 + l < n) v[q] += p[q];
+  }
+#pragma unroll
   for (int q = 0; q < kVirt; ++q) {
-    const int vw = w + q * (NT / 32);  // virtual warp
-    const int vt = vw * 32 + l;        // virtual thread of finish_sum
-    double v = 0.0;
-    for (int64_t i = vt; i < n; i += kFinishThreads) v += part[i];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (l == 0) sm[vw] = v;
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    if (l == 0) sm[w + q * (NT / 32)] = v[q];
   }
   __syncthreads();
   if (w == 0) {

@@ -59,6 +59,8 @@ __global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const 
   if (ub < nb) rapply::fetch_program<NT>(src + ub * stride, prog, stride);
   for (int q = threadIdx.x; q <= t.n_lolo; q += NT) sm.lolo_c[q] = q < t.n_lolo ? __ldg(t.lolo_c + q) : 0.0;
   if (threadIdx.x < B) reinterpret_cast<T*>(hvr_dyn)[(size_t)t.maxrows * B + threadIdx.x] = T(0);
+  chain_next();
+  chain_wait();
   int w = 0;
   for (; ub < nb; ub += gridDim.x, w ^= 1)
     rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(
@@ -295,6 +297,8 @@ __global__ void copy_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t 
 // y += a*x, as ublas evaluates v += s*w: the product rounds, then the sum.
 template <typename T>
 __global__ void axpy_kernel(double a, const T* __restrict__ x, T* __restrict__ y, int64_t n) {
+  chain_next();
+  chain_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (T)__dadd_rn((double)y[i], __dmul_rn(a, (double)x[i]));
 }
@@ -447,6 +451,8 @@ __global__ void __launch_bounds__(kRedThreads) lanczos_update_fin_kernel(
     const T* __restrict__ x, const T* __restrict__ vprev, const double* __restrict__ beta_prev, double beta_val,
     T* __restrict__ y, int64_t n, double* __restrict__ partB) {
   __shared__ double sm[33];
+  chain_next();
+  chain_wait();
   const double alpha = finish_sum_in_cta<kRedThreads>(alpha_part, n_apart, sm);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *alpha_out = alpha;
@@ -470,6 +476,8 @@ __global__ void __launch_bounds__(kRedThreads) lanczos_normalize_fin_kernel(cons
                                                                            double* beta_host, T* __restrict__ y,
                                                                            int64_t n) {
   __shared__ double sm[33];
+  chain_next();
+  chain_wait();
   const double beta = sqrt(finish_sum_in_cta<kRedThreads>(beta_part, n_bpart, sm));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *beta_out = beta;
@@ -646,7 +654,7 @@ int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double*
   const int64_t nb = t.n_blk / B;
   if (g > nb) g = nb;
   if (g < 1) return AED_OK;
-  kern<<<(unsigned)g, NT, dyn, st>>>(t, x, y, alpha_part);
+  launch_chained(kern, (unsigned)g, NT, dyn, st, t, x, y, alpha_part);
   return check_launch("hvr_kernel");
 }
 
@@ -850,7 +858,7 @@ int launch_copy(const T* x, T* y, int64_t n, cudaStream_t st) {
 
 template <typename T>
 int launch_axpy(double a, const T* x, T* y, int64_t n, cudaStream_t st) {
-  axpy_kernel<T><<<elem_grid(n), 256, 0, st>>>(a, x, y, n);
+  launch_chained(axpy_kernel<T>, elem_grid(n), 256, 0, st, a, x, y, n);
   return check_launch("axpy_kernel");
 }
 
@@ -890,15 +898,16 @@ int launch_lanczos_update_fin(const double* alpha_part, int64_t n_apart, double*
                               cudaStream_t st) {
   const int64_t nch = red_chunks(n);
   const int grid = (int)(nch < (int64_t)num_sms() * 8 ? nch : (int64_t)num_sms() * 8);
-  lanczos_update_fin_kernel<T><<<grid < 1 ? 1 : grid, kRedThreads, 0, st>>>(
-      alpha_part, n_apart, alpha, alpha_host, x, vprev, beta_prev, beta_val, y, n, partB);
+  launch_chained(lanczos_update_fin_kernel<T>, grid < 1 ? 1 : grid, kRedThreads, 0, st, alpha_part, n_apart, alpha,
+                 alpha_host, x, vprev, beta_prev, beta_val, y, n, partB);
   return check_launch("lanczos_update_fin_kernel");
 }
 
 template <typename T>
 int launch_lanczos_normalize_fin(const double* beta_part, int64_t n_bpart, double* beta, double* beta_host, T* y,
                                  int64_t n, cudaStream_t st) {
-  lanczos_normalize_fin_kernel<T><<<elem_grid(n), kRedThreads, 0, st>>>(beta_part, n_bpart, beta, beta_host, y, n);
+  launch_chained(lanczos_normalize_fin_kernel<T>, elem_grid(n), kRedThreads, 0, st, beta_part, n_bpart, beta, beta_host,
+                 y, n);
   return check_launch("lanczos_normalize_fin_kernel");
 }
 

@@ -374,6 +374,8 @@ __global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, co
   __shared__ double red[kMomThreads / 32];
   const uint32_t n_base = (uint32_t)rw.n_base;
   for (uint32_t k = threadIdx.x; k < n_base; k += NT) cf[k] = __ldg(rw.cf + k);
+  chain_next();
+  chain_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const uint32_t jmask = (1u << rw.jbits) - 1u;
@@ -734,10 +736,8 @@ int mom_rows_build(const MomParams& mp, const DevTables& t, const MomTables& m, 
 template <int NT, int U, int MINB>
 void mom_rows_go(const MomRows& r, bool diag_first, unsigned grid, size_t dyn, const double2* x, double2* y,
                  double* alpha_part, cudaStream_t st) {
-  if (diag_first)
-    mom_rows_kernel<true, NT, U, MINB><<<grid, NT, dyn, st>>>(r, x, y, alpha_part);
-  else
-    mom_rows_kernel<false, NT, U, MINB><<<grid, NT, dyn, st>>>(r, x, y, alpha_part);
+  launch_chained(diag_first ? mom_rows_kernel<true, NT, U, MINB> : mom_rows_kernel<false, NT, U, MINB>, grid, NT, dyn, st,
+                 r, x, y, alpha_part);
 }
 
 // A tile per CTA.  Many tiles: 256 threads, five CTAs per SM (48 registers,

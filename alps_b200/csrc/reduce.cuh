@@ -17,6 +17,30 @@ namespace aed {
 
 constexpr int kFinishThreads = 1024;
 
+// Programmatic dependent launch: a kernel of the Lanczos chain lets the next
+// one start at once (chain_next), and waits for the one before it to be
+// complete before it touches anything that one writes (chain_wait).  What runs
+// before chain_wait reads only the handle's tables.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch a kernel of the chain.
+template <typename... K, typename... A>
+inline cudaError_t launch_chained(void (*kern)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                                  A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, (K)args...);
+}
+
 // Block reduction: warp shuffles, then warp 0 over the warp sums; the total is
 // returned to every thread.  sm needs 33 doubles.
 template <int NT>

@@ -625,6 +625,8 @@ __global__ void __launch_bounds__(NT, MINB) spin_rows_kernel(const SpinDev t, co
   if ((int64_t)blockIdx.x < nb) spin_fetch<NT>(t, blockIdx.x, prog, (size_t)B * pb);
   for (int q = threadIdx.x; q <= vals.n; q += NT) sm.val[q] = q < vals.n ? vals.v[q] : 0.0;
   if (threadIdx.x < B) reinterpret_cast<double*>(spin_dyn)[(size_t)t.maxrows * B + threadIdx.x] = 0.0;
+  chain_next();
+  chain_wait();
   int w = 0;
   for (int64_t ub = blockIdx.x; ub < nb; ub += gridDim.x, w ^= 1)
     spin_rows_bundle<D, B, NT>(t, ub + gridDim.x < nb ? ub + gridDim.x : -1, x, y, alpha_part, sm, spin_dyn,
@@ -1374,7 +1376,7 @@ int spin_rows_go(const SpinDev& t, const SpinRowVals& vals, const double* x, dou
   }
   if (per_sm < 1) return kSpinRowsNone;
   const int64_t nb = t.n_rblk / B, cap = (int64_t)sm_count() * per_sm;
-  kern<<<(unsigned)(nb < cap ? nb : cap), NT, dyn, st>>>(t, vals, x, y, alpha_part);
+  launch_chained(kern, (unsigned)(nb < cap ? nb : cap), NT, dyn, st, t, vals, x, y, alpha_part);
   return check_launch_counted("spin_rows_kernel");
 }
 

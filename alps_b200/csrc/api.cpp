@@ -355,8 +355,7 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
   cudaEvent_t e0, e1;
   AED_CUDA_TRY(cudaEventCreate(&e0));
   AED_CUDA_TRY(cudaEventCreate(&e1));
-  int best = 0;
-  float best_ms = 1e30f;
+  std::vector<float> ms_of((size_t)hv_num_variants(), 1e30f);
   int rc = AED_OK;
   // as solves run them: with the per-tile <x,y> partials; best of three
   for (int v = 0; v < hv_num_variants() && !rc; ++v) {
@@ -373,22 +372,26 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
       cudaEventSynchronize(e1);
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = v;
-      }
+      ms_of[v] = std::min(ms_of[v], ms);
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
+  // the first within 5 % of the fastest: the forms of one row width stand in
+  // order of CTA size, and beside the products of other streams smaller CTAs
+  // do better than alone (5x5 with 11 up FP64, 256 and 512 threads: 165 and 162
+  // us alone, 138 and 155 a product with three handles in turn)
+  const float least = *std::min_element(ms_of.begin(), ms_of.end());
+  int best = 0;
+  while (!(ms_of[best] <= 1.05f * least)) ++best;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[key] = best;
   }
   if (std::getenv("AED_VERBOSE"))
     std::fprintf(stderr, "[aed] apply %s D=%lld: variant %s (%.3f ms)\n", f32 ? "fp32" : "fp64", (long long)D,
-                 hv_variant_name(best), best_ms);
+                 hv_variant_name(best), ms_of[best]);
   *out = best;
   return AED_OK;
 }
@@ -586,7 +589,7 @@ int aed_create(const aed_model_desc* model, int precision, int device, aed_handl
   if ((rc = mem_dev_alloc_n(&h->d_thi, nhi)) || (rc = mem_dev_alloc_n(&h->d_tlo, nlo)) ||
       (rc = mem_dev_alloc_n(&h->d_lolist, nlo)) || (rc = mem_dev_alloc_n(&h->d_looff, h->tab.looff.size())) ||
       (rc = mem_dev_alloc_n(&h->d_tile_h, th.size())) || (rc = mem_dev_alloc_n(&h->d_tile_r, tr.size())) ||
-      (rc = mem_dev_alloc_n(&h->d_scal, 8)) || (rc = mem_dev_alloc_n(&h->d_flag, 1)) ||
+      (rc = mem_dev_alloc_n(&h->d_scal, 8)) || (rc = mem_dev_alloc_n(&h->d_flag, 2)) ||
       (rc = mem_dev_alloc_n(&h->d_blk_h, blk.size() + 1)) ||
       (rc = mem_dev_alloc_n(&h->d_tfirst, tf.size() + 1)) || (rc = mem_dev_alloc_n(&h->d_xtab, xt.size() + 1)) ||
       (rc = mem_dev_alloc_n(&h->d_dg, (size_t)h->tab.D)) || (rc = mem_dev_alloc_n(&h->d_partA, th.size() + 1)) ||
@@ -607,7 +610,7 @@ int aed_create(const aed_model_desc* model, int precision, int device, aed_handl
   if (!blk.empty()) cudaMemcpyAsync(h->d_blk_h, blk.data(), blk.size() * 4, cudaMemcpyHostToDevice, h->stream);
   if (!tf.empty()) cudaMemcpyAsync(h->d_tfirst, tf.data(), tf.size() * 4, cudaMemcpyHostToDevice, h->stream);
   if (!xt.empty()) cudaMemcpyAsync(h->d_xtab, xt.data(), xt.size() * 2, cudaMemcpyHostToDevice, h->stream);
-  cudaMemsetAsync(h->d_flag, 0, sizeof(uint32_t), h->stream);
+  cudaMemsetAsync(h->d_flag, 0, 2 * sizeof(uint32_t), h->stream);
   const cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
     release(h);

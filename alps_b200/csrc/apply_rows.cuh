@@ -23,10 +23,10 @@
 // size, DRAM) behind 32 warps per SM; part costs on 6x5 FP32 (3.93 ms, a copy
 // with one part left out): hi-part flips 1.15 ms, crossing 1.48, lo-part 0.83;
 // L=28 FP64 (1.34 ms): outside the lo part 0.83, lo-part 0.29.
-// Measured (one box, with partials, us; the bundle apply before: one block of x
-// in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1396 (1684), FP32
-// 786 (1102); 6x5 FP64 6930 (8730), FP32 3970 (5570); L=24 FP64 92 (133), FP32
-// 60 (88); L=16 FP64 8.4 (18.4).
+// Measured (L2 flushed, with partials, us; in brackets the apply before: one
+// block of x in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1266
+// (1684), FP32 771 (1102); 6x5 FP32 3700 (5570); L=24 FP64
+// 92 (133), FP32 59 (88); L=16 FP64 8.4 (18.4).
 //
 // Reference paths are relative to the ALPS source tree.
 #pragma once
@@ -59,6 +59,7 @@ struct alignas(sizeof(T) * B) RowVec {
 struct RowsSmem {
   double lolo_c[kMaxBonds + 1];  // the last: 0, of the padding entries
   double red[kMaxItems][kHvThreads / 32];
+  uint32_t ticket[2];  // Taker::slot
 };
 
 // A bundle's program: a head, then the flips outside the lo part that apply to
@@ -392,6 +393,36 @@ __device__ __forceinline__ int form_program(const ApplyCtx& c, const DevTables& 
   return n1 + n2;
 }
 
+// Bundles handed out on demand: a CTA works on bundles blockIdx.x and
+// blockIdx.x + gridDim.x, then on what it draws from a counter, so that a
+// sector with a few bundles per CTA, the large ones first, ends evenly.  A draw
+// is made a whole bundle before its answer is needed, as the next bundle's
+// program is fetched a bundle ahead.  Every CTA stops at its first draw past
+// the end, so an apply over nb > 2 gridDim.x bundles makes nb - gridDim.x
+// draws, and the CTA that holds the last one zeroes the counter for the
+// handle's next apply, which reads it only after this one.  Rows and partials
+// do not depend on who forms them.
+struct Taker {
+  uint32_t* word;
+  uint32_t* slot;  // two words of shared memory, taken in turn
+  uint32_t nb, drawn;
+  __device__ __forceinline__ Taker(uint32_t* w, uint32_t* s, uint32_t n)
+      : word(w), slot(s), nb(n), drawn(blockIdx.x + gridDim.x) {}
+  // thread 0, before the barrier that precedes take(w)
+  __device__ __forceinline__ void publish(int w) {
+    if (threadIdx.x == 0) {
+      slot[w] = drawn;
+      if (drawn == nb + gridDim.x - 1u) *word = 0u;
+    }
+  }
+  // every thread, after that barrier; the next publish(w) is two barriers on
+  __device__ __forceinline__ uint32_t take(int w) {
+    const uint32_t b = slot[w];
+    if (b < nb && threadIdx.x == 0) drawn = 2u * gridDim.x + atomicAdd(word, 1u);
+    return b;
+  }
+};
+
 // A program on its way from `src` into shared memory (every thread; waited for
 // by the next rows_bundle).
 template <int NT>
@@ -402,23 +433,26 @@ __device__ __forceinline__ void fetch_program(const unsigned char* src, unsigned
   }
 }
 
-// The bundle whose program is in (or on its way into) prog; the next one's
-// (next == nullptr: none) goes to `other` while this one runs.
-template <typename T, typename Acc, int B, int NT, int U, int UC>
+// The bundle whose program is in (or on its way into) prog.  fetch_next() is
+// called by every thread once nobody reads the previous bundle's program any
+// more: it starts the copy of the next one's.
+template <typename T, typename Acc, int B, int NT, int U, int UC, class Next>
 __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restrict__ x, T* y,
                                             double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
-                                            unsigned char* prog, unsigned char* other,
-                                            const unsigned char* __restrict__ next, int next_bytes, int cap) {
+                                            unsigned char* prog, int cap, Next&& fetch_next) {
   constexpr bool kOrdered = sizeof(T) == 8;
   using Row = RowVec<T, B>;
   Row* rows = reinterpret_cast<Row*>(xs);
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();  // this program is here; the previous bundle is done with x, red and `other`
-  if (next) fetch_program<NT>(next, other, next_bytes);
+  __syncthreads();  // this program is here; the previous bundle is done with x, red and its program
+  if (!kOrdered) fetch_next();
   const RowHead& hd = *reinterpret_cast<const RowHead*>(prog);
   const Program pg = program_at<B>(prog, cap);
   const int nv = hd.nv;
-  if (nv == 0) return;  // padding of the block list
+  if (nv == 0) {  // padding of the block list
+    if (kOrdered) fetch_next();
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lbase = hd.lbase, nk = hd.nk;
   uint32_t bj[B];
@@ -436,6 +470,9 @@ __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restr
     rows[i] = a;
     if (two) rows[i + NT] = b;
   }
+  // FP64: behind the loads of x (chain L=26, 512 threads, 350 us a product when
+  // it stood before them, now 332; FP32 6x5 3754 us here, 3575 before them)
+  if (kOrdered) fetch_next();
   __syncthreads();
   const int n1 = hd.n1, n2 = hd.n2, full = hd.full, Nlo = t.Nlo;
   const unsigned char* cs = reinterpret_cast<const unsigned char*>(sm.lolo_c);

@@ -90,9 +90,10 @@ __device__ __forceinline__ void rows_items(const BatchArgs& a, int i0, int i1, i
       if (threadIdx.x < B) reinterpret_cast<T*>(xs)[(size_t)I.t.maxrows * B + threadIdx.x] = T(0);
     }
     run(I, [&](const T* x, T* y, double* alpha_part, bool last) {
-      rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(t, x, y, alpha_part, sm.rows, xs, dyn + w * prog,
-                                                                  dyn + (w ^ 1) * prog, last ? next : nullptr,
-                                                                  next_bytes, I.t.rcap[kEl][kTab]);
+      rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(
+          t, x, y, alpha_part, sm.rows, xs, dyn + w * prog, I.t.rcap[kEl][kTab], [&] {
+            if (last && next) rapply::fetch_program<NT>(next, dyn + (w ^ 1) * prog, next_bytes);
+          });
     });
     it = nit;
     w ^= 1;

@@ -40,7 +40,7 @@ struct aed_handle {
   double* d_partA = nullptr;  // per-tile partial sums (n_tiles)
   double* d_partB = nullptr;  // per-chunk partial sums (red_chunks(D))
   double* d_scal = nullptr;   // 8 device scalars
-  uint32_t* d_flag = nullptr;  // raised by a kernel whose bounded wait gave up
+  uint32_t* d_flag = nullptr;  // two words: DevTables::flag
   float* d_dgf = nullptr;      // FP32 handles: the diagonal rounded to FP32
   double* h_scal = nullptr;   // 8 pinned host scalars
   int hv_var[2] = {-1, -1};  // apply variant per precision (FP64, FP32), -1 = not tuned yet

@@ -44,7 +44,10 @@ __global__ void __launch_bounds__(kHvThreads, MINB) hv_kernel(const __grid_const
 }
 
 // y = H x over bundles with x interleaved in shared memory (apply_rows.cuh).
-template <typename T, typename Acc, int B, int NT, int MINB>
+// DRAW: bundles by rapply::Taker (more than two per CTA), else round robin.
+// (With 296 bytes of arguments the host needed 0.4 us more per launch than with
+// the 288 that these are, a multiple of 32; a smaller struct gained nothing.)
+template <typename T, typename Acc, int B, int NT, int MINB, bool DRAW>
 __global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const T* __restrict__ x, T* y,
                                                        double* __restrict__ alpha_part) {
   extern __shared__ __align__(16) unsigned char hvr_dyn[];
@@ -54,18 +57,29 @@ __global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const 
   const int stride = t.rstride[kEl][kTab], cap = t.rcap[kEl][kTab];
   unsigned char* prog = hvr_dyn + (((size_t)(t.maxrows + 1) * kRow + 15) & ~(size_t)15);
   const unsigned char* src = t.rprog[kEl][kTab];
-  const int64_t nb = t.n_blk / B;
-  int64_t ub = blockIdx.x;
-  if (ub < nb) rapply::fetch_program<NT>(src + ub * stride, prog, stride);
+  rapply::fetch_program<NT>(src + (int64_t)blockIdx.x * stride, prog, stride);  // the grid is at most nb
   for (int q = threadIdx.x; q <= t.n_lolo; q += NT) sm.lolo_c[q] = q < t.n_lolo ? __ldg(t.lolo_c + q) : 0.0;
   if (threadIdx.x < B) reinterpret_cast<T*>(hvr_dyn)[(size_t)t.maxrows * B + threadIdx.x] = T(0);
   chain_next();
   chain_wait();
+  const uint32_t nb = (uint32_t)(t.n_blk / B);
+  auto bundle = [&](int w, auto&& fetch_next) {
+    rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(t, x, y, alpha_part, sm, hvr_dyn, prog + w * stride,
+                                                                cap, fetch_next);
+  };
+  auto fetch = [&](uint32_t b, int w) {
+    if (b < nb) rapply::fetch_program<NT>(src + (int64_t)b * stride, prog + w * stride, stride);
+  };
   int w = 0;
-  for (; ub < nb; ub += gridDim.x, w ^= 1)
-    rapply::rows_bundle<T, Acc, B, NT, rapply::kU, rapply::kUC>(
-        t, x, y, alpha_part, sm, hvr_dyn, prog + w * stride, prog + (w ^ 1) * stride,
-        ub + gridDim.x < nb ? src + (ub + gridDim.x) * stride : nullptr, stride, cap);
+  if constexpr (DRAW) {
+    rapply::Taker taker(t.flag + 1, sm.ticket, nb);
+    for (uint32_t b = blockIdx.x; b < nb; w ^= 1) {
+      taker.publish(w);
+      bundle(w, [&] { fetch(b = taker.take(w), w ^ 1); });
+    }
+  } else {
+    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x, w ^= 1) bundle(w, [&] { fetch(b + gridDim.x, w ^ 1); });
+  }
 }
 
 // The rows apply's programs, one warp per bundle.
@@ -623,19 +637,32 @@ int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* 
 // at this sector's dynamic shared memory (sectors of one process share a few
 // sizes).  Not for couplings that are not finite: a flip that a row does not
 // take adds c * 0.
+//
+// Bundles are drawn from a counter when there are more than three per CTA and
+// several CTAs to an SM.  Measured, round robin against drawn, us with L2
+// flushed, FP64: chain L=28 (384 threads) 1422 / 1266, L=26 (256) 350 / 332,
+// 5x5 with 11 up 190 / 173, L=26 with 9 up 134 / 112, L=24 at 3.5 bundles per
+// CTA 95.8 / 91.5; FP32 6x5 3870 / 3620.  With less to even out the hand-out
+// only costs (0.4 us of the chain L=20's 11.7), and with one CTA of 1024
+// threads on an SM it costs more than it evens out (L=28: 1444 / 1501).
 template <typename T, typename Acc, int ROW, int NT, int MINB>
 int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
   constexpr int B = ROW / (int)sizeof(T), kTab = ROW == 16 ? 0 : 1, kEl = sizeof(T) == 8 ? 0 : 1;
-  if (!t.low_e || !t.rprog[kEl][kTab] || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
+  if (!t.low_e || !t.rprog[kEl][kTab] || !t.flag || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
   const size_t dyn = rapply::rows_smem_bytes(ROW, t.maxrows, t.rstride[kEl][kTab]);
-  auto kern = hvr_kernel<T, Acc, B, NT, MINB>;
+  constexpr bool kDraws = NT <= 512;
+  auto kern = hvr_kernel<T, Acc, B, NT, MINB, false>;
+  auto draws = hvr_kernel<T, Acc, B, NT, MINB, kDraws>;
   static int limit_rc = -1;
   static size_t static_bytes = 0;
   static std::map<size_t, int> grids;  // dyn -> grid (0: does not fit)
   int grid = 0;
   {
     std::lock_guard<std::mutex> lk(g_grid_mu);
-    if (limit_rc < 0) limit_rc = raise_smem_limit(kern, &static_bytes);
+    if (limit_rc < 0) {
+      limit_rc = raise_smem_limit(draws, &static_bytes);
+      if (limit_rc == AED_OK) limit_rc = raise_smem_limit(kern, &static_bytes);
+    }
     if (limit_rc == AED_ERR_CUDA) return limit_rc;
     auto it = grids.find(dyn);
     if (it == grids.end()) {
@@ -654,7 +681,7 @@ int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double*
   const int64_t nb = t.n_blk / B;
   if (g > nb) g = nb;
   if (g < 1) return AED_OK;
-  launch_chained(kern, (unsigned)g, NT, dyn, st, t, x, y, alpha_part);
+  launch_chained(kDraws && nb > 3 * g ? draws : kern, (unsigned)g, NT, dyn, st, t, x, y, alpha_part);
   return check_launch("hvr_kernel");
 }
 

@@ -30,7 +30,8 @@ struct DevTables {
   const uint32_t* tfirst = nullptr;  // 2^Nhi: index of the first tile of each hi block
   int64_t n_blk = 0;
   int maxrows = 0;  // rows of the largest hi block
-  // raised by a kernel whose bounded wait gave up (read and cleared by the host)
+  // [0] raised by a kernel whose bounded wait gave up (read and cleared by the
+  // host); [1] bundles drawn by the apply that runs, zero between applies
   uint32_t* flag = nullptr;
   // FP32 handles: M(i,i) rounded to FP32 (D floats), read by the FP32 applies
   // in place of dg (half its bytes; the FP64 applies keep dg)

@@ -68,3 +68,28 @@ def test_rows_apply_keeps_infinities_to_their_rows():
             if name.startswith("row"):
                 ham.time_apply(x, y, 1, i, False)
                 assert np.array_equal(y.download(), want, equal_nan=True), (name, precision)
+
+
+@pytest.mark.parametrize("n_up", [9, 17])
+def test_drawn_bundles_are_each_taken_once_apply_after_apply(n_up):
+    """Sectors of many bundles per CTA, where CTAs draw their bundles: several applies in a row, odd ones on new states."""
+    n = 26
+    rng = np.random.default_rng(n_up)
+    bonds = _bonds("ring", n, rng)
+    names = ed.apply_variants()
+    for precision in (ed.FP64, ed.FP32):
+        ham = ed.Hamiltonian(n, n_up, bonds, precision=precision)
+        x, y = ham.new_vector(), ham.new_vector()
+        for reps in (1, 4):
+            x.upload(rng.normal(size=ham.dim))
+            ham.time_apply(x, y, 1, 0, True)
+            want = y.download()
+            for i, name in enumerate(names):
+                if not name.startswith("row"):
+                    continue
+                y.upload(np.full(ham.dim, 3.0))
+                try:
+                    ham.time_apply(x, y, reps, i, True)
+                except ed.AEDError:
+                    continue  # its shared memory does not fit
+                assert np.array_equal(y.download(), want), (name, precision)

@@ -24,7 +24,7 @@
 // with one part left out): hi-part flips 1.15 ms, crossing 1.48, lo-part 0.83;
 // L=28 FP64 (1.34 ms): outside the lo part 0.83, lo-part 0.29.
 // Measured (L2 flushed, with partials, us; in brackets the apply before: one
-// block of x in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1266
+// block of x in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1200
 // (1684), FP32 771 (1102); 6x5 FP32 3700 (5570); L=24 FP64
 // 92 (133), FP32 59 (88); L=16 FP64 8.4 (18.4).
 //
@@ -37,7 +37,6 @@ namespace aed {
 namespace rapply {
 
 using apply::ApplyCtx;
-using apply::kCrossOp;
 using apply::kTileRows;
 using apply::SPair;
 using apply::TileOp;
@@ -47,8 +46,13 @@ constexpr int kMaxB = 4;
 // together.  They fill the 64 registers of 1024 threads per SM without a spill;
 // eight, or four crossing ones, spill and were 5-25 % slower on L=28 and 6x5.
 constexpr int kU = 4, kUC = 2;
-constexpr uint32_t kNullOp = 0x80000001u;     // an op that no row takes (no byte offset of an element)
-constexpr uint32_t kCrossTest = 0x80008000u;  // null bit and the required lo-bit value
+constexpr uint32_t kNullNb = 0x80000001u;  // FP32: an op that no row takes (no byte offset of an element)
+// FP64 ops, TileOp::mc: 0 a hi-part flip; a crossing flip has kCrossFlip, its
+// column of the crossing table (lo bit << Nlo, 20 bits) and, where the lo bit
+// must be set, kWantSet, the bits that the table's sign-extended entry then
+// has; kNullFlip: no row takes it.  kNoCross on the first op of a group of kU
+// ops: none of the group's ops, of any block, is a crossing flip.
+constexpr uint32_t kWantSet = 0xa0000000u, kNullFlip = 0x20000000u, kCrossFlip = 1u << 20, kNoCross = 1u << 30;
 constexpr int kMaxItems = 32;  // (block, tile) pairs of a bundle: 4 blocks of at most 7 tiles
 
 template <typename T, int B>
@@ -68,8 +72,8 @@ struct RowsSmem {
 //   [0, n1), those to larger ones in [n1, n1 + n2);
 //   FP32: c[o * B + j] and nb[o * B + j], the hi-part flips at o < n1, the
 //   crossing ones in [n1, n1 + n2) with their lo bit and required values in bits[o].
-// Lists are as long as the longest block's, rounded up to a multiple of the
-// unrolling, filled with null ops.  Programs depend on the couplings alone: a
+// Lists are as long as the longest block's, rounded up to a multiple of two
+// (FP32 crossing flips: of kUC), filled with null ops.  Programs depend on the couplings alone: a
 // handle forms them once (launch_row_progs), `cap` ops each, and a CTA copies
 // the next bundle's while it runs one.  (Listed in the apply, by a warp per
 // block while the others staged x, they put a chain of dependent loads and a
@@ -144,33 +148,52 @@ __device__ __forceinline__ void lo_terms(const uint2* __restrict__ tp, int np, c
   }
 }
 
-// FP64: n ops of every block (a multiple of U), U at a time for all B blocks:
-// their loads first, then the terms in order.  A crossing flip that the row
-// does not take adds c * 0, as a null op adds 0 * 0: neither changes a sum that
-// is never -0 (the couplings are finite).
+// FP64: U ops of every block: their loads first, then the terms in order.  A
+// crossing flip that the row does not take adds c * 0, as a null op adds
+// 0 * 0: neither changes a sum that is never -0 (the couplings are finite).
+template <typename T, typename Acc, int B, int U, bool CROSS>
+__device__ __forceinline__ void hi_group(const TileOp* ops, uint32_t r, const int16_t* __restrict__ xt,
+                                         const T* __restrict__ x, Acc (&acc)[B]) {
+  T xv[U][B];
+  double c[U][B];
+#pragma unroll
+  for (int v = 0; v < U; ++v)
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const TileOp e = ops[v * B + j];
+      c[v][j] = e.c;
+      uint32_t at = r;
+      if (CROSS && e.mc != 0u) at = (uint32_t)(int)__ldg(xt + (e.mc & 0xfffffu));
+      xv[v][j] = T(0);
+      if (((CROSS ? at ^ e.mc : e.mc) & (CROSS ? kWantSet : kNullFlip)) == 0u) xv[v][j] = __ldg(x + (e.nb + at));
+    }
+#pragma unroll
+  for (int v = 0; v < U; ++v)
+#pragma unroll
+    for (int j = 0; j < B; ++j) acc[j].add(c[v][j], xv[v][j]);
+}
+
+// FP64: n ops of every block (n even), U at a time and a last two.  Groups
+// without a crossing flip, marked when the program is formed, skip the table
+// load, its address and the test of its entry: on the chain L=28 the apply issues
+// in 73 % of its cycles and spends 60 % of its time here.  Together with the
+// remainder of two (the lists were padded to four) chain L=28 1191 -> 1124 us,
+// 5x5 with 11 up 138 -> 129.  The choice made per block of the bundle takes the short
+// form more often, but waits for one block's table entries before the other's
+// loads go out: 1218 and 140 us.
 template <typename T, typename Acc, int B, int U>
-__device__ __forceinline__ void hi_terms(const TileOp* ops, int n, uint32_t r, const uint16_t* __restrict__ xt,
-                                         int Nlo, const T* __restrict__ x, Acc (&acc)[B]) {
+__device__ __forceinline__ void hi_terms(const TileOp* ops, int n, uint32_t r, const int16_t* __restrict__ xt,
+                                         const T* __restrict__ x, Acc (&acc)[B]) {
+  static_assert(U == 4, "a remainder of two");
+  int o = 0;
 #pragma unroll 1
-  for (int o = 0; o < n; o += U) {
-    T xv[U][B];
-    double c[U][B];
-#pragma unroll
-    for (int v = 0; v < U; ++v)
-#pragma unroll
-      for (int j = 0; j < B; ++j) {
-        const TileOp e = ops[(o + v) * B + j];
-        c[v][j] = e.c;
-        uint32_t at = r;
-        if (e.mc != 0u) at = __ldg(xt + (((e.mc >> 16) & 0xffu) << Nlo));
-        xv[v][j] = T(0);
-        if (((at ^ e.mc) & kCrossTest) == 0u) xv[v][j] = __ldg(x + (e.nb + at));
-      }
-#pragma unroll
-    for (int v = 0; v < U; ++v)
-#pragma unroll
-      for (int j = 0; j < B; ++j) acc[j].add(c[v][j], xv[v][j]);
+  for (; o + U <= n; o += U) {
+    if (ops[o * B].mc & kNoCross)
+      hi_group<T, Acc, B, U, false>(ops + o * B, r, xt, x, acc);
+    else
+      hi_group<T, Acc, B, U, true>(ops + o * B, r, xt, x, acc);
   }
+  if (o < n) hi_group<T, Acc, B, 2, true>(ops + o * B, r, xt, x, acc);
 }
 
 // FP32: hi-part flips [0, n) of every block (n even), of which those below
@@ -206,7 +229,7 @@ __device__ __forceinline__ void hihi_terms(const Program& pg, int nfull, int n, 
     for (int v = 0; v < UT; ++v) {
       const NB nb = *reinterpret_cast<const NB*>(pg.nb + (o + v) * B);
 #pragma unroll
-      for (int j = 0; j < B; ++j) xv[v][j] = nb.v[j] != kNullOp ? at_byte(x, nb.v[j] + rb) : T(0);
+      for (int j = 0; j < B; ++j) xv[v][j] = nb.v[j] != kNullNb ? at_byte(x, nb.v[j] + rb) : T(0);
     }
 #pragma unroll
     for (int v = 0; v < UT; ++v) add(o + v, xv[v]);
@@ -287,29 +310,30 @@ __device__ __forceinline__ void compile_f64(const ApplyCtx& c, const uint32_t* _
   auto emit = [&](int at, const SPair& e) {
     const uint32_t flo = e.flip & c.lm, nb = __ldg(thi + (h ^ (e.flip >> c.Nlo)));
     const uint32_t v = (e.cond & c.lm) != 0u ? 1u : 0u;
-    ops[at * B + j] = flo == 0u
-                          ? TileOp{0u, nb, e.c}
-                          : TileOp{kCrossOp | ((uint32_t)(__ffs(flo) - 1) << 16) | (v << 15), nb - (v << 15), e.c};
+    // (a sign-extended table entry is the rank - v 2^15)
+    ops[at * B + j] = flo == 0u ? TileOp{0u, nb, e.c}
+                                : TileOp{kCrossFlip | (uint32_t)(__ffs(flo) - 1) << c.Nlo | (v ? kWantSet : 0u),
+                                         nb + (v << 15), e.c};
   };
   const int lane = threadIdx.x & 31;
   int n = walk_list(low, c.np, h, c.Nlo, c.lm, 0, 0, emit);
-  for (int q = n + lane; q < l1; q += 32) ops[q * B + j] = {kNullOp, 0u, 0.0};
+  for (int q = n + lane; q < l1; q += 32) ops[q * B + j] = {kNullFlip, 0u, 0.0};
   n = walk_list(rise, c.np, h, c.Nlo, c.lm, 0, l1, emit);
-  for (int q = n + lane; q < l1 + l2; q += 32) ops[q * B + j] = {kNullOp, 0u, 0.0};
+  for (int q = n + lane; q < l1 + l2; q += 32) ops[q * B + j] = {kNullFlip, 0u, 0.0};
 }
 
 template <int B>
 __device__ __forceinline__ void compile_f32(const ApplyCtx& c, const uint32_t* __restrict__ thi, const SPair* low,
                                             uint32_t h, int j, int l1, int l2, const Program& pg) {
   const int lane = threadIdx.x & 31;
-  auto put = [&](int at, uint32_t nb, double cc) {  // nb: bytes (a multiple of 4), or kNullOp
+  auto put = [&](int at, uint32_t nb, double cc) {  // nb: bytes (a multiple of 4), or kNullNb
     pg.nb[at * B + j] = nb;
     pg.c[at * B + j] = cc;
   };
   int n = walk_list(low, c.np, h, c.Nlo, c.lm, 1, 0, [&](int at, const SPair& e) {
     put(at, __ldg(thi + (h ^ (e.flip >> c.Nlo))) * 4u, e.c);
   });
-  for (int q = n + lane; q < l1; q += 32) put(q, kNullOp, 0.0);
+  for (int q = n + lane; q < l1; q += 32) put(q, kNullNb, 0.0);
   n = walk_list(low, c.np, h, c.Nlo, c.lm, 2, l1, [&](int at, const SPair& e) {
     put(at, __ldg(thi + (h ^ (e.flip >> c.Nlo))) * 4u, e.c);
     const uint32_t b = (uint32_t)(__ffs(e.flip & c.lm) - 1);
@@ -341,8 +365,8 @@ __device__ __forceinline__ int list_lengths(const ApplyCtx& c, const DevTables& 
     if (kOrdered || j == 0)
       l2 = max(l2, walk_list(kOrdered ? rise : low, c.np, h, c.Nlo, c.lm, kOrdered ? 0 : 2, 0, none));
   }
-  *n1 = kOrdered ? (l1 + U - 1) / U * U : (l1 + 1) / 2 * 2;
-  *n2 = kOrdered ? (l2 + U - 1) / U * U : (l2 + UC - 1) / UC * UC;
+  *n1 = (l1 + 1) / 2 * 2;
+  *n2 = kOrdered ? (l2 + 1) / 2 * 2 : (l2 + UC - 1) / UC * UC;
   *full = nv == B ? f : 0;
   return nv;
 }
@@ -381,12 +405,22 @@ __device__ __forceinline__ int form_program(const ApplyCtx& c, const DevTables& 
     } else {  // no such block in the bundle: null ops
       for (int q = lane; q < n1 + n2; q += 32) {
         if constexpr (kOrdered) {
-          pg.ops[q * B + j] = {kNullOp, 0u, 0.0};
+          pg.ops[q * B + j] = {kNullFlip, 0u, 0.0};
         } else {
-          pg.nb[q * B + j] = kNullOp;
+          pg.nb[q * B + j] = kNullNb;
           pg.c[q * B + j] = 0.0;
         }
       }
+    }
+  }
+  if constexpr (kOrdered) {  // the groups without crossing flips
+    __syncwarp();
+    const int g1 = n1 / U, g2 = n2 / U;
+    for (int g = lane; g < g1 + g2; g += 32) {
+      TileOp* o = pg.ops + (g < g1 ? g * U : n1 + (g - g1) * U) * B;
+      uint32_t any = 0u;
+      for (int q = 0; q < U * B; ++q) any |= o[q].mc;
+      if (!(any & kCrossFlip)) o->mc |= kNoCross;
     }
   }
   if (lane == 0) *reinterpret_cast<RowHead*>(out) = hd;
@@ -480,6 +514,7 @@ __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restr
 #pragma unroll 1
   for (uint32_t r = threadIdx.x; r < nk; r += NT) {
     const uint16_t* xt = t.xtab + lbase + r;
+    const int16_t* xs16 = reinterpret_cast<const int16_t*>(xt);
     const uint32_t s = s0 + (r >> 5);
     const uint32_t w = __ldg(t.low_w + s);
     const uint2* tp = t.low_e + ((size_t)s * t.low_st * 32 + lane);
@@ -489,7 +524,7 @@ __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restr
       double dg[B];
 #pragma unroll
       for (int j = 0; j < B; ++j) dg[j] = j < nv ? __ldg(t.dg + bj[j] + r) : 0.0;
-      hi_terms<T, Acc, B, U>(pg.ops, n1, r, xt, Nlo, x, acc);
+      hi_terms<T, Acc, B, U>(pg.ops, n1, r, xs16, x, acc);
       lo_terms<T, Acc, B>(tp, wl, xs, cs, acc);
       {
         const Row own = rows[r];
@@ -497,7 +532,7 @@ __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restr
         for (int j = 0; j < B; ++j) acc[j].add(dg[j], own.v[j]);
       }
       lo_terms<T, Acc, B>(tp + wl * 32, wu, xs, cs, acc);
-      hi_terms<T, Acc, B, U>(pg.ops + n1 * B, n2, r, xt, Nlo, x, acc);
+      hi_terms<T, Acc, B, U>(pg.ops + n1 * B, n2, r, xs16, x, acc);
     } else {
       const Row own = rows[r];
 #pragma unroll

@@ -150,8 +150,7 @@ void release(aed_handle* h) {
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
                   (void*)h->d_slol, (void*)h->d_srblk, (void*)h->d_stfirst, (void*)h->d_slow_w, (void*)h->d_sxtab,
                   (void*)h->d_slow_e, (void*)h->d_slokey, (void*)h->d_srprog, (void*)h->d_slodiag, (void*)h->d_sxoff, (void*)h->d_sxdiag, (void*)h->d_scross,
-                  (void*)h->d_low_e, (void*)h->d_low_w, (void*)h->d_rprog[0][0], (void*)h->d_rprog[0][1],
-                  (void*)h->d_rprog[1][0], (void*)h->d_rprog[1][1], (void*)h->d_lolo})
+                  (void*)h->d_low_e, (void*)h->d_low_w, (void*)h->d_rprog, (void*)h->d_lolo})
     mem_dev_free(p, h->stream);
   mom_rows_free(h->mrows, h->stream);
   delete h->mp;
@@ -209,21 +208,29 @@ int upload_lo_table(aed_handle* h) {
     if ((rc = launch_row_need(h->P, t, e == 0 ? 8 : 4, d_ops + 2 * e, h->stream))) return rc;
   AED_CUDA_TRY(cudaMemcpyAsync(ops, d_ops, sizeof ops, cudaMemcpyDeviceToHost, h->stream));
   AED_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  // one block for all forms: each allocation of its own costs the first handle
+  // of a size 0.1 to 0.4 ms
+  size_t at[2][2] = {}, bytes = 0;
   for (int e = 0; e < n_elem; ++e)
     for (int row = 0; row < 2; ++row) {
       const int elem = e == 0 ? 8 : 4;
       t.rcap[e][row] = std::max(2, (ops[2 * e + row] + 1) & ~1);
       t.rstride[e][row] = row_prog_stride(elem, row, t.rcap[e][row]);
-      const size_t bytes = (size_t)(t.n_blk / row_blocks(elem, row)) * (size_t)t.rstride[e][row];
-      if (bytes > h->d_rprog_n[e][row]) {
-        mem_dev_free(h->d_rprog[e][row], h->stream);
-        h->d_rprog[e][row] = nullptr;
-        h->d_rprog_n[e][row] = 0;
-        if (mem_dev_alloc_n(&h->d_rprog[e][row], bytes)) return AED_OK;
-        h->d_rprog_n[e][row] = bytes;
-      }
-      if ((rc = launch_row_progs(h->P, t, elem, row, h->d_rprog[e][row], h->d_lolo, h->stream))) return rc;
-      t.rprog[e][row] = h->d_rprog[e][row];
+      at[e][row] = bytes;
+      bytes += ((size_t)(t.n_blk / row_blocks(elem, row)) * (size_t)t.rstride[e][row] + 255) & ~(size_t)255;
+    }
+  if (bytes > h->d_rprog_n) {
+    mem_dev_free(h->d_rprog, h->stream);
+    h->d_rprog = nullptr;
+    h->d_rprog_n = 0;
+    if (mem_dev_alloc_n(&h->d_rprog, bytes)) return AED_OK;
+    h->d_rprog_n = bytes;
+  }
+  for (int e = 0; e < n_elem; ++e)
+    for (int row = 0; row < 2; ++row) {
+      unsigned char* p = h->d_rprog + at[e][row];
+      if ((rc = launch_row_progs(h->P, t, e == 0 ? 8 : 4, row, p, h->d_lolo, h->stream))) return rc;
+      t.rprog[e][row] = p;
     }
   return AED_OK;
 }

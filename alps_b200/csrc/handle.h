@@ -33,8 +33,8 @@ struct aed_handle {
   uint2* d_low_e = nullptr;   // the same in slices of 32 rows (DevTables::low_e)
   uint32_t* d_low_w = nullptr;
   size_t d_low_n = 0;         // pairs allocated
-  unsigned char* d_rprog[2][2] = {};  // the rows apply's programs (DevTables::rprog)
-  size_t d_rprog_n[2][2] = {};
+  unsigned char* d_rprog = nullptr;  // the rows apply's programs (DevTables::rprog), one form after the other
+  size_t d_rprog_n = 0;
   double* d_lolo = nullptr;
   uint16_t* d_xtab = nullptr;  // crossing-flip table
   double* d_partA = nullptr;  // per-tile partial sums (n_tiles)

@@ -114,8 +114,8 @@ __host__ __device__ inline size_t rows_smem_bytes(int row_bytes, int maxrows, in
 // The value at a 32-bit byte offset (an FP32 vector of at most 2^30 rows; the
 // largest sector has 601 M): one add per address.
 template <typename T>
-__device__ __forceinline__ T at_byte(const T* __restrict__ p, uint32_t off) {
-  return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off));
+__device__ __forceinline__ T at_byte(const T* p, uint32_t off) {
+  return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off);
 }
 
 // The lo-part flips of one part of the slice: np pairs of entries.
@@ -153,7 +153,7 @@ __device__ __forceinline__ void lo_terms(const uint2* __restrict__ tp, int np, c
 // 0 * 0: neither changes a sum that is never -0 (the couplings are finite).
 template <typename T, typename Acc, int B, int U, bool CROSS>
 __device__ __forceinline__ void hi_group(const TileOp* ops, uint32_t r, const int16_t* __restrict__ xt,
-                                         const T* __restrict__ x, Acc (&acc)[B]) {
+                                         const T* x, Acc (&acc)[B]) {
   T xv[U][B];
   double c[U][B];
 #pragma unroll
@@ -165,7 +165,7 @@ __device__ __forceinline__ void hi_group(const TileOp* ops, uint32_t r, const in
       uint32_t at = r;
       if (CROSS && e.mc != 0u) at = (uint32_t)(int)__ldg(xt + (e.mc & 0xfffffu));
       xv[v][j] = T(0);
-      if (((CROSS ? at ^ e.mc : e.mc) & (CROSS ? kWantSet : kNullFlip)) == 0u) xv[v][j] = __ldg(x + (e.nb + at));
+      if (((CROSS ? at ^ e.mc : e.mc) & (CROSS ? kWantSet : kNullFlip)) == 0u) xv[v][j] = x[e.nb + at];
     }
 #pragma unroll
   for (int v = 0; v < U; ++v)
@@ -183,7 +183,7 @@ __device__ __forceinline__ void hi_group(const TileOp* ops, uint32_t r, const in
 // loads go out: 1218 and 140 us.
 template <typename T, typename Acc, int B, int U>
 __device__ __forceinline__ void hi_terms(const TileOp* ops, int n, uint32_t r, const int16_t* __restrict__ xt,
-                                         const T* __restrict__ x, Acc (&acc)[B]) {
+                                         const T* x, Acc (&acc)[B]) {
   static_assert(U == 4, "a remainder of two");
   int o = 0;
 #pragma unroll 1
@@ -200,7 +200,7 @@ __device__ __forceinline__ void hi_terms(const TileOp* ops, int n, uint32_t r, c
 // nfull are real for all of them.  rb: the row's rank in bytes.
 template <typename T, typename Acc, int B, int U>
 __device__ __forceinline__ void hihi_terms(const Program& pg, int nfull, int n, uint32_t rb,
-                                           const T* __restrict__ x, Acc (&acc)[B]) {
+                                           const T* x, Acc (&acc)[B]) {
   using NB = RowVec<uint32_t, B>;
   using CB = RowVec<double, B == 1 ? 1 : 2>;
   auto add = [&](int o, const T (&xv)[B]) {
@@ -242,7 +242,7 @@ __device__ __forceinline__ void hihi_terms(const Program& pg, int nfull, int n, 
 // adds c * 0.
 template <typename T, typename Acc, int B, int U>
 __device__ __forceinline__ void cross_terms(const Program& pg, int o0, int n, const uint16_t* __restrict__ xt, int Nlo,
-                                            const T* __restrict__ x, Acc (&acc)[B]) {
+                                            const T* x, Acc (&acc)[B]) {
   using NB = RowVec<uint32_t, B>;
   using CB = RowVec<double, B == 1 ? 1 : 2>;
   if (n == 0) return;
@@ -471,8 +471,8 @@ __device__ __forceinline__ void fetch_program(const unsigned char* src, unsigned
 // called by every thread once nobody reads the previous bundle's program any
 // more: it starts the copy of the next one's.
 template <typename T, typename Acc, int B, int NT, int U, int UC, class Next>
-__device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restrict__ x, T* y,
-                                            double* __restrict__ alpha_part, RowsSmem& sm, unsigned char* xs,
+__device__ __forceinline__ void rows_bundle(const DevTables& t, const T* x, T* y, double* alpha_part,
+                                            RowsSmem& sm, unsigned char* xs,
                                             unsigned char* prog, int cap, Next&& fetch_next) {
   constexpr bool kOrdered = sizeof(T) == 8;
   using Row = RowVec<T, B>;
@@ -498,8 +498,8 @@ __device__ __forceinline__ void rows_bundle(const DevTables& t, const T* __restr
     const bool two = i + NT < nk;
 #pragma unroll
     for (int j = 0; j < B; ++j) {
-      a.v[j] = j < nv ? __ldg(x + bj[j] + i) : T(0);
-      b.v[j] = j < nv && two ? __ldg(x + bj[j] + i + NT) : T(0);
+      a.v[j] = j < nv ? x[bj[j] + i] : T(0);
+      b.v[j] = j < nv && two ? x[bj[j] + i + NT] : T(0);
     }
     rows[i] = a;
     if (two) rows[i + NT] = b;

@@ -48,8 +48,7 @@ __global__ void __launch_bounds__(kHvThreads, MINB) hv_kernel(const __grid_const
 // (With 296 bytes of arguments the host needed 0.4 us more per launch than with
 // the 288 that these are, a multiple of 32; a smaller struct gained nothing.)
 template <typename T, typename Acc, int B, int NT, int MINB, bool DRAW>
-__global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const T* __restrict__ x, T* y,
-                                                       double* __restrict__ alpha_part) {
+__global__ void __launch_bounds__(NT, MINB) hvr_kernel(const DevTables t, const T* x, T* y, double* alpha_part) {
   extern __shared__ __align__(16) unsigned char hvr_dyn[];
   __shared__ rapply::RowsSmem sm;
   constexpr int kRow = sizeof(T) * B, kTab = kRow == 16 ? 0 : 1;
@@ -310,11 +309,23 @@ __global__ void copy_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t 
 
 // y += a*x, as ublas evaluates v += s*w: the product rounds, then the sum.
 template <typename T>
-__global__ void axpy_kernel(double a, const T* __restrict__ x, T* __restrict__ y, int64_t n) {
+__global__ void axpy_kernel(double a, const T* x, T* y, int64_t n) {
   chain_next();
   chain_wait();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = (T)__dadd_rn((double)y[i], __dmul_rn(a, (double)x[i]));
+  constexpr int U = 4;  // loads of four elements before their stores
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (; i + (U - 1) * stride < n; i += U * stride) {
+    T xv[U], yv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      xv[u] = x[i + u * stride];
+      yv[u] = y[i + u * stride];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) y[i + u * stride] = (T)__dadd_rn((double)yv[u], __dmul_rn(a, (double)xv[u]));
+  }
+  for (; i < n; i += stride) y[i] = (T)__dadd_rn((double)y[i], __dmul_rn(a, (double)x[i]));
 }
 
 template <typename T>
@@ -339,8 +350,7 @@ __global__ void __launch_bounds__(kFinishThreads) finish_sum_kernel(const double
 // in a full chunk issue all their loads before the arithmetic (4-byte loads leave too few bytes in
 // flight otherwise); the arithmetic and the order of the sum are the same, so are the bits.
 template <typename T>
-__device__ __forceinline__ double update_chunk(double alpha, double b, const T* __restrict__ x,
-                                               const T* __restrict__ vprev, T* __restrict__ y, int64_t e0,
+__device__ __forceinline__ double update_chunk(double alpha, double b, const T* x, const T* vprev, T* y, int64_t e0,
                                                int64_t e1) {
   double acc = 0.0;
   if constexpr (sizeof(T) == 4) {
@@ -397,7 +407,7 @@ __device__ __forceinline__ double update_chunk(double alpha, double b, const T* 
 // FP64: 16-byte double2 vectors, two in flight, when y is 16-byte aligned,
 // then the tail element by element.
 template <typename T>
-__device__ __forceinline__ void normalize_elems(double beta, T* __restrict__ y, int64_t n) {
+__device__ __forceinline__ void normalize_elems(double beta, T* y, int64_t n) {
   const int64_t stride = (int64_t)gridDim.x * kRedThreads;
   int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
   if constexpr (sizeof(T) == 4) {
@@ -461,9 +471,8 @@ __global__ void __launch_bounds__(kRedThreads) lanczos_update_kernel(const doubl
 // saves a launch per step.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) lanczos_update_fin_kernel(
-    const double* __restrict__ alpha_part, int64_t n_apart, double* __restrict__ alpha_out, double* alpha_host,
-    const T* __restrict__ x, const T* __restrict__ vprev, const double* __restrict__ beta_prev, double beta_val,
-    T* __restrict__ y, int64_t n, double* __restrict__ partB) {
+    const double* alpha_part, int64_t n_apart, double* alpha_out, double* alpha_host, const T* x, const T* vprev,
+    const double* beta_prev, double beta_val, T* y, int64_t n, double* partB) {
   __shared__ double sm[33];
   chain_next();
   chain_wait();
@@ -484,10 +493,8 @@ __global__ void __launch_bounds__(kRedThreads) lanczos_update_fin_kernel(
 
 // The normalisation with beta's finishing sum folded in (as above).
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) lanczos_normalize_fin_kernel(const double* __restrict__ beta_part,
-                                                                           int64_t n_bpart,
-                                                                           double* __restrict__ beta_out,
-                                                                           double* beta_host, T* __restrict__ y,
+__global__ void __launch_bounds__(kRedThreads) lanczos_normalize_fin_kernel(const double* beta_part, int64_t n_bpart,
+                                                                           double* beta_out, double* beta_host, T* y,
                                                                            int64_t n) {
   __shared__ double sm[33];
   chain_next();

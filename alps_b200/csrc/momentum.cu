@@ -336,11 +336,11 @@ __global__ void __launch_bounds__(kMomThreads) mom_row_kernel(const __grid_const
 template <int U>
 __device__ __forceinline__ void mom_row_terms(const uint32_t (&e)[U], int jbits, uint32_t jmask, uint32_t n_base,
                                               const double2* cf, const double2* __restrict__ cfg,
-                                              const double2* __restrict__ x, double& are, double& aim) {
+                                              const double2* x, double& are, double& aim) {
   double2 xj[U];
 #pragma unroll
   for (int v = 0; v < U; ++v)
-    xj[v] = e[v] != kMomRowPad ? __ldg(x + (e[v] & jmask)) : make_double2(0.0, 0.0);
+    xj[v] = e[v] != kMomRowPad ? x[e[v] & jmask] : make_double2(0.0, 0.0);
 #pragma unroll
   for (int v = 0; v < U; ++v) {
     const uint32_t k = e[v] >> jbits;
@@ -355,7 +355,8 @@ __device__ __forceinline__ void mom_row_terms(const uint32_t (&e)[U], int jbits,
 }
 
 // y = H x from the stored rows, one row per thread.  A row's terms are a
-// coalesced stream of entries and, U at a time, the x_j they name, so the
+// coalesced stream of entries and, U at a time, the x_j they name (entries and
+// diagonal may come from the kernel just before: no non-coherent loads), so the
 // only dependent load left is x_j itself; the entries are read once and are
 // kept out of the way of x in L2.  The coefficients phase_t * element are
 // staged in shared memory, those of terms with n_j != n_i (an orbit that a
@@ -367,8 +368,8 @@ __device__ __forceinline__ void mom_row_terms(const uint32_t (&e)[U], int jbits,
 // a product on the J1-J2 chain L=28 and 287 on the spin-1 chain L=18; this one
 // 84.5 and 100.
 template <bool kDiagFirst, int NT, int U, int MINB>
-__global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, const double2* __restrict__ x, double2* y,
-                                                            double* __restrict__ alpha_part) {
+__global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, const double2* x, double2* y,
+                                                            double* alpha_part) {
   extern __shared__ __align__(16) unsigned char mom_rows_dyn[];
   double2* cf = reinterpret_cast<double2*>(mom_rows_dyn);
   __shared__ double red[kMomThreads / 32];
@@ -390,8 +391,8 @@ __global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, co
       const bool row = i < rw.dim;
       double are = 0.0, aim = 0.0;
       if (kDiagFirst && row) {
-        const double2 xi = __ldg(x + i);
-        const double d = __ldg(rw.diag + i);
+        const double2 xi = x[i];
+        const double d = rw.diag[i];
         are = d * xi.x;
         aim = d * xi.y;
       }
@@ -407,8 +408,8 @@ __global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, co
         mom_row_terms<1>(e, rw.jbits, jmask, n_base, cf, rw.cf, x, are, aim);
       }
       if (!kDiagFirst && row) {
-        const double2 xi = __ldg(x + i);
-        const double d = __ldg(rw.diag + i);
+        const double2 xi = x[i];
+        const double d = rw.diag[i];
         are = fma(d, xi.x, are);
         aim = fma(d, xi.y, aim);
       }
@@ -422,7 +423,7 @@ __global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, co
         for (int u = 0; u < kMomTileRows / kMomThreads; ++u) {
           const int64_t i = tile * kMomTileRows + u * kMomThreads + threadIdx.x;
           if (i < rw.dim) {
-            const double2 xi = __ldg(x + i), yi = y[i];
+            const double2 xi = x[i], yi = y[i];
             dot = fma(xi.x, yi.x, fma(xi.y, yi.y, dot));
           }
         }

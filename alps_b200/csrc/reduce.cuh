@@ -20,7 +20,11 @@ constexpr int kFinishThreads = 1024;
 // Programmatic dependent launch: a kernel of the Lanczos chain lets the next
 // one start at once (chain_next), and waits for the one before it to be
 // complete before it touches anything that one writes (chain_wait).  What runs
-// before chain_wait reads only the handle's tables.
+// before chain_wait reads only the handle's tables.  The vectors, partials and
+// scalars of the chain are read by plain loads through pointers that promise
+// nothing: memory written while a kernel lives is none for a non-coherent load
+// (__ldg, or what the compiler makes of const __restrict__), and the accesses of
+// a __restrict__ pointer may be moved across the wait.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -97,7 +101,7 @@ __device__ __forceinline__ void finish_sum(const double* __restrict__ part, int6
 // tree exactly as in finish_sum, so the result is bit-identical.  For short
 // partial lists, where every CTA of a kernel can afford to read them all.
 template <int NT>
-__device__ __forceinline__ double finish_sum_in_cta(const double* __restrict__ part, int64_t n, double* sm) {
+__device__ __forceinline__ double finish_sum_in_cta(const double* part, int64_t n, double* sm) {
   static_assert(NT % 32 == 0 && kFinishThreads % NT == 0, "block size");
   constexpr int kVirt = kFinishThreads / NT;  // virtual warps per real warp
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;

@@ -615,8 +615,7 @@ __global__ void __launch_bounds__(kSpinThreads) spin_hv_kernel(const __grid_cons
 // The rows apply (spin_rows.cuh).
 template <int D, int B, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) spin_rows_kernel(const SpinDev t, const __grid_constant__ SpinRowVals vals,
-                                                             const double* __restrict__ x, double* y,
-                                                             double* __restrict__ alpha_part) {
+                                                             const double* x, double* y, double* alpha_part) {
   extern __shared__ __align__(16) unsigned char spin_dyn[];
   __shared__ SpinRowsSmem sm;
   const size_t pb = spin_block_prog_bytes(D, t.n_hh, t.n_x, t.n_key);

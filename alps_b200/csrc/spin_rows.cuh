@@ -203,8 +203,8 @@ __device__ __forceinline__ void spin_fetch(const SpinDev& t, int64_t ub, unsigne
 // Bundle ub, whose programs are in (or on their way into) prog; the next
 // bundle's (next < 0: none) go to other while this one runs.
 template <int D, int B, int NT>
-__device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next, const double* __restrict__ x,
-                                                 double* y, double* __restrict__ alpha_part, SpinRowsSmem& sm,
+__device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next, const double* x, double* y,
+                                                 double* alpha_part, SpinRowsSmem& sm,
                                                  unsigned char* xs, unsigned char* prog, unsigned char* other,
                                                  size_t pb) {
   constexpr int BITS = D <= 2 ? 1 : D <= 4 ? 2 : 3;
@@ -228,8 +228,8 @@ __device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next,
     const bool two = i + NT < nk;
 #pragma unroll
     for (int j = 0; j < B; ++j) {
-      a.v[j] = j < nv ? __ldg(x + bj[j] + i) : 0.0;
-      b.v[j] = j < nv && two ? __ldg(x + bj[j] + i + NT) : 0.0;
+      a.v[j] = j < nv ? x[bj[j] + i] : 0.0;
+      b.v[j] = j < nv && two ? x[bj[j] + i + NT] : 0.0;
     }
     rows[i] = a;
     if (two) rows[i + NT] = b;
@@ -287,7 +287,7 @@ __device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next,
 #pragma unroll
       for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int j = 0; j < B; ++j) v[q][j] = __ldg(xr + g[j].nb[o + q]);
+        for (int j = 0; j < B; ++j) v[q][j] = xr[g[j].nb[o + q]];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -299,7 +299,7 @@ __device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next,
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int j = 0; j < B; ++j) v[q][j] = o + q < nhh[j] ? __ldg(xr + g[j].nb[o + q]) : 0.0;
+        for (int j = 0; j < B; ++j) v[q][j] = o + q < nhh[j] ? xr[g[j].nb[o + q]] : 0.0;
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -318,8 +318,8 @@ __device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next,
 #pragma unroll
         for (int j = 0; j < B; ++j) {
           v[j] = w[j] = 0.0;
-          if (e != kSpinNone) v[j] = __ldg(x + (g[j].xop[o].x + (e & 0xffffffu)));
-          if (f != kSpinNone) w[j] = __ldg(x + (g[j].xop[o + 1].x + (f & 0xffffffu)));
+          if (e != kSpinNone) v[j] = x[g[j].xop[o].x + (e & 0xffffffu)];
+          if (f != kSpinNone) w[j] = x[g[j].xop[o + 1].x + (f & 0xffffffu)];
         }
         if (e != kSpinNone) {
           const double c = g[0].xc[o * D + (e >> 24)];
@@ -343,8 +343,8 @@ __device__ __forceinline__ void spin_rows_bundle(const SpinDev& t, int64_t next,
           const uint32_t e = __ldg(t.xtab + a.y + u);
           const uint32_t f = two ? __ldg(t.xtab + b.y + u) : kSpinNone;
           double v = 0.0, w = 0.0;
-          if (e != kSpinNone) v = __ldg(x + (a.x + (e & 0xffffffu)));
-          if (f != kSpinNone) w = __ldg(x + (b.x + (f & 0xffffffu)));
+          if (e != kSpinNone) v = x[a.x + (e & 0xffffffu)];
+          if (f != kSpinNone) w = x[b.x + (f & 0xffffffu)];
           if (e != kSpinNone) acc[j] = fma(g[j].xc[o * D + (e >> 24)], v, acc[j]);
           if (f != kSpinNone) acc[j] = fma(g[j].xc[(o + 1) * D + (f >> 24)], w, acc[j]);
         }

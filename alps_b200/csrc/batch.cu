@@ -21,6 +21,7 @@
 #include "apply.cuh"
 #include "apply_rows.cuh"
 #include "batch.cuh"
+#include "launch_limits.h"
 #include "reduce.cuh"
 #include "rr_core.h"
 #include "tmatrix_core.h"
@@ -861,21 +862,13 @@ const Cand32 kCand32[kBatchCand32] = {
     {b_hv32<512, 2>, 512, "n512"},
     {b_hv32<1024, 1>, 1024, "n1024"},
 };
-int g_c32[kBatchCand32] = {}, g_c32_smem[kBatchCand32] = {-1, -1, -1, -1};
-int g_hv64 = 0, g_hv64_smem = -1;
-int g_rr = 0, g_rr_smem = -1;
+KernelLimits g_c32[kBatchCand32], g_hv64, g_rr;
 
-// Grid of an apply kernel for `smem` bytes of dynamic shared memory (cached per size).
+// Grid of an apply kernel for `smem` bytes of dynamic shared memory.
 template <typename K>
-int hv_grid(K kern, int threads, int smem, int* g, int* g_smem) {
-  if (smem != *g_smem) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem);
-    *g = sms() * (per < 1 ? 1 : per);
-    *g_smem = smem;
-  }
-  return *g;
+int hv_grid(K kern, int threads, int smem, KernelLimits& limits) {
+  const int per = limits.ctas_per_sm((const void*)kern, threads, (size_t)smem);
+  return sms() * (per < 1 ? 1 : per);
 }
 
 int check(const char* what) {
@@ -907,9 +900,9 @@ size_t batch_hv_smem_limit() {
 
 int batch_prepare(const BatchArgs& a) {
   for (int c = 0; c < kBatchCand32; ++c)
-    hv_grid(kCand32[c].kern, kCand32[c].threads, a.hv_smem, &g_c32[c], &g_c32_smem[c]);
-  hv_grid(b_hv64, kHvThreads, a.hv_smem64, &g_hv64, &g_hv64_smem);
-  hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, &g_rr, &g_rr_smem);
+    hv_grid(kCand32[c].kern, kCand32[c].threads, a.hv_smem, g_c32[c]);
+  hv_grid(b_hv64, kHvThreads, a.hv_smem64, g_hv64);
+  hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, g_rr);
   return check("batched apply attributes");
 }
 
@@ -927,8 +920,7 @@ int batch_launch_hv32(const BatchArgs& a, int cand, int bucket, cudaStream_t st)
   const int lo = bucket == 0 ? -1 : kBatchBucketHi[bucket - 1];
   const int hi = bucket + 1 == kBatchBuckets ? 0x7fffffff : kBatchBucketHi[bucket];
   const Cand32& k = kCand32[cand];
-  k.kern<<<hv_grid(k.kern, k.threads, a.hv_smem, &g_c32[cand], &g_c32_smem[cand]), k.threads, a.hv_smem, st>>>(
-      a, bucket, lo, hi);
+  k.kern<<<hv_grid(k.kern, k.threads, a.hv_smem, g_c32[cand]), k.threads, a.hv_smem, st>>>(a, bucket, lo, hi);
   return check("batched FP32 apply");
 }
 
@@ -974,7 +966,7 @@ int batch_record_step(const BatchArgs& a, const int* choice32, cudaStream_t st) 
     const int rc = batch_launch_hv32(a, choice32[b], b, st);
     if (rc) return rc;
   }
-  b_hv64<<<hv_grid(b_hv64, kHvThreads, a.hv_smem64, &g_hv64, &g_hv64_smem), kHvThreads, a.hv_smem64, st>>>(a);
+  b_hv64<<<hv_grid(b_hv64, kHvThreads, a.hv_smem64, g_hv64), kHvThreads, a.hv_smem64, st>>>(a);
   b_alpha<<<ni, 256, 0, st>>>(a);
   b_update<<<gchunk, kRedThreads, 0, st>>>(a);
   b_beta<<<ni, 256, 0, st>>>(a);
@@ -988,7 +980,7 @@ int batch_record_check(const BatchArgs& a, cudaStream_t st) {
   const int gchunk = sms() * 8;
   b_check<<<ni, 32, 0, st>>>(a);
   b_rr_combine<<<gchunk, kRedThreads, 0, st>>>(a);
-  b_rr_apply<<<hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, &g_rr, &g_rr_smem), kHvThreads, a.hv_smem64, st>>>(a);
+  b_rr_apply<<<hv_grid(b_rr_apply, kHvThreads, a.hv_smem64, g_rr), kHvThreads, a.hv_smem64, st>>>(a);
   b_rr_gram<<<gchunk, kRedThreads, 0, st>>>(a);
   b_rr_finish<<<ni, 256, 0, st>>>(a, 0);
   b_rr_solve<<<(ni + 127) / 128, 128, 0, st>>>(a);

@@ -15,12 +15,14 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <type_traits>
 
 #include "apply.cuh"
 #include "apply_rows.cuh"
 #include "apply_stream.cuh"
 #include "kernels.cuh"
+#include "launch_limits.h"
 #include "reduce.cuh"
 
 namespace aed {
@@ -597,30 +599,9 @@ constexpr int kSmallVariant = 12;  // row8n1024: the most threads on each of the
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 
 // Launch shapes are computed once per kernel (and per shared-memory size or
-// sector shape) and kept in maps guarded by g_grid_mu: handles on several host
-// threads launch the same kernels.  The dynamic shared-memory limit of a
-// kernel is raised once, to the most the device allows, so that a launch on
-// one thread never sees another thread's smaller limit.
+// sector shape) and kept in maps guarded by a mutex: handles on several host
+// threads launch the same kernels.
 std::mutex g_grid_mu;
-
-template <typename K>
-int raise_smem_limit(K kern, size_t* static_bytes) {
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) {
-    const cudaError_t e = cudaGetLastError();
-    return fail(AED_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
-  }
-  const int most = optin - (int)fa.sharedSizeBytes;
-  if (most > 0 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) {
-    const cudaError_t e = cudaGetLastError();
-    return fail(AED_ERR_CUDA, std::string("kernel shared memory limit: ") + cudaGetErrorString(e));
-  }
-  *static_bytes = fa.sharedSizeBytes;
-  return most > 0 ? AED_OK : kVariantNotApplicable;
-}
 
 template <typename T, typename Acc, int R, int B>
 int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
@@ -660,35 +641,16 @@ int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double*
   constexpr bool kDraws = NT <= 512;
   auto kern = hvr_kernel<T, Acc, B, NT, MINB, false>;
   auto draws = hvr_kernel<T, Acc, B, NT, MINB, kDraws>;
-  static int limit_rc = -1;
-  static size_t static_bytes = 0;
-  static std::map<size_t, int> grids;  // dyn -> grid (0: does not fit)
-  int grid = 0;
-  {
-    std::lock_guard<std::mutex> lk(g_grid_mu);
-    if (limit_rc < 0) {
-      limit_rc = raise_smem_limit(draws, &static_bytes);
-      if (limit_rc == AED_OK) limit_rc = raise_smem_limit(kern, &static_bytes);
-    }
-    if (limit_rc == AED_ERR_CUDA) return limit_rc;
-    auto it = grids.find(dyn);
-    if (it == grids.end()) {
-      int per_sm = 0;
-      int dev = 0, optin = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      if (limit_rc == AED_OK && static_bytes + dyn <= (size_t)optin)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, dyn);
-      it = grids.emplace(dyn, per_sm < 1 ? 0 : num_sms() * per_sm).first;
-    }
-    grid = it->second;
-  }
-  if (grid <= 0) return kVariantNotApplicable;
-  int64_t g = grid;
+  static KernelLimits kern_limits, draws_limits;
+  const int per_sm = kern_limits.ctas_per_sm((const void*)kern, NT, dyn);
+  if (per_sm < 0) return per_sm;
+  if (per_sm == 0) return kVariantNotApplicable;
+  int64_t g = (int64_t)num_sms() * per_sm;
   const int64_t nb = t.n_blk / B;
   if (g > nb) g = nb;
   if (g < 1) return AED_OK;
-  launch_chained(kDraws && nb > 3 * g ? draws : kern, (unsigned)g, NT, dyn, st, t, x, y, alpha_part);
+  const bool draw = kDraws && nb > 3 * g && draws_limits.ctas_per_sm((const void*)draws, NT, dyn) > 0;
+  launch_chained(draw ? draws : kern, (unsigned)g, NT, dyn, st, t, x, y, alpha_part);
   return check_launch("hvr_kernel");
 }
 
@@ -715,36 +677,30 @@ int launch_stream(int OB, const HvParams& P, const DevTables& t, const T* x, T* 
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(t.xtab)) & 15u)
     return kVariantNotApplicable;
   auto kern = hvs_kernel<T, Acc, U, kOwnD>;
-  static int limit_rc = -1;
-  static size_t static_bytes = 0;
-  static std::map<std::pair<int, int>, StreamShape> shapes;  // (maxrows, OB) -> shape
+  static KernelLimits limits;
+  size_t most = 0;
+  if (const int rc = limits.most_dynamic((const void*)kern, &most)) return rc;
+  static std::map<std::tuple<size_t, int, int>, StreamShape> shapes;  // (most, maxrows, OB) -> shape
   StreamShape sh;
   {
     std::lock_guard<std::mutex> lk(g_grid_mu);
-    if (limit_rc < 0) limit_rc = raise_smem_limit(kern, &static_bytes);
-    if (limit_rc == AED_ERR_CUDA) return limit_rc;
-    const auto key = std::make_pair(t.maxrows, OB);
+    const auto key = std::make_tuple(most, t.maxrows, OB);
     auto it = shapes.find(key);
     if (it == shapes.end()) {
       StreamShape n;
-      int dev = 0, optin = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
       n.cfg.own_bytes = (uint32_t)align16((size_t)t.maxrows * sizeof(T) + 32);
       n.cfg.xoff = n.cfg.own_bytes;
       n.cfg.stage_bytes = n.cfg.xoff + (uint32_t)align16((size_t)t.maxrows * 2 + 32);
       const uint32_t ownd_bytes = kOwnD ? (uint32_t)align16((size_t)t.maxrows * 8 + 32) : 0u;
       n.cfg.ownd_off = (uint32_t)OB * n.cfg.own_bytes;
       n.cfg.ring_off = n.cfg.ownd_off + ownd_bytes;
-      const int64_t avail = (int64_t)optin - (int64_t)static_bytes - 1024;
+      const int64_t avail = (int64_t)most - 1024;
       const int64_t S = (avail - (int64_t)n.cfg.ring_off) / (int64_t)n.cfg.stage_bytes;
-      if (limit_rc == AED_OK && S >= 2) {
+      if (S >= 2) {
         n.cfg.S = (int)(S < sapply::kMaxStages ? S : sapply::kMaxStages);
         n.cfg.OB = OB;
         n.dyn = (size_t)n.cfg.ring_off + (size_t)n.cfg.S * n.cfg.stage_bytes;
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, sapply::kThreads, n.dyn);
-        n.fits = per_sm >= 1;
+        n.fits = limits.ctas_per_sm((const void*)kern, sapply::kThreads, n.dyn) > 0;
       }
       it = shapes.emplace(key, n).first;
     }

@@ -16,12 +16,11 @@
 
 #include <algorithm>
 #include <cmath>
-#include <map>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
 #include "handle.h"
+#include "launch_limits.h"
 #include "mom_rows.cuh"
 #include "reduce.cuh"
 #include "spin.cuh"
@@ -1349,31 +1348,10 @@ int spin_rows_go(const SpinDev& t, const SpinRowVals& vals, const double* x, dou
                  cudaStream_t st) {
   auto kern = spin_rows_kernel<D, B, NT, MINB>;
   const size_t dyn = spin_rows_smem_bytes(B, t.d, t.maxrows, t.n_hh, t.n_x, t.n_key);
-  static std::mutex mu;
-  static std::map<size_t, int> grids;  // shared memory -> CTAs per SM
-  static bool raised = false;
-  int per_sm = 0;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!raised) {
-      int dev = 0, optin = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      cudaFuncAttributes fa{};
-      AED_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
-      AED_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        optin - (int)fa.sharedSizeBytes));
-      raised = true;
-    }
-    auto it = grids.find(dyn);
-    if (it == grids.end()) {
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, dyn);
-      cudaGetLastError();
-      it = grids.emplace(dyn, per_sm).first;
-    }
-    per_sm = it->second;
-  }
-  if (per_sm < 1) return kSpinRowsNone;
+  static KernelLimits limits;
+  const int per_sm = limits.ctas_per_sm((const void*)kern, NT, dyn);
+  if (per_sm < 0) return per_sm;
+  if (per_sm == 0) return kSpinRowsNone;
   const int64_t nb = t.n_rblk / B, cap = (int64_t)sm_count() * per_sm;
   launch_chained(kern, (unsigned)(nb < cap ? nb : cap), NT, dyn, st, t, vals, x, y, alpha_part);
   return check_launch_counted("spin_rows_kernel");

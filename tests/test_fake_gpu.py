@@ -1,0 +1,47 @@
+"""Host code of the engine that a single GPU cannot show: limits per device, the tuner's choice, admission to the
+batch.  On a fake CUDA runtime (fake_gpu.py); no GPU."""
+
+import pytest
+
+import fake_gpu
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return fake_gpu.link(str(tmp_path_factory.mktemp("fake")))
+
+
+CHAINS = """
+def chain(n):
+    return [(i, (i + 1) % n, 1.0, 1.0) for i in range(n)]
+def product(ham):
+    x, y = ham.new_vector(), ham.new_vector()
+    ham.mult(x, y)
+    x.free(); y.free()
+"""
+
+
+@pytest.mark.parametrize("make", ["ed.Hamiltonian(28, 14, chain(28), device=dev)",  # 55 KB of x rows
+                                  "ed.Hamiltonian(30, 15, chain(30), precision=ed.FP32, device=dev)",
+                                  "ed.Hamiltonian(16, 8, chain(16), device=dev)",
+                                  "ed.Hamiltonian(18, 18, chain(18), two_s=2, device=dev)"])
+def test_products_on_the_second_device_of_a_process(lib, make):
+    """A kernel's limit of dynamic shared memory belongs to a device: a handle on another one raises it there too."""
+    fake_gpu.run(lib, CHAINS + f"""
+fake.fake_set_cost(b"9hv_kernel", 1.0)  # the tuner takes a rows apply
+for dev in (0, 1, 0):
+    ham = {make}
+    product(ham)
+    ham.close()
+""")
+
+
+def test_servers_on_two_devices_of_a_process(lib):
+    fake_gpu.run(lib, CHAINS + """
+servers = [ed.Server(precision=ed.FP64, device=dev, max_slots=2, lane_min_dim=-1) for dev in (0, 1)]
+tickets = [s.submit(28, 14, chain(28), nev=1) for s in servers]
+for s, t in zip(servers, tickets):
+    s.step()
+    s.cancel(t)
+    s.close()
+""")

@@ -385,13 +385,16 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
-  // the first within 5 % of the fastest: the forms of one row width stand in
-  // order of CTA size, and beside the products of other streams smaller CTAs
-  // do better than alone (5x5 with 11 up FP64, 256 and 512 threads: 165 and 162
-  // us alone, 138 and 155 a product with three handles in turn)
+  // the first rows apply within 5 % of the fastest: the forms of one row width
+  // stand in order of CTA size, and beside the products of other streams smaller
+  // CTAs do better than alone (5x5 with 11 up FP64, 256 and 512 threads: 165 and
+  // 162 us alone, 138 and 155 a product with three handles in turn).  The tile
+  // apply (0) only where it beats them by more: it does not start while its
+  // predecessor ends, which a product timed alone does not show
   const float least = *std::min_element(ms_of.begin(), ms_of.end());
-  int best = 0;
-  while (!(ms_of[best] <= 1.05f * least)) ++best;
+  int best = 1;
+  while (best < hv_num_variants() && !(ms_of[best] <= 1.05f * least)) ++best;
+  if (best == hv_num_variants()) best = 0;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[key] = best;

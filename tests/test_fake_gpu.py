@@ -45,3 +45,19 @@ for s, t in zip(servers, tickets):
     s.cancel(t)
     s.close()
 """)
+
+
+@pytest.mark.parametrize("tile,rows,want", [(1.0, 1.04, "hvr_kernel"), (1.0, 1.0, "hvr_kernel"),
+                                            (1.04, 1.0, "hvr_kernel"), (1.0, 1.1, "hv_kernel"), (0.0, 0.0, "hvr_kernel")])
+def test_the_tile_apply_wins_no_near_tie(lib, tile, rows, want):
+    """The tuner takes the tile apply only where it is more than 5 % faster than every rows apply."""
+    fake_gpu.run(lib, CHAINS + f"""
+fake.fake_set_cost(b"9hv_kernel", {tile})
+fake.fake_set_cost(b"hvr_kernel", {rows})
+for precision in (ed.FP64, ed.FP32):
+    ham = ed.Hamiltonian(16, 8, chain(16), precision=precision)
+    product(ham)
+    before = fake.fake_launches(b"{want}")
+    product(ham)
+    assert fake.fake_launches(b"{want}") == before + 1
+""")

@@ -11,71 +11,74 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "aed_internal.h"
 
 namespace aed {
 
-// Of one kernel (a static object beside its launch).
+// Of one kernel (a static object beside its launch; a launch-bound product asks
+// on every call, so the few entries are searched in turn).
 class KernelLimits {
  public:
   // CTAs of `threads` threads with `dyn` bytes of dynamic shared memory that an
   // SM of the current device holds; 0: none, negative: an error code.
   int ctas_per_sm(const void* kern, int threads, size_t dyn) {
     std::lock_guard<std::mutex> lk(mu_);
-    Device* d = nullptr;
-    if (const int rc = device(kern, &d)) return rc;
-    if (dyn > d->most) return 0;
-    const auto key = std::make_pair(threads, dyn);
-    auto it = d->ctas.find(key);
-    if (it == d->ctas.end()) {
-      int n = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&n, kern, threads, dyn, 0) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-      }
-      it = d->ctas.emplace(key, n < 0 ? 0 : n).first;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    for (const Shape& s : shapes_)
+      if (s.dev == dev && s.threads == threads && s.dyn == dyn) return s.ctas;
+    size_t most = 0;
+    if (const int rc = raise(kern, dev, &most)) return rc;
+    int n = 0;
+    if (dyn <= most &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&n, kern, threads, dyn, 0) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
     }
-    return it->second;
+    shapes_.push_back({dev, threads, dyn, n < 0 ? 0 : n});
+    return shapes_.back().ctas;
   }
   // The most dynamic shared memory a CTA of the kernel may take on the current device.
   int most_dynamic(const void* kern, size_t* most) {
     std::lock_guard<std::mutex> lk(mu_);
-    Device* d = nullptr;
-    const int rc = device(kern, &d);
-    *most = rc ? 0 : d->most;
-    return rc;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return raise(kern, dev, most);
   }
 
  private:
-  struct Device {
-    size_t most = 0;
-    std::map<std::pair<int, size_t>, int> ctas;  // by (threads, dynamic shared memory)
+  struct Shape {
+    int dev, threads;
+    size_t dyn;
+    int ctas;
   };
-  int device(const void* kern, Device** out) {
-    int dev = 0, optin = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    auto it = devices_.find(dev);
-    if (e == cudaSuccess && it == devices_.end()) {
-      Device d;
+  int raise(const void* kern, int dev, size_t* most) {
+    *most = 0;
+    auto it = most_.find(dev);
+    if (it == most_.end()) {
+      int optin = 0;
+      size_t bytes = 0;
       cudaFuncAttributes fa{};
-      e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+      cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
       if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
       if (e == cudaSuccess && optin > (int)fa.sharedSizeBytes) {
-        d.most = (size_t)optin - fa.sharedSizeBytes;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.most);
+        bytes = (size_t)optin - fa.sharedSizeBytes;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       }
-      if (e == cudaSuccess) it = devices_.emplace(dev, d).first;
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(AED_ERR_CUDA, std::string("kernel shared memory limit: ") + cudaGetErrorString(e));
+      }
+      it = most_.emplace(dev, bytes).first;
     }
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(AED_ERR_CUDA, std::string("kernel shared memory limit: ") + cudaGetErrorString(e));
-    }
-    *out = &it->second;
+    *most = it->second;
     return AED_OK;
   }
   std::mutex mu_;
-  std::map<int, Device> devices_;
+  std::vector<Shape> shapes_;
+  std::map<int, size_t> most_;  // by device: the raised limit
 };
 
 }  // namespace aed

@@ -163,37 +163,10 @@ void release(aed_handle* h) {
   delete h;
 }
 
-// (Re)build the lo-neighbour table of the handle's couplings on the device.
-int upload_lo_table(aed_handle* h) {
-  const int W = h->P.n_lolo;
-  const size_t n = ((size_t)W << h->tab.Nlo) + 1;
-  int rc = AED_OK;
-  if (n > h->d_ell_n) {  // grow only: new couplings usually keep the flips
-    mem_dev_free(h->d_ell, h->stream);
-    h->d_ell = nullptr;
-    h->d_ell_n = 0;
-    if ((rc = mem_dev_alloc_n(&h->d_ell, n))) return rc;
-    h->d_ell_n = n;
-  }
-  h->dt.ell = h->d_ell;
-  h->dt.ell_w = W;
-  if ((rc = launch_lo_table(h->P, h->dt, h->d_ell, h->stream))) return rc;
-  // and in slices of 32 rows for the rows apply
-  const size_t slices = lo_slices(h->tab.Nlo), need = slices * (size_t)lo_slice_pairs(W) * 32;
-  if (need > h->d_low_n) {
-    mem_dev_free(h->d_low_e, h->stream);
-    h->d_low_e = nullptr;
-    h->d_low_n = 0;
-    if ((rc = mem_dev_alloc_n(&h->d_low_e, need))) return rc;
-    h->d_low_n = need;
-  }
-  if (!h->d_low_w && (rc = mem_dev_alloc_n(&h->d_low_w, slices))) return rc;
-  h->dt.low_e = h->d_low_e;
-  h->dt.low_w = h->d_low_w;
-  h->dt.low_st = lo_slice_pairs(W);
-  if ((rc = launch_lo_slices(h->P, h->dt, h->d_low_e, h->d_low_w, h->stream))) return rc;
-  // and the rows apply's programs (an FP32 handle's refinement applies H to
-  // FP64 vectors too); without memory for them the tile apply serves the handle
+// The rows apply's programs of the handle's couplings (an FP32 handle's
+// refinement applies H to FP64 vectors too); without memory for them the tile
+// apply serves the handle.
+int form_programs(aed_handle* h) {
   DevTables& t = h->dt;
   for (auto& e : t.rprog) e[0] = e[1] = nullptr;
   t.n_lolo = h->P.n_lolo;
@@ -202,7 +175,7 @@ int upload_lo_table(aed_handle* h) {
   t.lolo_c = h->d_lolo;
   const int n_elem = h->precision == AED_FP32 ? 2 : 1;
   int* d_ops = reinterpret_cast<int*>(h->d_scal);  // free between calls
-  int ops[4] = {};
+  int ops[4] = {}, rc = AED_OK;
   AED_CUDA_TRY(cudaMemsetAsync(d_ops, 0, sizeof ops, h->stream));
   for (int e = 0; e < n_elem; ++e)
     if ((rc = launch_row_need(h->P, t, e == 0 ? 8 : 4, d_ops + 2 * e, h->stream))) return rc;
@@ -233,6 +206,41 @@ int upload_lo_table(aed_handle* h) {
       t.rprog[e][row] = p;
     }
   return AED_OK;
+}
+
+// (Re)build the lo-neighbour table of the handle's couplings on the device.
+int upload_lo_table(aed_handle* h) {
+  const int W = h->P.n_lolo;
+  const size_t n = ((size_t)W << h->tab.Nlo) + 1;
+  int rc = AED_OK;
+  if (n > h->d_ell_n) {  // grow only: new couplings usually keep the flips
+    mem_dev_free(h->d_ell, h->stream);
+    h->d_ell = nullptr;
+    h->d_ell_n = 0;
+    if ((rc = mem_dev_alloc_n(&h->d_ell, n))) return rc;
+    h->d_ell_n = n;
+  }
+  h->dt.ell = h->d_ell;
+  h->dt.ell_w = W;
+  if ((rc = launch_lo_table(h->P, h->dt, h->d_ell, h->stream))) return rc;
+  // and in slices of 32 rows for the rows apply
+  const size_t slices = lo_slices(h->tab.Nlo), need = slices * (size_t)lo_slice_pairs(W) * 32;
+  if (need > h->d_low_n) {
+    mem_dev_free(h->d_low_e, h->stream);
+    h->d_low_e = nullptr;
+    h->d_low_n = 0;
+    if ((rc = mem_dev_alloc_n(&h->d_low_e, need))) return rc;
+    h->d_low_n = need;
+  }
+  if (!h->d_low_w && (rc = mem_dev_alloc_n(&h->d_low_w, slices))) return rc;
+  h->dt.low_e = h->d_low_e;
+  h->dt.low_w = h->d_low_w;
+  h->dt.low_st = lo_slice_pairs(W);
+  if ((rc = launch_lo_slices(h->P, h->dt, h->d_low_e, h->d_low_w, h->stream))) return rc;
+  const bool had = h->dt.rprog[0][0] != nullptr;
+  rc = form_programs(h);
+  if (had != (h->dt.rprog[0][0] != nullptr)) h->hv_var[0] = h->hv_var[1] = -1;  // the other choices: choose again
+  return rc;
 }
 
 int check_vec(const aed_handle* h, const void* p, const char* name) {
@@ -342,6 +350,10 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
       *out = v;
       return AED_OK;
     }
+  }
+  if (!h->P.finite || !h->dt.rprog[f32 ? 1 : 0][0]) {  // the tile apply alone: nothing to time or to keep for others
+    *out = 0;
+    return AED_OK;
   }
   const int64_t D = h->tab.D;
   int bucket = 0;

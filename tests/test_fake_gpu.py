@@ -61,3 +61,35 @@ for precision in (ed.FP64, ed.FP32):
     product(ham)
     assert fake.fake_launches(b"{want}") == before + 1
 """)
+
+
+OVERFLOW = """
+over = lambda n: chain(n) + [(0, 1, 0.0, 1.5e308)] * 4  # finite couplings whose merged flip is not
+fake.fake_set_cost(b"9hv_kernel", 1.0)
+def takes(ham, kernel):
+    before = fake.fake_launches(kernel)
+    product(ham)
+    return fake.fake_launches(kernel) > before
+"""
+
+
+@pytest.mark.parametrize("precision", ["ed.FP64", "ed.FP32"])
+def test_a_handle_without_programs_takes_the_tile_apply(lib, precision):
+    """Couplings that overflow when merged have no rows apply: the sizes that are not timed take the tile apply too,
+    and the choice is neither kept for other handles nor for the handle's next couplings."""
+    fake_gpu.run(lib, CHAINS + OVERFLOW + f"""
+for n in (8, 16):  # not timed; timed
+    odd = ed.Hamiltonian(n, n // 2, over(n), precision={precision})
+    x, y = odd.new_vector(), odd.new_vector()
+    assert odd.time_apply(x, y, 1)[1] == 0
+    assert takes(odd, b"9hv_kernel") and not takes(odd, b"hvr_kernel")
+    ham = ed.Hamiltonian(n, n // 2, chain(n), precision={precision})
+    product(ham)
+    assert takes(ham, b"hvr_kernel") and not takes(ham, b"9hv_kernel")
+    odd.set_couplings(chain(n))
+    product(odd)
+    assert takes(odd, b"hvr_kernel") and not takes(odd, b"9hv_kernel")
+    odd.set_couplings(over(n))
+    assert takes(odd, b"9hv_kernel") and not takes(odd, b"hvr_kernel")
+    assert odd.time_apply(x, y, 1)[1] == 0
+""")

@@ -111,7 +111,8 @@ struct aed_server {
   bool dirty = true;
   cudaGraphExec_t graph = nullptr;
   bool graph_stale = true;
-  int hv_smem = 0, hv_smem64 = 0, prog32 = 0, prog64 = 0;  // shared memory of the applies in the graph (batch.cuh)
+  // shared memory of the applies in the graph (batch.cuh), from the largest block and programs admitted so far
+  int hv_smem = 0, hv_smem64 = 0, maxrows = 0, prog32 = 0, prog64 = 0;
   int64_t launches = 0;
   // the FP32 apply kernel of each sector-size bucket (batch.cuh), tuned on
   // the first resident work of the bucket unless AED_BATCH_VARIANT forces one
@@ -261,21 +262,19 @@ int admit(aed_server* s, int k, const std::shared_ptr<Request>& r) {
     t.rcap[e][e] = row_cap_bound(elem, P);
     t.rstride[e][e] = row_prog_stride(elem, e, t.rcap[e][e]);
   }
-  {  // the graph's applies need more shared memory: capture again
+  {  // the largest programs and blocks so far, which any sector and 128 bonds fit (32 sites: 12870 rows of 16
+     // bytes and two programs of 8512); more than the graph's applies have: capture again
+    const int rows = std::max(s->maxrows, sec->maxrows);
     const int p64 = std::max(s->prog64, t.rstride[0][0]), p32 = std::max(s->prog32, t.rstride[1][1]);
-    const size_t m64 = batch_hv_smem_bytes(8, sec->maxrows, p64), m32 = batch_hv_smem_bytes(4, sec->maxrows, p32);
-    if (std::max(m64, m32) > batch_hv_smem_limit())
-      return fail(AED_ERR_INVALID, "sector too large for the batched apply's shared memory");
-    const size_t grow64 = 2 * (size_t)(p64 - s->prog64), grow32 = 2 * (size_t)(p32 - s->prog32);
-    const size_t n64 = std::max(m64, s->hv_smem64 + grow64), n32 = std::max(m32, s->hv_smem + grow32);
-    if (p64 > s->prog64 || p32 > s->prog32 || n64 > (size_t)s->hv_smem64 || n32 > (size_t)s->hv_smem) {
-      const size_t lim = batch_hv_smem_limit();
-      if (std::max(n64, n32) > lim)
+    if (rows > s->maxrows || p64 > s->prog64 || p32 > s->prog32) {
+      const size_t n64 = batch_hv_smem_bytes(8, rows, p64), n32 = batch_hv_smem_bytes(4, rows, p32);
+      if (std::max(n64, n32) > batch_hv_smem_limit())
         return fail(AED_ERR_INVALID, "sector too large for the batched apply's shared memory");
+      s->maxrows = rows;
       s->prog64 = p64;
       s->prog32 = p32;
-      s->hv_smem64 = (int)std::min(lim, (n64 + 1023) & ~(size_t)1023);
-      s->hv_smem = (int)std::min(lim, (n32 + 1023) & ~(size_t)1023);
+      s->hv_smem64 = (int)n64;
+      s->hv_smem = (int)n32;
       s->graph_stale = true;
     }
   }

@@ -93,3 +93,17 @@ for n in (8, 16):  # not timed; timed
     assert takes(odd, b"9hv_kernel") and not takes(odd, b"hvr_kernel")
     assert odd.time_apply(x, y, 1)[1] == 0
 """)
+
+
+def test_admission_to_the_batch_does_not_depend_on_what_came_before(lib):
+    """The largest blocks (32 sites) beside programs of every size up to 128 bonds, one after the other."""
+    fake_gpu.run(lib, CHAINS + """
+srv = ed.Server(precision=ed.FP64, max_slots=200, lane_min_dim=-1)
+tickets = [srv.submit(32, 8, chain(32), nev=1)]
+pairs = [(i, j, 1.0, 1.0) for i in range(16) for j in range(16, 32)]
+for n in range(1, 129):
+    tickets.append(srv.submit(32, 2, pairs[:n], nev=1))
+    srv.step()
+assert all(srv.poll(t) is None for t in tickets)  # resident: none was refused
+assert srv.stats()["resident"] == 129
+""")

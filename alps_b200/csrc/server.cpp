@@ -146,8 +146,31 @@ int dmalloc(aed_server* s, void** p, size_t bytes) {
 // FP64 Lanczos refinement.
 int rr_kmax_of(int nev) { return std::min(kMaxRR, nev + 3); }
 
+// Entries of a sector's block list (build_block_list).
+int64_t block_entries(const BasisTables& t) {
+  int64_t n = 0, c = 1;  // c: hi parts with p bits
+  for (int p = 0; p <= t.Nhi; ++p) {
+    if (t.n_up - p >= 0 && t.n_up - p <= t.Nlo) n += (c + kBundleMax - 1) / kBundleMax * kBundleMax;
+    c = c * (t.Nhi - p) / (p + 1);
+  }
+  return n;
+}
+
+// Bytes of a request's lo-neighbour table and of its applies' programs, as admit() allocates them.
+size_t row_table_bytes(const Model& m, const BasisTables& t, bool f32) {
+  HvParams P;
+  if (build_hv_params(m, t.Nlo, P)) return 0;  // refused at admission
+  size_t b = lo_slices(t.Nlo) * ((size_t)lo_slice_pairs(P.n_lolo) * 32 * sizeof(uint2) + 4);
+  for (int e = 0; e < (f32 ? 2 : 1); ++e) {
+    const int elem = e == 0 ? 8 : 4;
+    b += (size_t)(block_entries(t) / kBatchBundle) * (size_t)row_prog_stride(elem, e, row_cap_bound(elem, P));
+  }
+  return b;
+}
+
 // Bytes a request holds while resident (the admission footprint).
-size_t request_bytes(const aed_server* s, int N, int n_bonds, int64_t D, int nev, int cap, int n_store) {
+size_t request_bytes(const aed_server* s, const Model& m, const BasisTables& t, int nev, int cap, int n_store) {
+  const int64_t D = t.D;
   const size_t ldv = ((size_t)D * 4 + 255) & ~(size_t)255;
   size_t b = (size_t)D * 8;                      // diagonal
   b += 3 * (((size_t)D * 8 + 255) & ~(size_t)255);  // FP64 vectors
@@ -155,9 +178,7 @@ size_t request_bytes(const aed_server* s, int N, int n_bonds, int64_t D, int nev
   b += (size_t)sector_tiles_est(D) * 8 + (size_t)red_chunks(D) * 8;  // partials
   b += (size_t)cap * 8 * (2 + kCheckScratch + 1);                               // alpha/beta, scratch, coefficients
   b += sizeof(HvParams) + 4096;
-  const int nlo = std::max((N + 1) / 2, std::min(12, N - 2)), pairs = std::min(n_bonds, kMaxBonds);
-  b += lo_slices(nlo) * ((size_t)lo_slice_pairs(pairs) * 256 + 4);  // lo-neighbour table
-  b += ((size_t)1 << (N - nlo)) * (2 * sizeof(double) * 2 * (size_t)(pairs + 8) + 128);  // the applies' programs
+  b += row_table_bytes(m, t, s->precision == AED_FP32);
   if (s->precision == AED_FP32) {  // the Rayleigh-Ritz hand-over: K vectors and their images, sums
     const size_t k = (size_t)rr_kmax_of(nev);
     b += 2 * k * (((size_t)D * 8 + 255) & ~(size_t)255) + k * (size_t)cap * 8 +
@@ -706,7 +727,7 @@ int aed_server_submit(aed_server* s, const aed_model_desc* model, const aed_solv
   r->dim = t.D;
   const int cap = cap_of(*r, t.D);
   const int n_store = s->precision == AED_FP32 ? std::min(kServerStore, cap + 1) : 0;
-  r->footprint = request_bytes(s, r->model.N, (int)r->model.s1.size(), t.D, opts->nev, cap, n_store);
+  r->footprint = request_bytes(s, r->model, t, opts->nev, cap, n_store);
   if (r->footprint + sector_bytes(r->model.N, r->model.n_up) > s->budget)
     return fail(AED_ERR_ADMISSION, "request footprint (" + std::to_string(r->footprint) +
                                        " bytes) exceeds the server's HBM budget (" + std::to_string(s->budget) + ")");

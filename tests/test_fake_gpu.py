@@ -107,3 +107,23 @@ for n in range(1, 129):
 assert all(srv.poll(t) is None for t in tickets)  # resident: none was refused
 assert srv.stats()["resident"] == 129
 """)
+
+
+@pytest.mark.parametrize("precision", ["ed.FP64", "ed.FP32"])
+def test_a_request_is_admitted_by_what_it_allocates(lib, precision):
+    """The footprint holds what a resident request takes, and little more: also where few of the hi blocks exist."""
+    fake_gpu.run(lib, CHAINS + f"""
+pairs = [(i, j, 1.0, 1.0) for i in range(32) for j in range(i + 1, 32)]
+for n, n_up, bonds in [(32, 2, chain(32)), (32, 1, pairs[:128]), (24, 12, chain(24)), (16, 8, chain(16)),
+                       (12, 1, chain(12)), (4, 2, chain(4)), (30, 3, pairs[:100]), (27, 25, chain(27))]:
+    bonds = [b for b in bonds if b[1] < n]
+    srv = ed.Server(precision={precision}, max_slots=2, lane_min_dim=-1)
+    t = srv.submit(n, n_up, bonds, nev=1, max_iter=40)
+    srv.step()
+    used, held = srv.stats()["bytes_used"], fake.fake_pool_bytes()
+    assert held - (1 << 17) <= used <= 1.15 * held + (1 << 17), (n, n_up, used, held)  # tile lists are estimated
+    srv.cancel(t)
+    srv.step()
+    assert srv.stats()["bytes_used"] == 0
+    srv.close()
+""")

@@ -513,6 +513,22 @@ size_t lane_bytes(const aed_server* s, int64_t D, int n_store) {
   return (size_t)D * per_row + ((size_t)64 << 20);
 }
 
+// And of the programs of its rows applies (form_programs), at most: the other
+// tables fit the 64 MB above.
+size_t lane_program_bytes(const aed_server* s, const Model& m) {
+  BasisTables t;
+  HvParams P;
+  if (build_tables(m.N, m.n_up, t) || build_hv_params(m, t.Nlo, P)) return 0;
+  size_t b = 0;
+  for (int e = 0; e < (s->precision == AED_FP32 ? 2 : 1); ++e)
+    for (int row = 0; row < 2; ++row) {
+      const int elem = e == 0 ? 8 : 4;
+      b += (size_t)(block_entries(t) / row_blocks(elem, row)) *
+           (size_t)row_prog_stride(elem, row, row_cap_bound(elem, P));
+    }
+  return b;
+}
+
 void lane_main(aed_server* s, Lane* L) {
   cudaSetDevice(s->device);
   Request& r = *L->req;
@@ -777,7 +793,10 @@ int aed_server_step(aed_server* s, int32_t* n_pending) {
         ++it;
         continue;
       }
-      const size_t need = lane_bytes(s, r->dim, std::min(kServerStore, cap_of(*r, r->dim) + 1));
+      // (without memory for its programs a handle does without them: a request that fits but for
+      // them waits for an empty server, not for ever)
+      size_t need = lane_bytes(s, r->dim, std::min(kServerStore, cap_of(*r, r->dim) + 1));
+      if (need <= s->budget) need = std::min(s->budget, need + lane_program_bytes(s, r->model));
       if (s->used + need > s->budget) break;
       std::unique_ptr<Lane> L(new Lane);
       L->req = r;

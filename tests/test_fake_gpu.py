@@ -127,3 +127,24 @@ for n, n_up, bonds in [(32, 2, chain(32)), (32, 1, pairs[:128]), (24, 12, chain(
     assert srv.stats()["bytes_used"] == 0
     srv.close()
 """)
+
+
+def test_a_lane_is_counted_with_its_programs(lib):
+    """Two requests of one sector as single-instance solves, with few and with many flips outside the lo part; and a
+    budget that holds the lane but for its programs."""
+    fake_gpu.run(lib, CHAINS + """
+pairs = [(i, j, 1.0, 1.0) for i in range(15) for j in range(15, 30)]
+def counted(bonds, budget):
+    srv = ed.Server(precision=ed.FP64, max_slots=2, max_lanes=1, lane_min_dim=1000, hbm_budget=budget)
+    t = srv.submit(30, 5, bonds, nev=1, max_iter=20)
+    srv.step()
+    assert srv.stats()["queued"] == 0
+    used = srv.stats()["bytes_used"]  # 0 where the solve is over already
+    srv.close()
+    return used
+few = max(counted(pairs[:10], 8 << 30) for _ in range(5))
+many = max(counted(pairs[:120], 8 << 30) for _ in range(5))
+blocks = 4944  # hi parts of 15 sites with at most 5 up spins
+assert few == 0 or many == 0 or many - few > 110 * 16 * blocks
+counted(pairs[:120], (64 << 20) + 142506 * (60 + 16 * 24))
+""")

@@ -148,8 +148,7 @@ void release(aed_handle* h) {
                   (void*)h->d_reps, (void*)h->d_norm, (void*)h->d_mdiag, (void*)h->d_map, (void*)h->d_sthi,
                   (void*)h->d_stlo, (void*)h->d_slolist, (void*)h->d_slooff, (void*)h->d_sblk_hi,
                   (void*)h->d_sblk_off, (void*)h->d_stile_blk, (void*)h->d_stile_r, (void*)h->d_sreps,
-                  (void*)h->d_slol, (void*)h->d_srblk, (void*)h->d_stfirst, (void*)h->d_slow_w, (void*)h->d_sxtab,
-                  (void*)h->d_slow_e, (void*)h->d_slokey, (void*)h->d_srprog, (void*)h->d_slodiag, (void*)h->d_sxoff, (void*)h->d_sxdiag, (void*)h->d_scross,
+                  (void*)h->d_slol, (void*)h->d_srblk, (void*)h->d_stfirst, (void*)h->d_srows,
                   (void*)h->d_low_e, (void*)h->d_low_w, (void*)h->d_rprog, (void*)h->d_lolo})
     mem_dev_free(p, h->stream);
   mom_rows_free(h->mrows, h->stream);
@@ -845,59 +844,53 @@ int spin_rows_tables(aed_handle* h, bool* built) {
   if (const char* e = std::getenv("AED_SPIN_ROWS"); e && e[0] == '0') return AED_OK;
   SpinRowsPlan r;
   if (!spin_rows_plan(*h->sp, t, r)) return AED_OK;
-  const size_t slices = spin_low_slices(t), pairs = slices * (size_t)t.low_st * 32;
-  const size_t xt = (size_t)t.n_xtab * (2 * t.d - 1) * t.n_lo;
-  auto grow = [&](auto** p, size_t n) {
-    mem_dev_free(*p, h->stream);
-    *p = nullptr;
-    return mem_dev_alloc_n(p, n) == AED_OK;
-  };
-  bool ok = h->d_srblk && h->d_stfirst;
-  if (ok && (!h->d_slow_w || pairs > h->slow_n)) {
-    h->slow_n = 0;
-    ok = grow(&h->d_slow_e, pairs) && grow(&h->d_slow_w, slices) && grow(&h->d_slodiag, (size_t)t.n_lo) &&
-         grow(&h->d_slokey, (size_t)t.n_lo);
-    if (ok) h->slow_n = pairs;
+  if (!h->d_srblk || !h->d_stfirst) return AED_OK;
+  // one block for all tables: each allocation of its own costs the first handle
+  // of a size 0.1 to 0.4 ms
+  const size_t slices = spin_low_slices(t), n_lo = (size_t)t.n_lo;
+  const size_t bytes[] = {slices * (size_t)t.low_st * 32 * sizeof(uint2),
+                          slices * 4,
+                          n_lo * 8,
+                          n_lo,
+                          (size_t)t.n_xtab * (2 * t.d - 1) * n_lo * 4,
+                          r.cross.size() * sizeof(SpinCross),
+                          r.xoff.size() * 8,
+                          r.xdiag.size() * 8,
+                          spin_prog_bytes(t)};
+  enum { kLowE, kLowW, kLodiag, kLokey, kXtab, kCross, kXoff, kXdiag, kProg, kTables };
+  size_t at[kTables], need = 0;
+  for (int q = 0; q < kTables; ++q) {
+    at[q] = need;
+    need += (bytes[q] + 255) & ~(size_t)255;
   }
-  if (ok && xt > h->sxtab_n) {
-    h->sxtab_n = 0;
-    ok = grow(&h->d_sxtab, xt);
-    if (ok) h->sxtab_n = xt;
+  if (need > h->srows_n) {
+    mem_dev_free(h->d_srows, h->stream);
+    h->d_srows = nullptr;
+    h->srows_n = 0;
+    if (mem_dev_alloc_n(&h->d_srows, need)) return AED_OK;
+    h->srows_n = need;
   }
-  if (ok && r.cross.size() > h->scross_n) {
-    h->scross_n = 0;
-    ok = grow(&h->d_scross, r.cross.size()) && grow(&h->d_sxoff, r.xoff.size()) && grow(&h->d_sxdiag, r.xdiag.size());
-    if (ok) h->scross_n = r.cross.size();
-  }
-  const size_t progs = spin_prog_bytes(t);
-  if (ok && progs > h->srprog_n) {
-    h->srprog_n = 0;
-    ok = grow(&h->d_srprog, progs);
-    if (ok) h->srprog_n = progs;
-  }
-  if (!ok) return AED_OK;
-  if (!r.cross.empty()) {
-    AED_CUDA_TRY(cudaMemcpyAsync(h->d_scross, r.cross.data(), r.cross.size() * sizeof(SpinCross),
-                                 cudaMemcpyHostToDevice, h->stream));
-    AED_CUDA_TRY(cudaMemcpyAsync(h->d_sxoff, r.xoff.data(), r.xoff.size() * 8, cudaMemcpyHostToDevice, h->stream));
-    AED_CUDA_TRY(cudaMemcpyAsync(h->d_sxdiag, r.xdiag.data(), r.xdiag.size() * 8, cudaMemcpyHostToDevice, h->stream));
-  }
-  int rc = launch_spin_rows_tables(*h->sp, t, r, h->d_slow_e, h->d_slow_w, h->d_slodiag, h->d_slokey, h->d_sxtab,
-                                         h->stream);
+  unsigned char* p[kTables];
+  for (int q = 0; q < kTables; ++q) p[q] = h->d_srows + at[q];
+  const void* up[] = {r.cross.data(), r.xoff.data(), r.xdiag.data()};
+  for (int q = 0; q < (r.cross.empty() ? 0 : 3); ++q)
+    AED_CUDA_TRY(cudaMemcpyAsync(p[kCross + q], up[q], bytes[kCross + q], cudaMemcpyHostToDevice, h->stream));
+  int rc = launch_spin_rows_tables(*h->sp, t, r, (uint2*)p[kLowE], (uint32_t*)p[kLowW], (double*)p[kLodiag], p[kLokey],
+                                   (uint32_t*)p[kXtab], h->stream);
   if (rc) return rc;
   t.rblk = h->d_srblk;
   t.tfirst = h->d_stfirst;
-  t.low_e = h->d_slow_e;
-  t.low_w = h->d_slow_w;
-  t.lodiag = h->d_slodiag;
-  t.lokey = h->d_slokey;
-  t.cross = h->d_scross;
-  t.xtab = h->d_sxtab;
-  t.xoff = h->d_sxoff;
-  t.xdiag = h->d_sxdiag;
-  t.rprog = h->d_srprog;
+  t.low_e = (const uint2*)p[kLowE];
+  t.low_w = (const uint32_t*)p[kLowW];
+  t.lodiag = (const double*)p[kLodiag];
+  t.lokey = p[kLokey];
+  t.cross = (const SpinCross*)p[kCross];
+  t.xtab = (const uint32_t*)p[kXtab];
+  t.xoff = (const double*)p[kXoff];
+  t.xdiag = (const double*)p[kXdiag];
+  t.rprog = p[kProg];
   h->srow_vals = r.vals;
-  if ((rc = launch_spin_progs(*h->sp, t, h->d_srprog, h->stream))) return rc;
+  if ((rc = launch_spin_progs(*h->sp, t, p[kProg], h->stream))) return rc;
   AED_CUDA_TRY(cudaStreamSynchronize(h->stream));  // r goes out of scope
   *built = true;
   return AED_OK;

@@ -68,13 +68,9 @@ struct aed_handle {
   uint32_t *d_sthi = nullptr, *d_stlo = nullptr, *d_slolist = nullptr, *d_slooff = nullptr;
   uint32_t *d_sblk_hi = nullptr, *d_sblk_off = nullptr, *d_stile_blk = nullptr, *d_stile_r = nullptr;
   // the rows apply's tables (SpinDev::rblk ..)
-  uint32_t *d_srblk = nullptr, *d_stfirst = nullptr, *d_slow_w = nullptr, *d_sxtab = nullptr;
-  uint2* d_slow_e = nullptr;
-  uint8_t* d_slokey = nullptr;
-  unsigned char* d_srprog = nullptr;
-  double *d_slodiag = nullptr, *d_sxoff = nullptr, *d_sxdiag = nullptr;
-  aed::SpinCross* d_scross = nullptr;
-  size_t slow_n = 0, sxtab_n = 0, scross_n = 0, srprog_n = 0;
+  uint32_t *d_srblk = nullptr, *d_stfirst = nullptr;
+  unsigned char* d_srows = nullptr;  // one after the other
+  size_t srows_n = 0;                // bytes allocated
   aed::SpinRowVals srow_vals{};
   uint2* d_slol = nullptr;  // the lo table of the tabulated Sz-sector apply (sdev.lol), slol_bytes allocated
   size_t slol_bytes = 0;

@@ -211,27 +211,34 @@ int form_programs(aed_handle* h) {
 int upload_lo_table(aed_handle* h) {
   const int W = h->P.n_lolo;
   const size_t n = ((size_t)W << h->tab.Nlo) + 1;
+  // and in slices of 32 rows for the rows apply
+  const size_t slices = lo_slices(h->tab.Nlo), need = slices * (size_t)lo_slice_pairs(W) * 32;
   int rc = AED_OK;
-  if (n > h->d_ell_n) {  // grow only: new couplings usually keep the flips
+  // grow only (new couplings usually keep the flips), the old blocks given back
+  // once there are new ones: without memory the handle keeps the tables it reads
+  uint32_t* ell = nullptr;
+  uint2* low = nullptr;
+  if (n > h->d_ell_n) rc = mem_dev_alloc_n(&ell, n);
+  if (!rc && need > h->d_low_n) rc = mem_dev_alloc_n(&low, need);
+  if (!rc && !h->d_low_w) rc = mem_dev_alloc_n(&h->d_low_w, slices);
+  if (rc) {
+    mem_dev_free(ell, h->stream);
+    mem_dev_free(low, h->stream);
+    return rc;
+  }
+  if (ell) {
     mem_dev_free(h->d_ell, h->stream);
-    h->d_ell = nullptr;
-    h->d_ell_n = 0;
-    if ((rc = mem_dev_alloc_n(&h->d_ell, n))) return rc;
+    h->d_ell = ell;
     h->d_ell_n = n;
+  }
+  if (low) {
+    mem_dev_free(h->d_low_e, h->stream);
+    h->d_low_e = low;
+    h->d_low_n = need;
   }
   h->dt.ell = h->d_ell;
   h->dt.ell_w = W;
   if ((rc = launch_lo_table(h->P, h->dt, h->d_ell, h->stream))) return rc;
-  // and in slices of 32 rows for the rows apply
-  const size_t slices = lo_slices(h->tab.Nlo), need = slices * (size_t)lo_slice_pairs(W) * 32;
-  if (need > h->d_low_n) {
-    mem_dev_free(h->d_low_e, h->stream);
-    h->d_low_e = nullptr;
-    h->d_low_n = 0;
-    if ((rc = mem_dev_alloc_n(&h->d_low_e, need))) return rc;
-    h->d_low_n = need;
-  }
-  if (!h->d_low_w && (rc = mem_dev_alloc_n(&h->d_low_w, slices))) return rc;
   h->dt.low_e = h->d_low_e;
   h->dt.low_w = h->d_low_w;
   h->dt.low_st = lo_slice_pairs(W);
@@ -1232,6 +1239,8 @@ int aed_set_couplings(aed_handle* h, const aed_model_desc* model) {
   }
   DeviceGuard g(h->device);
   AED_CUDA_TRY(cudaStreamSynchronize(h->stream));  // no apply of the old couplings in flight
+  const Model old_model = h->model;
+  const HvParams old_P = h->P;
   h->model = m;
   h->P = P;
   // the recurrence of the last solve belongs to the old Hamiltonian
@@ -1250,7 +1259,13 @@ int aed_set_couplings(aed_handle* h, const aed_model_desc* model) {
     AED_CUDA_TRY(cudaStreamSynchronize(h->stream));
     return AED_OK;
   }
-  if ((rc = upload_lo_table(h))) return rc;
+  if ((rc = upload_lo_table(h))) {
+    if (rc == AED_ERR_NOMEM) {  // nothing was touched: the old couplings stay
+      h->model = old_model;
+      h->P = old_P;
+    }
+    return rc;
+  }
   rc = launch_diag_table(h->P, h->dt, h->d_dg, h->stream);
   if (!rc && h->d_dgf) rc = launch_round_to_f32(h->d_dg, h->d_dgf, h->tab.D, h->stream);
   if (rc) return rc;

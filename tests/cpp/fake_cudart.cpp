@@ -26,6 +26,8 @@ std::map<std::string, double> g_cost;                   // ms of the launches wh
 std::map<void*, size_t> g_pool;                         // stream-ordered blocks
 size_t g_pool_bytes = 0;
 double g_clock = 0.0;
+bool g_no_memory = false;
+int g_frees = 0;
 struct Event {
   double at;
 };
@@ -62,6 +64,8 @@ extern "C" {
 void fake_set_optin(int dev, int bytes) { g_optin[dev] = bytes; }
 void fake_set_cost(const char* part, double ms) { g_cost[part] = ms; }
 size_t fake_pool_bytes() { return g_pool_bytes; }
+void fake_no_memory(int on) { g_no_memory = on != 0; }
+int fake_frees() { return g_frees; }  // blocks given back by cudaFree
 int fake_launches(const char* part) {
   std::lock_guard<std::mutex> lk(g_mu);
   int n = 0;
@@ -139,17 +143,25 @@ cudaError_t cudaGetLastError() {
   t_err = cudaSuccess;
   return e;
 }
-cudaError_t cudaMalloc(void** p, size_t n) {
+static cudaError_t host_alloc(void** p, size_t n) {
   *p = std::calloc(n ? n : 1, 1);
   return *p ? cudaSuccess : set(cudaErrorMemoryAllocation);
 }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  *p = nullptr;
+  return g_no_memory ? set(cudaErrorMemoryAllocation) : host_alloc(p, n);
+}
 cudaError_t cudaFree(void* p) {
+  ++g_frees;
   std::free(p);
   return cudaSuccess;
 }
-cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
-cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return host_alloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return host_alloc(p, n); }
+cudaError_t cudaFreeHost(void* p) {
+  std::free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) {
   const cudaError_t e = cudaMalloc(p, n);
   std::lock_guard<std::mutex> lk(g_mu);
@@ -162,7 +174,8 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t) {
     g_pool_bytes -= g_pool[p];
     g_pool.erase(p);
   }
-  return cudaFree(p);
+  std::free(p);
+  return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* fr, size_t* tot) {
   *fr = *tot = (size_t)180 << 30;

@@ -148,3 +148,24 @@ blocks = 4944  # hi parts of 15 sites with at most 5 up spins
 assert few == 0 or many == 0 or many - few > 110 * 16 * blocks
 counted(pairs[:120], (64 << 20) + 142506 * (60 + 16 * 24))
 """)
+
+
+@pytest.mark.parametrize("precision", ["ed.FP64", "ed.FP32"])
+def test_couplings_without_memory_leave_the_handle_its_tables(lib, precision):
+    """New couplings whose tables find no memory are refused; the tables that a later product reads stay allocated."""
+    fake_gpu.run(lib, CHAINS + f"""
+ham = ed.Hamiltonian(16, 8, chain(16), precision={precision})
+product(ham)
+ed.empty_cache()
+before = fake.fake_frees()
+fake.fake_no_memory(1)
+try:
+    ham.set_couplings([(i, j, 1.0, 1.0) for i in range(16) for j in range(i + 1, 16)])
+    assert False
+except ed.AEDError as e:
+    assert e.code == ed.ERR_NOMEM
+assert fake.fake_frees() == before
+fake.fake_no_memory(0)
+ham.set_couplings(chain(16))
+product(ham)
+""")

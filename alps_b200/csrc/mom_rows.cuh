@@ -33,6 +33,7 @@ struct MomRowMarks {
   unsigned long long norm[kMomRowNorms];
   uint32_t used[kMomRowNorms];
   uint32_t many;  // more normalisations than slots
+  unsigned long long total;  // sum of the slices' widths (mom_row_scan_kernel)
 };
 
 struct MomRowSpec {

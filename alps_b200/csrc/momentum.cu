@@ -330,6 +330,53 @@ __global__ void __launch_bounds__(kMomThreads) mom_row_kernel(const __grid_const
   }
 }
 
+// off[s] = sum of width[0 .. s), off[n] and marks->total the sum of all (off
+// means something where that is below 2^32).  One CTA, eight neighbouring
+// widths per thread and pass.
+__global__ void __launch_bounds__(1024) mom_row_scan_kernel(const uint32_t* __restrict__ width, int64_t n,
+                                                            uint32_t* __restrict__ off,
+                                                            MomRowMarks* __restrict__ marks) {
+  constexpr int U = 8;
+  __shared__ unsigned long long sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long run = 0;
+  for (int64_t b = 0; b < n; b += 1024 * U) {
+    const int64_t i0 = b + (int64_t)threadIdx.x * U;
+    uint32_t w[U];
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      w[u] = i0 + u < n ? width[i0 + u] : 0u;
+      mine += w[u];
+    }
+    unsigned long long upto = mine;  // of this warp's threads up to this one
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    unsigned long long before = 0, all = 0;
+    for (int q = 0; q < 32; ++q) {
+      if (q < warp) before += sums[q];
+      all += sums[q];
+    }
+    unsigned long long at = run + before + upto - mine;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u < n) {
+        off[i0 + u] = (uint32_t)at;
+        at += w[u];
+      }
+    run += all;
+    __syncthreads();  // sums are read
+  }
+  if (threadIdx.x == 0) {
+    off[n] = (uint32_t)run;
+    marks->total = run;
+  }
+}
+
 // U terms of a row: the x_j of all of them asked for, then added in order.  A
 // padding entry adds 0 * 0; a term whose n_j differs from n_i has its
 // coefficient beyond the n_base staged ones, in global memory.
@@ -634,11 +681,11 @@ int mom_rows_begin(const double* norm, int64_t dim, MomRowStore& rs, cudaStream_
 }
 
 int mom_rows_plan(const MomParams& mp, int64_t dim, MomRowSpec& spec, MomRowStore& rs, cudaStream_t st) {
-  const int64_t slices = (dim + 31) / 32;
+  mom_row_scan_kernel<<<1, 1024, 0, st>>>(rs.width, (dim + 31) / 32, rs.off, rs.marks);
+  int rc = check_launch_counted("mom_row_scan_kernel");
+  if (rc) return rc;
   MomRowMarks mk;
-  std::vector<uint32_t> w((size_t)slices), o((size_t)slices + 1);
   AED_CUDA_TRY(cudaMemcpyAsync(&mk, rs.marks, sizeof mk, cudaMemcpyDeviceToHost, st));
-  AED_CUDA_TRY(cudaMemcpyAsync(w.data(), rs.width, (size_t)slices * 4, cudaMemcpyDeviceToHost, st));
   AED_CUDA_TRY(cudaStreamSynchronize(st));
   if (mk.many) return kMomRowsNone;
   // the ratios n_j / n_i that occur, 1 first
@@ -663,14 +710,8 @@ int mom_rows_plan(const MomParams& mp, int64_t dim, MomRowSpec& spec, MomRowStor
   while (((int64_t)1 << jb) <= dim) ++jb;  // dim < 2^jb
   if (n_idx > (size_t)kMomRowIdx || n_idx >= ((uint64_t)1 << (32 - jb))) return kMomRowsNone;  // no entry is all ones
   spec.jbits = jb;
-  uint64_t run = 0;
-  for (int64_t s = 0; s < slices; ++s) {
-    o[(size_t)s] = (uint32_t)run;
-    run += w[(size_t)s];
-  }
-  o[(size_t)slices] = (uint32_t)run;
-  if (run >= 0xffffffffull) return kMomRowsNone;
-  const size_t need = (size_t)run * 32;
+  if (mk.total >= 0xffffffffull) return kMomRowsNone;
+  const size_t need = (size_t)mk.total * 32;
   if (need > rs.ent_cap) {
     mem_dev_free(rs.ent, st);
     rs.ent = nullptr;
@@ -688,9 +729,8 @@ int mom_rows_plan(const MomParams& mp, int64_t dim, MomRowSpec& spec, MomRowStor
         cf[k++] = f * mp.phase_re[t];
         cf[k++] = f * mp.phase_im[t];
       }
-  AED_CUDA_TRY(cudaMemcpyAsync(rs.off, o.data(), o.size() * 4, cudaMemcpyHostToDevice, st));
   AED_CUDA_TRY(cudaMemcpyAsync(rs.cf, cf.data(), cf.size() * 8, cudaMemcpyHostToDevice, st));
-  AED_CUDA_TRY(cudaStreamSynchronize(st));  // o and cf go out of scope
+  AED_CUDA_TRY(cudaStreamSynchronize(st));  // cf goes out of scope, and the applies read it before they wait
   return AED_OK;
 }
 

@@ -169,3 +169,13 @@ fake.fake_no_memory(0)
 ham.set_couplings(chain(16))
 product(ham)
 """)
+
+
+@pytest.mark.parametrize("n,total,two_s", [(10, 10, 2), (18, 18, 2), (9, 13, 3), (8, 16, 4), (16, 8, 1)])
+def test_spin_s_products_take_the_rows_apply(lib, n, total, two_s):
+    """What the comparison with the tile apply on a GPU rests on: these sectors have a plan."""
+    fake_gpu.run(lib, CHAINS + f"""
+ham = ed.Hamiltonian({n}, {total}, chain({n}), two_s={two_s}, generic=True)
+product(ham)
+assert fake.fake_launches(b"spin_rows_kernel") == 1 and fake.fake_launches(b"spin_hv_kernel") == 0
+""")

@@ -56,7 +56,7 @@ struct HvParams {
   int N, Nlo, n_up;
   int n_pairs;  // entries in low[] and rise[]
   int n_diag;
-  int finite;  // every flip's coefficient is finite
+  int finite, finite32;  // every flip's coefficient is finite, also when rounded to FP32
   uint32_t lomask;
   // pairs in ascending-column order for a row: "low" flips (target < source)
   // sorted by (hi desc, lo asc); "rise" flips (target > source) by (hi asc, lo desc)

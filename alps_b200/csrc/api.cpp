@@ -357,7 +357,7 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
       return AED_OK;
     }
   }
-  if (!h->P.finite || !h->dt.rprog[f32 ? 1 : 0][0]) {  // the tile apply alone: nothing to time or to keep for others
+  if (!rows_apply_finite(f32 ? 4 : 8, h->P) || !h->dt.rprog[f32 ? 1 : 0][0]) {  // the tile apply alone: nothing to time or to keep for others
     *out = 0;
     return AED_OK;
   }

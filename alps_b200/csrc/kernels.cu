@@ -603,6 +603,15 @@ constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 // threads launch the same kernels.
 std::mutex g_grid_mu;
 
+// AED_FP32_ACCUM=twosum: the row sums of the FP32 applies, which round the couplings to FP32.
+bool fp32_twosum() {
+  static const bool on = [] {
+    const char* e = std::getenv("AED_FP32_ACCUM");
+    return e && std::string(e) == "twosum";
+  }();
+  return on;
+}
+
 template <typename T, typename Acc, int R, int B>
 int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
   static int grid_all = 0;
@@ -636,7 +645,8 @@ int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* 
 template <typename T, typename Acc, int ROW, int NT, int MINB>
 int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
   constexpr int B = ROW / (int)sizeof(T), kTab = ROW == 16 ? 0 : 1, kEl = sizeof(T) == 8 ? 0 : 1;
-  if (!t.low_e || !t.rprog[kEl][kTab] || !t.flag || t.maxrows <= 0 || !P.finite) return kVariantNotApplicable;
+  if (!t.low_e || !t.rprog[kEl][kTab] || !t.flag || t.maxrows <= 0 || !rows_apply_finite(sizeof(T), P))
+    return kVariantNotApplicable;
   const size_t dyn = rapply::rows_smem_bytes(ROW, t.maxrows, t.rstride[kEl][kTab]);
   constexpr bool kDraws = NT <= 512;
   auto kern = hvr_kernel<T, Acc, B, NT, MINB, false>;
@@ -745,6 +755,8 @@ int launch_hv_t(int v, const HvParams& P, const DevTables& t, const T* x, T* y, 
   }
 }
 
+bool rows_apply_finite(int elem, const HvParams& P) { return elem == 4 && fp32_twosum() ? P.finite32 : P.finite; }
+
 int hv_num_variants() { return kNumVariants; }
 bool hv_variant_tuned(int v) { return v == 0 || (v > 0 && v < kNumVariants && kVariants[v].kind == 2); }
 int hv_small_variant() { return kSmallVariant; }
@@ -757,11 +769,7 @@ int launch_hv_f64(int variant, const HvParams& P, const DevTables& t, const doub
 
 int launch_hv_f32(int variant, const HvParams& P, const DevTables& t, const float* x, float* y,
                   double* alpha_part, cudaStream_t st) {
-  static const bool twosum = [] {
-    const char* e = std::getenv("AED_FP32_ACCUM");
-    return e && std::string(e) == "twosum";
-  }();
-  if (twosum) return launch_hv_t<float, AccTwoSum32>(variant, P, t, x, y, alpha_part, st);
+  if (fp32_twosum()) return launch_hv_t<float, AccTwoSum32>(variant, P, t, x, y, alpha_part, st);
   return launch_hv_t<float, AccWide32>(variant, P, t, x, y, alpha_part, st);
 }
 

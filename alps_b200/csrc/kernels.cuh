@@ -66,6 +66,8 @@ int launch_hv_f64(int variant, const HvParams& P, const DevTables& t, const doub
 int launch_hv_f32(int variant, const HvParams& P, const DevTables& t, const float* x, float* y,
                   double* alpha_part, cudaStream_t st);
 constexpr int kVariantNotApplicable = 2;
+// Whether the rows applies take P's couplings for vectors of `elem` bytes an element: all finite, as they use them.
+bool rows_apply_finite(int elem, const HvParams& P);
 int hv_num_variants();
 const char* hv_variant_name(int v);
 // The variant of sectors too small to time.

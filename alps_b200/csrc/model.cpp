@@ -137,8 +137,11 @@ int build_hv_params(const Model& m, int Nlo, HvParams& P) {
   P.n_lolo = 0;
   for (int i = 0; i < P.n_pairs; ++i)
     if ((P.low[i].mhi >> Nlo) == 0u) P.lolo_c[P.n_lolo++] = P.low[i].c;
-  P.finite = 1;  // the merged coefficients may overflow
-  for (int i = 0; i < P.n_pairs; ++i) P.finite &= std::isfinite(P.low[i].c) ? 1 : 0;
+  P.finite = P.finite32 = 1;  // the merged coefficients may overflow
+  for (int i = 0; i < P.n_pairs; ++i) {
+    P.finite &= std::isfinite(P.low[i].c) ? 1 : 0;
+    P.finite32 &= std::isfinite((float)P.low[i].c) ? 1 : 0;
+  }
   return AED_OK;
 }
 

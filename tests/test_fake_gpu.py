@@ -179,3 +179,18 @@ ham = ed.Hamiltonian({n}, {total}, chain({n}), two_s={two_s}, generic=True)
 product(ham)
 assert fake.fake_launches(b"spin_rows_kernel") == 1 and fake.fake_launches(b"spin_hv_kernel") == 0
 """)
+
+
+def test_twosum_rows_of_couplings_beyond_fp32_take_the_tile_apply(lib):
+    """The compensated FP32 sums round the couplings to FP32, where they may overflow."""
+    fake_gpu.run(lib, CHAINS + OVERFLOW + """
+for n in (8, 16):
+    big = chain(n) + [(0, 1, 0.0, 1e39)]
+    for precision, rows in ((ed.FP32, False), (ed.FP64, True)):
+        ham = ed.Hamiltonian(n, n // 2, big, precision=precision)
+        product(ham)
+        assert takes(ham, b"hvr_kernel") == rows and takes(ham, b"9hv_kernel") != rows
+    ham = ed.Hamiltonian(n, n // 2, chain(n) + [(0, 2, 0.0, 1.0)], precision=ed.FP32)
+    product(ham)
+    assert takes(ham, b"hvr_kernel")
+""", {"AED_FP32_ACCUM": "twosum"})

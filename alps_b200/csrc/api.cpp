@@ -405,8 +405,8 @@ int pick_variant(aed_handle* h, bool f32, const void* x, void* y, int* out) {
   if (rc) return rc;
   // the first rows apply within 5 % of the fastest: the forms of one row width
   // stand in order of CTA size, and beside the products of other streams smaller
-  // CTAs do better than alone (5x5 with 11 up FP64, 256 and 512 threads: 165 and
-  // 162 us alone, 138 and 155 a product with three handles in turn).  The tile
+  // CTAs do better than alone (5x5 with 11 up FP64, 256 and 512 threads: 158 and
+  // 161 us alone, 129 and 146 a product with three handles in turn).  The tile
   // apply (0) only where it beats them by more: it does not start while its
   // predecessor ends, which a product timed alone does not show
   const float least = *std::min_element(ms_of.begin(), ms_of.end());

@@ -20,13 +20,14 @@
 // they are formed from the finished rows, after the bundle.
 //
 // Bound by the latency of the x loads outside the lo part (L2 and, above its
-// size, DRAM) behind 32 warps per SM; part costs on 6x5 FP32 (3.93 ms, a copy
+// size, DRAM) behind 32 warps per SM; part costs on 6x5 FP32 (of 3.93 ms, a copy
 // with one part left out): hi-part flips 1.15 ms, crossing 1.48, lo-part 0.83;
-// L=28 FP64 (1.34 ms): outside the lo part 0.83, lo-part 0.29.
-// Measured (L2 flushed, with partials, us; in brackets the apply before: one
-// block of x in shared memory, 4 rows per thread): J1-J2 chain L=28 FP64 1266
-// (1684; before hi_terms had its short form), FP32 771 (1102); 6x5 FP32 3700 (5570); L=24 FP64
-// 92 (133), FP32 59 (88); L=16 FP64 8.4 (18.4).
+// L=28 FP64 (of 1.34 ms, before hi_terms had its short form): outside the lo
+// part 0.83, lo-part 0.29.
+// Measured (applies in a row, with partials, us; in brackets the apply before:
+// one block of x in shared memory, 4 rows per thread, L2 flushed between its
+// applies): J1-J2 chain L=28 FP64 1173 (1684), FP32 771 (1102); 6x5 FP32 3870
+// (5570); L=24 FP64 84 (133), FP32 64 (88).
 //
 // Reference paths are relative to the ALPS source tree.
 #pragma once

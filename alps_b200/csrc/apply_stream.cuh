@@ -15,7 +15,7 @@
 // run ahead of the arithmetic by the depth of the ring, so the gathers no
 // longer stall on dependent global loads.
 //
-// Each row adds its terms in the same order as the tile and bundle applies
+// Each row adds its terms in the same order as the tile and rows applies
 // (apply.cuh, apply_rows.cuh), so FP64 rows are bit-identical to
 // y = prod(M, x) of the reference's explicit matrix
 // (src/ietl/interface/ublas.h:57-63 over hamiltonian_matrix.hpp:307-345),

@@ -25,7 +25,7 @@ struct aed_handle {
   uint32_t* d_looff = nullptr;
   uint32_t* d_tile_h = nullptr;
   uint32_t* d_tile_r = nullptr;
-  uint32_t* d_blk_h = nullptr;   // block list of the bundle apply
+  uint32_t* d_blk_h = nullptr;   // block list of the rows and stream applies
   uint32_t* d_tfirst = nullptr;  // first tile of each hi block
   double* d_dg = nullptr;     // per-row diagonal
   uint32_t* d_ell = nullptr;  // lo-neighbour table

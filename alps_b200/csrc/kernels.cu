@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kHvThreads, MINB) hv_kernel(const __grid_const
 }
 
 // y = H x over bundles with x interleaved in shared memory (apply_rows.cuh).
-// DRAW: bundles by rapply::Taker (more than two per CTA), else round robin.
+// DRAW: bundles by rapply::Taker (more than three per CTA), else round robin.
 // (With 296 bytes of arguments the host needed 0.4 us more per launch than with
 // the 288 that these are, a multiple of 32; a smaller struct gained nothing.)
 template <typename T, typename Acc, int B, int NT, int MINB, bool DRAW>
@@ -635,13 +635,14 @@ int launch_one(const HvParams& P, const DevTables& t, const T* x, T* y, double* 
 // sizes).  Not for couplings that are not finite: a flip that a row does not
 // take adds c * 0.
 //
-// Bundles are drawn from a counter when there are more than three per CTA and
-// several CTAs to an SM.  Measured, round robin against drawn, us with L2
-// flushed, FP64: chain L=28 (384 threads) 1422 / 1266, L=26 (256) 350 / 332,
-// 5x5 with 11 up 190 / 173, L=26 with 9 up 134 / 112, L=24 at 3.5 bundles per
-// CTA 95.8 / 91.5; FP32 6x5 3870 / 3620.  With less to even out the hand-out
-// only costs (0.4 us of the chain L=20's 11.7), and with one CTA of 1024
-// threads on an SM it costs more than it evens out (L=28: 1444 / 1501).
+// Bundles are drawn from a counter when there are more than three per CTA of at
+// most 512 threads.  Measured, round robin against drawn (applies in a row, with
+// partials, us), FP64: chain L=28 (384 threads) 1375 / 1175, L=26 (256) 319 /
+// 306, 5x5 with 11 up (256) 174 / 158, L=26 with 9 up (256) 120 / 104, L=24 (256,
+// 3.5 bundles per CTA) 89 / 84; FP32 6x5 (512) 4297 / 3877.  With less to even
+// out the hand-out only costs (0.4 us of the chain L=20's 11.7), and with one CTA
+// of 1024 threads on an SM it costs more than it evens out (L=28, when the
+// counter came: 1444 / 1501).
 template <typename T, typename Acc, int ROW, int NT, int MINB>
 int launch_rows(const HvParams& P, const DevTables& t, const T* x, T* y, double* alpha_part, cudaStream_t st) {
   constexpr int B = ROW / (int)sizeof(T), kTab = ROW == 16 ? 0 : 1, kEl = sizeof(T) == 8 ? 0 : 1;

@@ -24,7 +24,7 @@ struct DevTables {
   int64_t n_tiles;
   int64_t D;
   int Nlo, Nhi, n_up;
-  // block list of the bundle and rows applies (build_block_list): hi blocks grouped by
+  // block list of the rows and stream applies (build_block_list): hi blocks grouped by
   // lo popcount, each group padded with kNoBlock to a multiple of kBundleMax
   const uint32_t* blk_h = nullptr;   // n_blk
   const uint32_t* tfirst = nullptr;  // 2^Nhi: index of the first tile of each hi block

@@ -413,7 +413,7 @@ __device__ __forceinline__ void mom_row_terms(const uint32_t (&e)[U], int jbits,
 // Bound by the x_j gathers (one 32-byte sector each from L2): the walking
 // kernel, bound by the latency of four dependent loads a term, took 225.5 us
 // a product on the J1-J2 chain L=28 and 287 on the spin-1 chain L=18; this one
-// 84.5 and 100.
+// 86 and 102.
 template <bool kDiagFirst, int NT, int U, int MINB>
 __global__ void __launch_bounds__(NT, MINB) mom_rows_kernel(const MomRows rw, const double2* x, double2* y,
                                                             double* alpha_part) {
@@ -783,8 +783,9 @@ void mom_rows_go(const MomRows& r, bool diag_first, unsigned grid, size_t dyn, c
 
 // A tile per CTA.  Many tiles: 256 threads, five CTAs per SM (48 registers,
 // no spill), four x_j in flight per thread: 84.5 us a product on the J1-J2
-// chain L=28 (1.43M rows), against 87.6 with six in flight at four CTAs, 86.0
-// with 512 threads and 92.8-107 with fewer, larger CTAs.  Up to four tiles
+// chain L=28 (1.43M rows; 86 in a stream of products on changing vectors),
+// against 87.6 with six in flight at four CTAs, 86.0 with 512 threads and
+// 92.8-107 with fewer, larger CTAs.  Up to four tiles
 // per SM the 1024 rows of a tile run side by side instead of four deep, so
 // that a small sector still fills the SMs: a solve of the chain L=22, k = pi
 // (32 tiles) takes 5.0 ms against 6.1 with 256 threads.

@@ -52,9 +52,9 @@ NEV = 2
 FP64_ITERATIONS_FALLBACK = 180  # mean of the first five inputs: 190, 142, 180, 182, 208
 
 # DRAM bytes (read + write) of one launch of the FP64 apply on this workload,
-# per apply variant, from ncu (dram__bytes_read.sum + dram__bytes_write.sum),
-# summarised in profiles/hvr_kernel_l28_fp64.md; null for a variant not captured.
-HV_TRAFFIC_L28_FP64 = {"row16n384": 2.229158e9}
+# per apply variant, from ncu (dram__bytes_read.sum + dram__bytes_write.sum);
+# null for a variant not captured.
+HV_TRAFFIC_L28_FP64 = {"row16n384": 2.162975e9}
 
 
 def j2_stream(n):
@@ -343,8 +343,7 @@ def run_ours(args):
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": peak_kind, "kernel": f"apply variant {vname} (FP64)", "apply_ms": t_apply * 1e3,
             "algorithmic_bytes_per_apply": b_apply, "traffic": HV_TRAFFIC_L28_FP64.get(vname),
-            "traffic_source": "profiles/hvr_kernel_l28_fp64.md (ncu dram__bytes_read.sum + dram__bytes_write.sum, "
-                              "one launch)",
+            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch",
             "note": "algorithmic bytes count every gathered x_j; shared memory and L2 serve most of them, so frac may "
                     "exceed 1; traffic is what DRAM moved"}
     print(f"[bench] fp64: {value:.3f} solves/s, iterations {iters}, apply {t_apply*1e3:.3f} ms "

@@ -638,7 +638,7 @@ def run_momentum(args):
                                    "2 pi m / 28, m = 0..27, lowest 2 eigenvalues per sector"},
             "lowest_over_momenta": lowest, "sz0_fp64_ground_state": e0,
             "rel_diff": abs(lowest - e0) / abs(e0), "sz0_fp64_solve_s": t_real,
-            "roofline": {"bound": "hbm", "kernel": "mom_hv_kernel", "achieved": ach, "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": "mom_rows_kernel", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "peak_kind": peak_kind, "apply_ms": ms0, "rows": dim0,
                          "algorithmic_bytes_per_row": b_row},
             "sectors": sectors}
@@ -671,7 +671,7 @@ def run_spin(args):
             "n_gpus": 1, "higher_is_better": True, "dtype": "f64", "data": "synthetic",
             "config": {"workload": "spin-1 Heisenberg chain L=18 periodic, J=1, Sz_total=0, D=%d" % ham.dim},
             "iterations": r["iterations"], "evals": r["evals"].tolist(),
-            "roofline": {"bound": "hbm", "kernel": "spin_hv_kernel", "achieved": ach, "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": "spin_rows_kernel", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "peak_kind": peak_kind, "apply_ms": ms,
                          "algorithmic_bytes_per_row": b_row, "offdiag_per_row_sampled": nbar}}
     ham.close()

@@ -7,6 +7,7 @@
 
 #include "aed_internal.h"
 #include "kernels.cuh"
+#include "launch_limits.h"
 #include "momentum.cuh"
 #include "spin.cuh"
 
@@ -109,12 +110,14 @@ namespace aed {
 
 // RAII device switch for an API call.
 struct DeviceGuard {
-  int prev = -1;
+  int prev = -1, outer = t_guarded_device;
   explicit DeviceGuard(int dev) {
     cudaGetDevice(&prev);
     if (prev != dev) cudaSetDevice(dev);
+    t_guarded_device = dev;
   }
   ~DeviceGuard() {
+    t_guarded_device = outer;
     int cur = -1;
     cudaGetDevice(&cur);
     if (prev >= 0 && cur != prev) cudaSetDevice(prev);

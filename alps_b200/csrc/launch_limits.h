@@ -17,6 +17,9 @@
 
 namespace aed {
 
+// The device that a DeviceGuard of this thread has made current (-1: none).
+inline thread_local int t_guarded_device = -1;
+
 // Of one kernel (a static object beside its launch; a launch-bound product asks
 // on every call, so the few entries are searched in turn).
 class KernelLimits {
@@ -25,8 +28,7 @@ class KernelLimits {
   // SM of the current device holds; 0: none, negative: an error code.
   int ctas_per_sm(const void* kern, int threads, size_t dyn) {
     std::lock_guard<std::mutex> lk(mu_);
-    int dev = 0;
-    cudaGetDevice(&dev);
+    const int dev = current();
     for (const Shape& s : shapes_)
       if (s.dev == dev && s.threads == threads && s.dyn == dyn) return s.ctas;
     size_t most = 0;
@@ -43,9 +45,7 @@ class KernelLimits {
   // The most dynamic shared memory a CTA of the kernel may take on the current device.
   int most_dynamic(const void* kern, size_t* most) {
     std::lock_guard<std::mutex> lk(mu_);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return raise(kern, dev, most);
+    return raise(kern, current(), most);
   }
 
  private:
@@ -54,6 +54,11 @@ class KernelLimits {
     size_t dyn;
     int ctas;
   };
+  static int current() {
+    int dev = t_guarded_device;
+    if (dev < 0) cudaGetDevice(&dev);
+    return dev;
+  }
   int raise(const void* kern, int dev, size_t* most) {
     *most = 0;
     auto it = most_.find(dev);
